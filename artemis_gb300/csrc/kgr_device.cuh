@@ -459,6 +459,55 @@ __device__ __forceinline__ bool test_leaves(const DeviceScene &s, const FastRay 
 	return false;
 }
 
+/* The persistent walk of one warp: each of its first `lanes` lanes walks one
+ * ray at a time and takes the next as soon as its own is finished, so a lane
+ * whose ray ends early does not idle until the longest ray of its warp is
+ * done.  One iteration descends to a leaf with the postponed-leaf rule
+ * (speculative_descend) and tests it.  All 32 lanes call it.
+ *   next(need, a, b)   warp-collective: whether a lane that needs a ray got
+ *                      one, {origin, -} and {direction, tmax}
+ *   done(best, hit)    the lane's ray is finished (hit: occluded, for ANY) */
+template <bool ANY, bool COUNT, int LAYOUT, class STACK, class Next, class Done>
+__device__ __forceinline__ void persistent_walk(const DeviceScene &s, STACK &stack, int lanes, TraceCounters *cnt,
+		Next next, Done done)
+{
+	bool have = false, exhausted = (int)(threadIdx.x & 31) >= lanes;
+	FastRay r;
+	kgr_hit best;
+	int32_t best_rank = 0x7fffffff;
+	int32_t ref = 0;
+	for (;;) {
+		bool need = !have && !exhausted;
+		if (__any_sync(0xffffffffu, need)) {
+			float4 a, b;
+			if (next(need, a, b)) {
+				r = fast_ray(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z));
+				best.prim = -1;
+				best.t = b.w;
+				best.b1 = 0.0f;
+				best.b2 = 0.0f;
+				best_rank = 0x7fffffff;
+				stack.clear();
+				ref = 0;
+				have = true;
+			} else if (need) {
+				exhausted = true;
+			}
+		}
+		if (!__any_sync(0xffffffffu, have))
+			break;
+		if (!have)
+			continue;
+		int32_t leaf = 0;
+		speculative_descend<LAYOUT, COUNT>(s, r, ref, leaf, best.t, stack, cnt);
+		bool occ = test_leaves<ANY, COUNT>(s, r, ref, leaf, best, best_rank, stack, cnt);
+		if (occ || ref == KGR_REF_NONE) {
+			done(best, occ);
+			have = false;
+		}
+	}
+}
+
 template <bool ANY, bool COUNT, int LAYOUT, class STACK>
 __device__ __forceinline__ bool trace_fast_stack(const DeviceScene &s, const f3 &o, const f3 &d,
 		float tmax, kgr_hit &best, STACK &stack, TraceCounters *cnt = nullptr)
