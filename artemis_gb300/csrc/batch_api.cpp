@@ -113,6 +113,8 @@ void kgr_batcher::render(const kgr_scene *scene, const kgr_batch_job *jobs, uint
 	fp.tune = tune;
 	DeviceScene s = scene->view();
 	PathBuffers pb = path_buffers();
+	if (side.stream)
+		pb.coop_rounds = KGR_COOP_ROUNDS_OVERLAPPED;
 	const BatchHeader *dh = reinterpret_cast<const BatchHeader *>(table.ptr);
 	const BatchJob *djobs = reinterpret_cast<const BatchJob *>(table.ptr + 16);
 

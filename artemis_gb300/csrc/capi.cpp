@@ -119,6 +119,7 @@ kgr::DeviceScene kgr_scene::view() const
 	s.cw_nodes = d_cw_nodes.ptr;
 	s.cw_tris = d_cw_tris.ptr;
 	s.cw_node_count = cw_node_count;
+	s.coop_nodes = d_coop_nodes.ptr;
 	s.quads = nullptr;
 	s.quad_count = 0;
 	s.has_env = 0;
@@ -130,7 +131,7 @@ kgr::DeviceScene kgr_scene::view() const
 uint64_t kgr_scene::device_bytes() const
 {
 	return d_positions.bytes() + d_normals.bytes() + d_tris.bytes() + d_bvh.bytes() + d_fast_tris.bytes()
-		+ d_fast_nodes.bytes() + d_wide_nodes.bytes() + d_cw_nodes.bytes() + d_cw_tris.bytes() + d_materials.bytes()
+		+ d_fast_nodes.bytes() + d_wide_nodes.bytes() + d_cw_nodes.bytes() + d_cw_tris.bytes() + d_coop_nodes.bytes() + d_materials.bytes()
 		+ d_lights.bytes();
 }
 
@@ -371,6 +372,22 @@ void finish_scene(kgr_scene *sc, const Tree &tree, const std::vector<PrimBox> &b
 		sc->cw_depth = cw_depth;
 		static_assert(sizeof(CwNode) == 80, "compressed node size");
 		KGR_REQUIRE(((uintptr_t)sc->d_cw_nodes.ptr & 15) == 0, KGR_ERR_INTERNAL, "compressed nodes misaligned");
+		/* the cooperative walk's nodes: made on the device, as a refit makes
+		 * them again */
+		std::vector<float4> tree_boxes(2 * tree.nodes.size());
+		for (size_t i = 0; i < tree.nodes.size(); i++) {
+			const TreeNode &n = tree.nodes[i];
+			tree_boxes[2 * i] = make_float4(n.bmin[0], n.bmin[1], n.bmin[2], 0.0f);
+			tree_boxes[2 * i + 1] = make_float4(n.bmax[0], n.bmax[1], n.bmax[2], 0.0f);
+		}
+		DevBuf<float4> d_boxes;
+		DevBuf<int32_t> d_kids;
+		d_boxes.upload(tree_boxes);
+		d_kids.upload(sc->plan.cw_kids);
+		coop_nodes(sc, d_kids.ptr, d_boxes.ptr, 0);
+		/* the scene may be traced on any stream from here on, and the two
+		 * uploads are released */
+		KGR_CUDA(cudaStreamSynchronize(0));
 	} else {
 		sc->plan.cw_kids.clear();
 	}
@@ -1224,6 +1241,7 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 		 * recursion. */
 		att->ensure_side_stream();
 		cudaStream_t side = att->side;
+		pb.coop_rounds = KGR_COOP_ROUNDS_OVERLAPPED;
 		pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
 		m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 		for (int d = 0; d <= last; d++) {
@@ -1527,8 +1545,10 @@ void render_pt_cached(kgr_attachment *att, const kgr_launch_info *info, const kg
 	 * cache's radiance is added, so each path's radiance is summed in the
 	 * order of the recursion. */
 	const bool overlap = att->opt_int("trace_overlap", 1) != 0;
-	if (overlap)
+	if (overlap) {
 		att->ensure_side_stream();
+		pb.coop_rounds = KGR_COOP_ROUNDS_OVERLAPPED;
+	}
 	int m = att->mark(-1, st);
 	pt_generate(pb, fp, st);
 	m = att->mark(STAGE_GENERATE, st, m);

@@ -729,6 +729,185 @@ __device__ __forceinline__ bool trace_cw(const DeviceScene &s, const f3 &o, cons
 	}
 }
 
+/* ------------------------------------------------- cooperative walk -- */
+
+/* The walk of one warp with eight lanes a ray, four rays at a time: lane j of
+ * a group tests slot j ^ octant of the group's node (CoopNode), so one node
+ * fetch covers eight children, and the children a ray reaches are visited in
+ * the slots' front-to-back order of its octant, lane 0's first.  A lane parks
+ * a reached leaf and the group's leaves are tested together, one lane a leaf.
+ *
+ * A ray alone waits about 300 ns for every node it visits (the fetch comes
+ * from L2) and 400 for every triangle; this walk has a third of the nodes on
+ * its path and tests the triangles of several leaves at once.  It is for ray
+ * counts that leave the GPU waiting for the longest walks (KGR_COOP_ROUNDS);
+ * with enough rays to fill it, the per-thread walks need fewer instructions a
+ * ray.  4,096 camera rays on the box scene: 43 -> 25 us a call.
+ * Tried and no better: the nearest child first, prefetching the children that
+ * wait, testing a leaf in the same step as the next node, and letting this
+ * walk take over the last rays of a persistent warp.
+ *
+ * The children of one node that are still to be visited stay on their lanes:
+ * a level of the stack is one {reference, distance} per lane, in local
+ * memory.  Candidates are compared per lane by (t, rank) and once across the
+ * group at the end, so the hit is that of the other layouts.
+ *   next(need, a, b)  warp-collective, need the same in a group's lanes:
+ *                     whether the group got a ray
+ *   done(hit, occ)    called by one lane of the group */
+struct CoopRay {
+	FastRay r;
+	uint32_t slot;         /* this lane's slot of every node */
+	float best_t;          /* of the group: what boxes are culled against */
+	kgr_hit own;           /* of this lane's triangles */
+	int32_t own_rank;
+};
+
+template <bool ANY, class Next, class Done>
+__device__ __forceinline__ void coop_walk(const DeviceScene &s, Next next, Done done)
+{
+	const unsigned full = 0xffffffffu;
+	const int lane = threadIdx.x & 31, j = lane & 7, gs = lane & 24;
+	uint2 level[KGR_COOP_LEVELS];
+	int sp = 0;
+	bool have = false, exhausted = false;
+	int32_t node = -1, leaf = 0;
+	CoopRay w;
+	w.best_t = 0.0f;
+	for (;;) {
+		bool need = !have && !exhausted;
+		if (__any_sync(full, need)) {
+			float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
+			bool got = next(need, a, b);
+			/* lanes 0, 1 and 2 of a group divide, one component each */
+			float c = j == 0 ? b.x : (j == 1 ? b.y : b.z);
+			float inv = 1.0f / (fabsf(c) > 1e-20f ? c : copysignf(1e-20f, c));
+			float ix = __shfl_sync(full, inv, gs), iy = __shfl_sync(full, inv, gs + 1),
+			      iz = __shfl_sync(full, inv, gs + 2);
+			if (got) {
+				w.r.o = mk(a.x, a.y, a.z);
+				w.r.d = mk(b.x, b.y, b.z);
+				w.r.ix = ix;
+				w.r.iy = iy;
+				w.r.iz = iz;
+				w.r.ox = a.x * ix;
+				w.r.oy = a.y * iy;
+				w.r.oz = a.z * iz;
+				w.slot = (uint32_t)j ^ ((ix < 0.0f ? 1u : 0u) | (iy < 0.0f ? 2u : 0u) | (iz < 0.0f ? 4u : 0u));
+				w.best_t = b.w;
+				w.own.prim = -1;
+				w.own.t = b.w;
+				w.own.b1 = 0.0f;
+				w.own.b2 = 0.0f;
+				w.own_rank = 0x7fffffff;
+				node = 0;
+				sp = 0;
+				have = true;
+			} else if (need) {
+				exhausted = true;
+			}
+		}
+		if (!__any_sync(full, have))
+			return;
+		/* the node's eight children */
+		int32_t ref = KGR_WIDE_EMPTY;
+		float tn = 0.0f;
+		bool hit = false;
+		if (node >= 0) {
+			float4 a, b;
+			ldg256(s.coop_nodes[node].slot + 2u * w.slot, a, b);
+			ref = __float_as_int(b.z);
+			tn = wide_child(w.r, a.x, a.y, a.z, a.w, b.x, b.y, ref, w.best_t);
+			hit = tn < __int_as_float(0x7f800000);
+		}
+		const bool inner = hit && ref >= 0, parks = hit && ref < 0;
+		uint32_t m = (__ballot_sync(full, inner) >> gs) & 0xffu;
+		int first = m ? __ffs(m) - 1 : 0;
+		int32_t to = __shfl_sync(full, ref, gs + first);
+		node = m ? to : -1;
+		if (m & (m - 1u)) {
+			level[sp] = make_uint2((uint32_t)(inner && j != first ? ref : KGR_WIDE_EMPTY), __float_as_uint(tn));
+			sp++;
+		}
+		/* leaves: parked until a lane has a second one or its group has no
+		 * node left */
+		bool out = have && node < 0 && sp == 0;
+		bool clash = parks && leaf != 0;
+		if (!clash && parks)
+			leaf = ref;
+		if (__any_sync(full, clash || out)) {
+			bool occ = false;
+			do {
+				while (__any_sync(full, leaf != 0)) {
+					if (leaf != 0) {
+						uint32_t code = ~(uint32_t)leaf;
+						if (cw_triangle<ANY, false>(s, w.r, code >> 3, w.own, w.own_rank, nullptr))
+							occ = true;
+						/* the leaf less its first triangle */
+						leaf = (code & 7u) == 0u ? 0 : (int32_t)~(code + 7u);
+					}
+				}
+				if (clash)
+					leaf = ref;
+				clash = false;
+				/* a group without nodes finishes its second leaf too */
+			} while (__any_sync(full, out && leaf != 0));
+			if (ANY) {
+				uint32_t g = (__ballot_sync(full, occ) >> gs) & 0xffu;
+				if (g) {
+					leaf = 0;
+					node = -1;
+					sp = 0;
+					out = true;
+				}
+				if (out) {
+					if (j == 0)
+						done(w.own, g != 0u);
+					have = false;
+				}
+			} else {
+				float t = w.own.t;
+				for (int x = 1; x < 8; x <<= 1)
+					t = fminf(t, __shfl_xor_sync(full, t, x));
+				w.best_t = t;
+				if (__any_sync(full, out)) {
+					int32_t rank = w.own.t == t ? w.own_rank : 0x7fffffff;
+					for (int x = 1; x < 8; x <<= 1) {
+						int32_t o = __shfl_xor_sync(full, rank, x);
+						rank = o < rank ? o : rank;
+					}
+					/* every candidate has a rank of its own; with none, lane 0
+					 * reports the miss */
+					bool mine = rank == 0x7fffffff ? j == 0 : (w.own.t == t && w.own_rank == rank);
+					if (out) {
+						if (mine)
+							done(w.own, false);
+						have = false;
+					}
+				}
+			}
+		}
+		/* groups without a node take the next child of the last level */
+		while (__any_sync(full, have && node < 0 && sp > 0)) {
+			bool pop = have && node < 0 && sp > 0;
+			uint2 e = make_uint2((uint32_t)KGR_WIDE_EMPTY, 0u);
+			if (pop)
+				e = level[sp - 1];
+			bool alive = (int32_t)e.x != KGR_WIDE_EMPTY && __uint_as_float(e.y) <= w.best_t;
+			uint32_t k = (__ballot_sync(full, alive) >> gs) & 0xffu;
+			int f = k ? __ffs(k) - 1 : 0;
+			int32_t n = __shfl_sync(full, (int32_t)e.x, gs + f);
+			if (pop) {
+				if (k)
+					node = n;
+				if (k & (k - 1u))
+					level[sp - 1].x = (uint32_t)(alive && j != f ? (int32_t)e.x : KGR_WIDE_EMPTY);
+				else
+					sp--;
+			}
+		}
+	}
+}
+
 template <bool ANY, bool COUNT, int LAYOUT = KGR_LAYOUT_FAST>
 __device__ __forceinline__ bool trace_fast(const DeviceScene &s, const f3 &o, const f3 &d,
 		float tmax, kgr_hit &best, TraceCounters *cnt = nullptr)

@@ -168,6 +168,29 @@ struct CwNode {
 	uint4 qb;      /* lo.z[0..7], hi.x[0..7] */
 	uint4 qc;      /* hi.y[0..7], hi.z[0..7] */
 };
+/* 256-byte eight-child node of the cooperative walk, eight lanes a ray: the
+ * compressed layout's tree (node i is CwNode i, slot j its slot j) with the
+ * padded boxes unquantised.  Slot j is {lo.x, hi.x, lo.y, hi.y}, {lo.z, hi.z,
+ * bits(ref), 0}: ref >= 0 an internal node, KGR_WIDE_EMPTY an empty slot,
+ * else a leaf ~((first << 3) | (n - 1)) over the compressed layout's triangle
+ * records. */
+struct CoopNode {
+	float4 slot[16];
+};
+/* The cooperative walk runs when there are at most this many rays for each of
+ * the groups the GPU holds at once (19,456 to 23,104 of them).  Closest-hit
+ * bounce rays on the box scene, the 0.26M- and the 1.16M-triangle terrain, us,
+ * this walk / the persistent one: 4,096 rays 31, 39, 43 / 48, 45, 58; 16,384
+ * rays 33, 45, 60 / 70, 68, 75; 65,536 rays 83, 88, 107 / 97, 91, 114; 131,072
+ * rays 147, 145, 190 / 121, 102, 121.  It takes more instructions a ray, so
+ * walks that share the GPU with another launch switch earlier: two 78,003-ray
+ * walks side by side (a 321 x 243 frame) 797 us a frame on the persistent walk
+ * and 872 with this one. */
+#define KGR_COOP_ROUNDS 4u
+#define KGR_COOP_ROUNDS_OVERLAPPED 2u
+/* most nodes on a path of the cooperative walk */
+#define KGR_COOP_LEVELS 16
+
 /* traversal stack entries of the compressed layout (node groups) */
 #define KGR_CW_STACK 32
 
@@ -232,6 +255,7 @@ struct DeviceScene {
 	const CwNode *cw_nodes;
 	const float4 *cw_tris; /* 3 per triangle, compressed-layout node order */
 	uint32_t cw_node_count;
+	const CoopNode *coop_nodes; /* one per compressed node; NULL: no cooperative walk */
 	/* lights of the launch beyond the scene's triangles: quad lights
 	 * (sampled only, never traced) and an environment texture */
 	const kgr_quad_light *quads;
@@ -317,6 +341,7 @@ struct kgr_scene {
 	kgr::DevBuf<kgr::WideNode> d_wide_nodes;
 	kgr::DevBuf<kgr::CwNode> d_cw_nodes;
 	kgr::DevBuf<float4> d_cw_tris;
+	kgr::DevBuf<kgr::CoopNode> d_coop_nodes;
 	kgr::DevBuf<kgr_material> d_materials;
 	kgr::DevBuf<kgr_triangle_light> d_lights;
 
@@ -401,6 +426,11 @@ inline double time_frames(F frame, int frames, cudaStream_t st)
  * boxes and triangle records, in place, on st. */
 enum { REFIT_TRANSFORM = 0, REFIT_POSITIONS = 1 };
 void refit_scene(kgr_scene *sc, int mode, const float *positions, const float *normals, cudaStream_t st);
+
+/* The cooperative walk's nodes from the compressed ones (topology) and the
+ * tree's boxes (2 float4 per tree node) and slots (8 per compressed node, -1
+ * empty), all on the device (refit.cu). */
+void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, cudaStream_t st);
 
 /* Traversal of a ray buffer (8 floats per ray) into hits or occlusion flags. */
 void launch_trace_closest(const DeviceScene &s, const float4 *rays, uint32_t n,

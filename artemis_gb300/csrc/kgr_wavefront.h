@@ -54,6 +54,9 @@ struct PathBuffers {
 	 * walks take rays 0 .. counters[CNT_SHADOW]-1 in order (the id of a
 	 * ray is its position) */
 	uint32_t *shadow_flags = nullptr;
+	/* the walks go to the cooperative walk (eight lanes a ray) up to this
+	 * many rays for each of the groups the launch holds */
+	uint32_t coop_rounds = KGR_COOP_ROUNDS;
 };
 
 /* The float4 arrays of the path state, in the order their allocators lay

@@ -294,60 +294,51 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) fast_persis
 	const int lane = threadIdx.x & 31;
 	TraceCounters cnt = {0, 0};
 	uint32_t p = 0;
-	bool have = false, exhausted = false;
-	FastRay r;
-	kgr_hit best;
-	int32_t best_rank = 0x7fffffff;
+	auto load = [&](uint32_t i, float4 &a, float4 &b) {
+		p = (ANY && !queue) ? i : queue[i];
+		a = ANY ? pb.sh_o[p] : pb.ray_o[p];
+		b = ANY ? pb.sh_d[p] : pb.ray_d[p];
+	};
+	auto done = [&](const kgr_hit &best, bool occ) {
+		if (ANY)
+			resolve_shadow(pb, p, occ);
+		else
+			pb.hit[p] = make_float4(__int_as_float(best.prim), best.t, best.b1, best.b2);
+	};
+	const uint32_t threads = gridDim.x * BLOCK;
+	if (LAYOUT == KGR_LAYOUT_FAST && !COUNT && s.coop_nodes && n <= pb.coop_rounds * (threads / 8u)) {
+		coop_walk<ANY>(s,
+			[&](bool need, float4 &a, float4 &b) {
+				/* one bit per group that needs a ray */
+				unsigned m = __ballot_sync(0xffffffffu, need) & 0x01010101u;
+				uint32_t base = 0;
+				if (lane == 0)
+					base = atomicAdd(fetch, (uint32_t)__popc(m));
+				base = __shfl_sync(0xffffffffu, base, 0);
+				uint32_t i = base + (uint32_t)__popc(m & ((1u << (lane & 24)) - 1u));
+				if (!need || i >= n)
+					return false;
+				load(i, a, b);
+				return true;
+			}, done);
+		return;
+	}
 	int32_t local_stack[KGR_STACK_DEPTH - SHORT];
 	typename StackOf<SHORT, BLOCK>::type stack(short_stack + threadIdx.x, local_stack);
-	int32_t ref = 0;
-	for (;;) {
-		bool need = !have && !exhausted;
-		unsigned m = __ballot_sync(0xffffffffu, need);
-		if (m) {
+	persistent_walk<ANY, COUNT, LAYOUT>(s, stack, 32, &cnt,
+		[&](bool need, float4 &a, float4 &b) {
+			unsigned m = __ballot_sync(0xffffffffu, need);
 			int leader = __ffs(m) - 1;
 			uint32_t base = 0;
 			if (lane == leader)
 				base = atomicAdd(fetch, (uint32_t)__popc(m));
 			base = __shfl_sync(0xffffffffu, base, leader);
-			if (need) {
-				uint32_t i = base + __popc(m & ((1u << lane) - 1u));
-				if (i < n) {
-					p = (ANY && !queue) ? i : queue[i];
-					float4 a = ANY ? pb.sh_o[p] : pb.ray_o[p];
-					float4 b = ANY ? pb.sh_d[p] : pb.ray_d[p];
-					r = fast_ray(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z));
-					best.prim = -1;
-					best.t = b.w;
-					best.b1 = 0.0f;
-					best.b2 = 0.0f;
-					best_rank = 0x7fffffff;
-					stack.clear();
-					ref = 0;
-					have = true;
-				} else {
-					exhausted = true;
-				}
-			}
-		}
-		if (!__any_sync(0xffffffffu, have))
-			break;
-		if (!have)
-			continue;
-		/* descend with the postponed-leaf rule (speculative_descend), then
-		 * test the leaves the descent collected */
-		int32_t leaf = 0;
-		speculative_descend<LAYOUT, COUNT>(s, r, ref, leaf, best.t, stack, &cnt);
-		bool occ = test_leaves<ANY, COUNT>(s, r, ref, leaf, best, best_rank, stack, &cnt);
-		bool done = occ || ref == KGR_REF_NONE;
-		if (done) {
-			if (ANY)
-				resolve_shadow(pb, p, occ);
-			else
-				pb.hit[p] = make_float4(__int_as_float(best.prim), best.t, best.b1, best.b2);
-			have = false;
-		}
-	}
+			uint32_t i = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
+			if (!need || i >= n)
+				return false;
+			load(i, a, b);
+			return true;
+		}, done);
 	if (COUNT)
 		add_visits(pb.visits + (ANY ? 2 : 0), cnt);
 }

@@ -272,6 +272,35 @@ __global__ void cw_nodes_kernel(const int32_t *__restrict__ kids, uint32_t nc, c
 	}
 }
 
+/* One slot of a cooperative node per thread: its child's padded box, and the
+ * reference from the compressed node's topology. */
+__global__ void coop_nodes_kernel(const int32_t *__restrict__ kids, uint32_t slots, const float4 *__restrict__ boxes,
+		const CwNode *__restrict__ cw, CoopNode *__restrict__ out)
+{
+	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) {
+		uint32_t c = i >> 3, j = i & 7u;
+		int32_t k = kids[i];
+		float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = make_float4(0.0f, 0.0f, __int_as_float(KGR_WIDE_EMPTY), 0.0f);
+		if (k >= 0) {
+			float mn[3], mx[3];
+			padded(boxes, k, mn, mx);
+			uint32_t imask = __float_as_uint(cw[c].origin.w) >> 24;
+			uint4 base = cw[c].base;
+			int32_t ref;
+			if ((imask >> j) & 1u) {
+				ref = (int32_t)(base.x + (uint32_t)__popc(imask & ((1u << j) - 1u)));
+			} else {
+				uint32_t meta = ((j < 4u ? base.z : base.w) >> (8u * (j & 3u))) & 0xffu;
+				ref = ~(int32_t)(((base.y + (meta & 31u)) << 3) | ((meta >> 5) - 1u));
+			}
+			a = make_float4(mn[0], mx[0], mn[1], mx[1]);
+			b = make_float4(mn[2], mx[2], __int_as_float(ref), 0.0f);
+		}
+		out[c].slot[2u * j] = a;
+		out[c].slot[2u * j + 1u] = b;
+	}
+}
+
 /* {v0, prim}, {v1 - v0}, {v2 - v0} in walk order; the primitive id stays */
 __global__ void triangle_records_kernel(uint32_t nt, const uint4 *__restrict__ tris, const float4 *__restrict__ pos,
 		float4 *rec)
@@ -344,6 +373,21 @@ void upload_plan(kgr_scene *sc)
 
 } /* namespace */
 
+void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, cudaStream_t st)
+{
+	static_assert(sizeof(CoopNode) == 256, "cooperative node size");
+	if (!sc->cw_node_count)
+		return;
+	sc->d_coop_nodes.alloc(sc->cw_node_count);
+	/* the walk reads a slot with one 32-byte vector load */
+	KGR_REQUIRE(((uintptr_t)sc->d_coop_nodes.ptr & 31) == 0, KGR_ERR_INTERNAL, "cooperative nodes misaligned");
+	size_t slots = 8 * (size_t)sc->cw_node_count;
+	KGR_REQUIRE(slots <= 0xffffffffu, KGR_ERR_UNSUPPORTED, "too many compressed nodes");
+	coop_nodes_kernel<<<grid_for(slots), REFIT_BLOCK, 0, st>>>(kids, (uint32_t)slots, boxes, sc->d_cw_nodes.ptr,
+		sc->d_coop_nodes.ptr);
+	KGR_CUDA(cudaGetLastError());
+}
+
 void refit_scene(kgr_scene *sc, int mode, const float *positions, const float *normals, cudaStream_t st)
 {
 	RefitPlan &pl = sc->plan;
@@ -397,6 +441,7 @@ void refit_scene(kgr_scene *sc, int mode, const float *positions, const float *n
 	if (sc->cw_node_count)
 		cw_nodes_kernel<<<grid_for(sc->cw_node_count), REFIT_BLOCK, 0, st>>>(d.cw_kids.ptr, sc->cw_node_count,
 			d.boxes.ptr, sc->d_cw_nodes.ptr);
+	coop_nodes(sc, d.cw_kids.ptr, d.boxes.ptr, st);
 	if (nt)
 		triangle_records_kernel<<<grid_for(nt), REFIT_BLOCK, 0, st>>>(nt, tris, pos, sc->d_fast_tris.ptr);
 	if (nt && sc->cw_node_count)

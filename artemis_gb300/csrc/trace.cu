@@ -89,6 +89,46 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_persistent_kernel(DeviceSce
 		});
 }
 
+/* The cooperative walk, eight lanes a ray; rays as above. */
+template <bool ANY>
+__global__ void __launch_bounds__(TRACE_BLOCK) trace_coop_kernel(DeviceScene s, const float4 *__restrict__ rays,
+		uint32_t n, kgr_hit *__restrict__ hits, uint32_t *__restrict__ occluded)
+{
+	__shared__ uint32_t taken;
+	if (threadIdx.x == 0)
+		taken = 0;
+	__syncthreads();
+	const int lane = threadIdx.x & 31, group = lane >> 3;
+	const uint32_t chunk = TRACE_BLOCK / 8;
+	uint32_t i = 0;
+	coop_walk<ANY>(s,
+		[&](bool need, float4 &a, float4 &b) {
+			/* one bit per group that needs a ray */
+			unsigned m = __ballot_sync(0xffffffffu, need) & 0x01010101u;
+			uint32_t base = 0;
+			if (lane == 0)
+				base = atomicAdd(&taken, (uint32_t)__popc(m));
+			base = __shfl_sync(0xffffffffu, base, 0);
+			if (!need)
+				return false;
+			uint32_t k = base + (uint32_t)__popc(m & ((1u << (8 * group)) - 1u));
+			uint32_t c = k / chunk;
+			uint64_t at = ((uint64_t)c * gridDim.x + blockIdx.x) * chunk + (k - c * chunk);
+			if (at >= n)
+				return false;
+			i = (uint32_t)at;
+			a = __ldg(&rays[2 * at]);
+			b = __ldg(&rays[2 * at + 1]);
+			return true;
+		},
+		[&](const kgr_hit &h, bool occ) {
+			if (ANY)
+				occluded[i] = occ ? 1u : 0u;
+			else
+				reinterpret_cast<float4 *>(hits)[i] = make_float4(__int_as_float(h.prim), h.t, h.b1, h.b2);
+		});
+}
+
 template <class K>
 int resident_blocks(K kernel, int block)
 {
@@ -105,6 +145,17 @@ void launch_trace_persistent(const DeviceScene &s, const float4 *rays, uint32_t 
 		cudaStream_t st)
 {
 	static const int resident = resident_blocks(trace_persistent_kernel<ANY, LAYOUT>, TRACE_BLOCK);
+	if (LAYOUT == KGR_LAYOUT_FAST && s.coop_nodes) {
+		/* up to KGR_COOP_ROUNDS rays for each of the resident groups */
+		static const int coop = resident_blocks(trace_coop_kernel<ANY>, TRACE_BLOCK);
+		const uint32_t groups = (uint32_t)coop * (TRACE_BLOCK / 8);
+		if (n <= KGR_COOP_ROUNDS * groups) {
+			const uint32_t blocks = (n + TRACE_BLOCK / 8 - 1) / (TRACE_BLOCK / 8);
+			trace_coop_kernel<ANY><<<blocks < (uint32_t)coop ? blocks : (uint32_t)coop, TRACE_BLOCK, 0, st>>>(s, rays,
+				n, hits, occluded);
+			return;
+		}
+	}
 	const uint32_t warps = (uint32_t)resident * (TRACE_BLOCK / 32);
 	/* Fewer rays than the resident lanes: every warp takes its share and the
 	 * rest of its lanes stay idle.  A warp's time is then the longest of a few

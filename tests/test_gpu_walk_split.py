@@ -26,3 +26,40 @@ def test_every_ray_is_walked_once(box, n, layout):
     rays[:, 7] = np.random.default_rng(n).uniform(0.0, 4.0, n)
     occ_ref, _ = osc.trace_any(rays)
     assert np.array_equal(sc.trace_any_host(rays, layout), occ_ref)
+
+
+def edge_rays(g, n):
+    """Zero direction components, NaN directions, origins far away and on the
+    scene's bounds, tmax 0, negative and NaN, among ordinary rays."""
+    rays = helpers.random_rays(g, n, 11)
+    rays[0::9, 4] = 0.0
+    rays[1::9, 5] = -0.0
+    rays[2::9, 4:6] = 0.0
+    rays[3::9, 6] = np.nan
+    rays[4::9, 0:3] -= 1000.0 * rays[4::9, 4:7]
+    rays[5::9, 0] = g.positions[:, 0].min()
+    rays[6::27, 7] = 0.0
+    rays[15::27, 7] = -1.0
+    rays[24::27, 7] = np.nan
+    return rays
+
+
+@pytest.mark.parametrize("n", [4000, 130000])
+def test_edge_rays_on_both_sides_of_the_split(box, n):
+    g, sc, _ = box
+    rays = edge_rays(g, n)
+    ref = sc.trace_closest_host(rays, kgr.LAYOUT_THREADED)
+    got = sc.trace_closest_host(rays)
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32))
+    assert np.array_equal(sc.trace_any_host(rays), sc.trace_any_host(rays, kgr.LAYOUT_THREADED))
+
+
+@pytest.mark.parametrize("scene,max_leaf", [("tiny", 4), ("box64", 1), ("box64", 8), ("terrain_s", 4)])
+def test_small_counts_on_every_tree(scene, max_leaf):
+    """A root of few children, one triangle a leaf, leaves too large for the
+    eight-child tree (the persistent walk takes the rays), a deep tree."""
+    g, sc, _ = helpers.both(scene, 2, max_leaf=max_leaf)
+    rays = np.concatenate([helpers.random_rays(g, 9001, 3), edge_rays(g, 999)])
+    ref = sc.trace_closest_host(rays, kgr.LAYOUT_THREADED)
+    assert np.array_equal(sc.trace_closest_host(rays).view(np.uint32), ref.view(np.uint32))
+    assert np.array_equal(sc.trace_any_host(rays), sc.trace_any_host(rays, kgr.LAYOUT_THREADED))
