@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) fast_persis
 	}
 	int32_t local_stack[KGR_STACK_DEPTH - SHORT];
 	typename StackOf<SHORT, BLOCK>::type stack(short_stack + threadIdx.x, local_stack);
-	persistent_walk<ANY, COUNT, LAYOUT>(s, stack, 32, &cnt,
+	persistent_walk<ANY, COUNT, LAYOUT>(s, stack, n >= KGR_REFILL_ROUNDS * threads ? KGR_REFILL_MANY : KGR_REFILL_FEW, &cnt,
 		[&](bool need, float4 &a, float4 &b) {
 			unsigned m = __ballot_sync(0xffffffffu, need);
 			int leader = __ffs(m) - 1;

@@ -1,8 +1,8 @@
 /*
  * trace.cu -- ray-buffer traversal kernels behind kgr_trace_closest and
  * kgr_trace_any: rays read as two 16-byte loads {o, unused} {d, tmax}, hits
- * written as one 16-byte store.  The fast and wide layouts run the
- * persistent walk; the threaded and compressed layouts one ray per thread.
+ * written as one 16-byte store.  One ray per thread, or, by the number of
+ * rays, eight lanes a ray or lanes that refill (launch_trace_persistent).
  */
 #include "kgr_device.cuh"
 #include "kgr_wavefront.h"
@@ -35,21 +35,30 @@ __global__ void __launch_bounds__(128) trace_rays_kernel(DeviceScene s, const fl
 }
 
 #define TRACE_BLOCK 128
+#define TRACE_CHUNK 64u
+/* between a bounce's best (31) and a camera ray's (8 to 20) */
+#define TRACE_REFILL 24
+
+/* The k-th ray of this block: it owns the chunks blockIdx, blockIdx + grid,
+ * blockIdx + 2 grid, ... of `chunk` consecutive rays.  Grows with k. */
+__device__ __forceinline__ uint64_t block_ray(uint32_t k, uint32_t chunk)
+{
+	uint32_t c = k / chunk;
+	return ((uint64_t)c * gridDim.x + blockIdx.x) * chunk + (k - c * chunk);
+}
 
 /* Bound by the latency of the node fetches (L2 and L1) and by the lanes of a
- * warp waiting for its longest walk.  Against one ray per thread over a
- * grid-stride loop: 2,073,600 bounce rays on the 1.16M-triangle terrain 1080
- * -> 878 us, 777,777 shadow rays on the 0.26M-triangle one 234 -> 199 us,
- * 4,096 camera rays on the box scene 72 -> 43 us.
- *
- * The fast and wide layouts: a resident grid whose lanes take the rays of
- * their block as they finish (persistent_walk).  Block b owns the chunks b,
- * b + grid, b + 2 grid, ... of `chunk` consecutive rays, handed out in order
- * by a counter in shared memory, so the call needs no device memory of its
- * own and calls may overlap on any streams. */
+ * warp waiting for its longest walk.  The fast and wide layouts with many rays:
+ * a resident grid whose lanes take the rays of their block as they finish
+ * (persistent_walk), handed out in order by a counter in shared memory, so the
+ * call needs no device memory of its own and calls may overlap on any streams.
+ * Against one ray per thread over a grid-stride loop, 2,073,600 rays on the
+ * box scene, the 0.26M- and the 1.16M-triangle terrain: bounce rays 1089, 857,
+ * 1084 -> 899, 718, 883 us, shadow rays 786, 539, 707 -> 562, 436, 554, camera
+ * rays 514, 374, 562 -> 572, 357, 483. */
 template <bool ANY, int LAYOUT>
 __global__ void __launch_bounds__(TRACE_BLOCK) trace_persistent_kernel(DeviceScene s, const float4 *__restrict__ rays,
-		uint32_t n, uint32_t chunk, int lanes, kgr_hit *__restrict__ hits, uint32_t *__restrict__ occluded)
+		uint32_t n, kgr_hit *__restrict__ hits, uint32_t *__restrict__ occluded)
 {
 	__shared__ uint32_t taken;
 	if (threadIdx.x == 0)
@@ -59,7 +68,7 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_persistent_kernel(DeviceSce
 	int32_t entries[KGR_STACK_DEPTH];
 	LocalStack stack(nullptr, entries);
 	uint32_t i = 0;
-	persistent_walk<ANY, false, LAYOUT>(s, stack, lanes, nullptr,
+	persistent_walk<ANY, false, LAYOUT>(s, stack, TRACE_REFILL, nullptr,
 		[&](bool need, float4 &a, float4 &b) {
 			unsigned m = __ballot_sync(0xffffffffu, need);
 			int leader = __ffs(m) - 1;
@@ -67,14 +76,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_persistent_kernel(DeviceSce
 			if (lane == leader)
 				base = atomicAdd(&taken, (uint32_t)__popc(m));
 			base = __shfl_sync(0xffffffffu, base, leader);
-			if (!need)
-				return false;
-			uint32_t k = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
-			uint32_t c = k / chunk;
-			/* a block asks at most once past its last chunk per lane, so this
-			 * stays far below 2^64; rays past the end are none */
-			uint64_t at = ((uint64_t)c * gridDim.x + blockIdx.x) * chunk + (k - c * chunk);
-			if (at >= n)
+			uint64_t at = block_ray(base + (uint32_t)__popc(m & ((1u << lane) - 1u)), TRACE_CHUNK);
+			if (!need || at >= n)
 				return false;
 			i = (uint32_t)at;
 			a = __ldg(&rays[2 * at]);
@@ -109,12 +112,8 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_coop_kernel(DeviceScene s, 
 			if (lane == 0)
 				base = atomicAdd(&taken, (uint32_t)__popc(m));
 			base = __shfl_sync(0xffffffffu, base, 0);
-			if (!need)
-				return false;
-			uint32_t k = base + (uint32_t)__popc(m & ((1u << (8 * group)) - 1u));
-			uint32_t c = k / chunk;
-			uint64_t at = ((uint64_t)c * gridDim.x + blockIdx.x) * chunk + (k - c * chunk);
-			if (at >= n)
+			uint64_t at = block_ray(base + (uint32_t)__popc(m & ((1u << (8 * group)) - 1u)), chunk);
+			if (!need || at >= n)
 				return false;
 			i = (uint32_t)at;
 			a = __ldg(&rays[2 * at]);
@@ -127,6 +126,16 @@ __global__ void __launch_bounds__(TRACE_BLOCK) trace_coop_kernel(DeviceScene s, 
 			else
 				reinterpret_cast<float4 *>(hits)[i] = make_float4(__int_as_float(h.prim), h.t, h.b1, h.b2);
 		});
+}
+
+int grid_for(uint32_t n, int block)
+{
+	int dev = 0, sms = 152;
+	cudaGetDevice(&dev);
+	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+	long long blocks = ((long long)n + block - 1) / block;
+	long long cap = (long long)sms * 16;
+	return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
 template <class K>
@@ -149,26 +158,21 @@ void launch_trace_persistent(const DeviceScene &s, const float4 *rays, uint32_t 
 		/* up to KGR_COOP_ROUNDS rays for each of the resident groups */
 		static const int coop = resident_blocks(trace_coop_kernel<ANY>, TRACE_BLOCK);
 		const uint32_t groups = (uint32_t)coop * (TRACE_BLOCK / 8);
-		if (n <= KGR_COOP_ROUNDS * groups) {
+		if (n <= KGR_COOP_ROUNDS_RAYS * groups) {
 			const uint32_t blocks = (n + TRACE_BLOCK / 8 - 1) / (TRACE_BLOCK / 8);
 			trace_coop_kernel<ANY><<<blocks < (uint32_t)coop ? blocks : (uint32_t)coop, TRACE_BLOCK, 0, st>>>(s, rays,
 				n, hits, occluded);
 			return;
 		}
 	}
-	const uint32_t warps = (uint32_t)resident * (TRACE_BLOCK / 32);
-	/* Fewer rays than the resident lanes: every warp takes its share and the
-	 * rest of its lanes stay idle.  A warp's time is then the longest of a few
-	 * walks, and the lanes that wait for one another's leaves are fewer:
-	 * 4,096 rays on the box scene 43 us at one lane a warp, 46 at 4, 55 at 8,
-	 * 63 at 16, 75 at 32.  Above warps x 32 rays the lanes are all in use and
-	 * refill. */
-	uint32_t lanes = (n + warps - 1) / warps;
-	lanes = lanes > 32 ? 32 : lanes;
-	const uint32_t chunk = lanes * (TRACE_BLOCK / 32);
-	const uint32_t chunks = (n + chunk - 1) / chunk;
-	const uint32_t grid = chunks < (uint32_t)resident ? chunks : (uint32_t)resident;
-	trace_persistent_kernel<ANY, LAYOUT><<<grid, TRACE_BLOCK, 0, st>>>(s, rays, n, chunk, (int)lanes, hits, occluded);
+	/* Few rays a lane: one ray per thread, as many blocks as it takes.  The
+	 * lanes hardly refill then, and the persistent walk's bookkeeping is 2 to
+	 * 7% of 77,000 to 200,000 rays (box scene and both terrains). */
+	if (n <= KGR_REFILL_ROUNDS * (uint32_t)resident * TRACE_BLOCK) {
+		trace_rays_kernel<ANY, LAYOUT><<<grid_for(n, TRACE_BLOCK), TRACE_BLOCK, 0, st>>>(s, rays, n, hits, occluded);
+		return;
+	}
+	trace_persistent_kernel<ANY, LAYOUT><<<resident, TRACE_BLOCK, 0, st>>>(s, rays, n, hits, occluded);
 }
 
 template <bool ANY>
@@ -193,16 +197,6 @@ __global__ void __launch_bounds__(128) trace_stats_kernel(DeviceScene s, const f
 		if ((threadIdx.x & 31) == 0)
 			atomicAdd(&counters[k], x);
 	}
-}
-
-int grid_for(uint32_t n, int block)
-{
-	int dev = 0, sms = 152;
-	cudaGetDevice(&dev);
-	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	long long blocks = ((long long)n + block - 1) / block;
-	long long cap = (long long)sms * 16;
-	return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
 __global__ void read_probe_kernel(const float4 *__restrict__ buf, size_t n, float4 *sink, int iters)
