@@ -87,3 +87,36 @@ def test_denoising_lowers_relmse():
     print(f"relMSE 4 spp: raw {raw:.4f}, denoised {den:.4f}")
     assert den < 0.5 * raw
     dn.close()
+
+
+@pytest.mark.parametrize("power", [0.0, 1.0, 2.0, 32.0, 63.5, 64.0, 1024.0])
+def test_every_normal_power_matches_oracle(power):
+    """Powers of two go by squaring, 64 by a loop of its own, others by powf."""
+    g, sc, _ = helpers.both("box4k", 1)
+    w, h = 37, 21
+    bufs = render_with_aovs(g, sc, w, h, 2, 3)
+    guides = kgr.DENOISE_NORMAL | kgr.DENOISE_POSITION
+    dn = kgr.Denoiser(w, h, guides)
+    dn.denoise(bufs[0].data_ptr(), bufs[1].data_ptr(), None, bufs[3].data_ptr(), iterations=3, normal_power=power)
+    torch.cuda.synchronize()
+    cpu = [b.cpu().numpy().reshape(h, w, 4) for b in bufs]
+    got = result_array(dn, w, h).reshape(h, w, 4)
+    ref = post_ref.denoise(cpu[0], cpu[1], cpu[2], cpu[3], guides, iterations=3, normal_power=power)
+    np.testing.assert_allclose(got, ref, rtol=1e-4, atol=1e-6)
+    dn.close()
+
+
+def test_infinite_and_nan_pixels_stay_where_they_are():
+    """A non-finite colour reaches only the taps of its own kind (hit or miss)."""
+    w, h = 33, 9
+    color = torch.rand((h, w, 4), device="cuda")
+    normal = torch.zeros((h, w, 4), device="cuda")
+    normal[:, :16, 2] = 1.0
+    color[4, 20, 0], color[2, 25, 1] = float("nan"), float("inf")
+    dn = kgr.Denoiser(w, h, kgr.DENOISE_NORMAL)
+    dn.denoise(color.data_ptr(), normal.data_ptr(), iterations=2)
+    torch.cuda.synchronize()
+    got = result_array(dn, w, h).reshape(h, w, 4)
+    assert np.isfinite(got[:, :16]).all()
+    assert np.isnan(got[4, 20, 0]) and not np.isfinite(got[2, 25, 1])
+    dn.close()
