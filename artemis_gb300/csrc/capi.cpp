@@ -292,8 +292,8 @@ uint32_t tree_depth(const Tree &t)
 	return best;
 }
 
-/* The tree half of the refit plan: nodes, primitive order, nodes grouped by
- * depth (deepest first, so a level's children are done before it). */
+/* The tree half of the refit plan: nodes and their parents, the leaves,
+ * primitive order. */
 void plan_tree(RefitPlan &pl, const Tree &tree, std::vector<int32_t> &&rec_node)
 {
 	size_t n = tree.nodes.size();
@@ -304,25 +304,23 @@ void plan_tree(RefitPlan &pl, const Tree &tree, std::vector<int32_t> &&rec_node)
 	}
 	pl.prim_order = tree.prim_order;
 	pl.rec_node = std::move(rec_node);
-	std::vector<std::vector<uint32_t>> levels;
-	if (n) {
-		std::vector<uint32_t> cur(1, 0u), next;
-		while (!cur.empty()) {
-			levels.push_back(cur);
-			next.clear();
-			for (uint32_t i : cur)
-				if (!tree.nodes[i].count) {
-					next.push_back((uint32_t)tree.nodes[i].left);
-					next.push_back((uint32_t)tree.nodes[i].right);
-				}
-			cur.swap(next);
+	pl.parent.assign(n, -1);
+	pl.leaves.clear();
+	std::vector<int32_t> todo;
+	if (n)
+		todo.push_back(0);
+	while (!todo.empty()) {
+		int32_t i = todo.back();
+		todo.pop_back();
+		const TreeNode &t = tree.nodes[i];
+		if (t.count) {
+			pl.leaves.push_back((uint32_t)i);
+			continue;
 		}
-	}
-	pl.level_order.clear();
-	pl.level_begin.assign(1, 0u);
-	for (size_t l = levels.size(); l-- > 0;) {
-		pl.level_order.insert(pl.level_order.end(), levels[l].begin(), levels[l].end());
-		pl.level_begin.push_back((uint32_t)pl.level_order.size());
+		pl.parent[t.left] = pl.parent[t.right] = i;
+		/* the left subtree's leaves first: neighbours in space */
+		todo.push_back(t.right);
+		todo.push_back(t.left);
 	}
 }
 
@@ -384,7 +382,7 @@ void finish_scene(kgr_scene *sc, const Tree &tree, const std::vector<PrimBox> &b
 		DevBuf<int32_t> d_kids;
 		d_boxes.upload(tree_boxes);
 		d_kids.upload(sc->plan.cw_kids);
-		coop_nodes(sc, d_kids.ptr, d_boxes.ptr, 0);
+		coop_nodes(sc, d_kids.ptr, d_boxes.ptr, false, 0);
 		/* the scene may be traced on any stream from here on, and the two
 		 * uploads are released */
 		KGR_CUDA(cudaStreamSynchronize(0));

@@ -302,8 +302,8 @@ struct RefitPlan {
 	 * prim_order[first, first + count) */
 	std::vector<int4> nodes;
 	std::vector<uint32_t> prim_order;
-	std::vector<uint32_t> level_order; /* node ids, deepest level first */
-	std::vector<uint32_t> level_begin; /* level l = level_order[level_begin[l], level_begin[l + 1]) */
+	std::vector<int32_t> parent;       /* tree node -> its parent (-1: the root, or not in the tree) */
+	std::vector<uint32_t> leaves;      /* the tree's leaves, left to right */
 	std::vector<int32_t> rec_node;     /* threaded record -> node, ~prim for leaf records */
 	std::vector<int2> fast_kids;       /* fast node -> its two child nodes (-1: none) */
 	std::vector<int4> wide_kids;       /* wide node -> its child nodes (-1: empty slot) */
@@ -316,7 +316,9 @@ struct RefitPlan {
 struct RefitDevice {
 	bool ready = false;
 	DevBuf<float4> obj_positions, obj_normals, boxes;
-	DevBuf<uint32_t> vertex_mesh, light_tri, prim_order, level_order;
+	DevBuf<uint32_t> vertex_mesh, light_tri, prim_order, leaves;
+	DevBuf<uint32_t> arrived; /* per tree node: children that have come by, over all refits */
+	DevBuf<int32_t> parent;
 	DevBuf<int32_t> normal_src, has_model, rec_node;
 	DevBuf<float> models;
 	DevBuf<int4> nodes, wide_kids;
@@ -433,8 +435,9 @@ void refit_scene(kgr_scene *sc, int mode, const float *positions, const float *n
 
 /* The cooperative walk's nodes from the compressed ones (topology) and the
  * tree's boxes (2 float4 per tree node) and slots (8 per compressed node, -1
- * empty), all on the device (refit.cu). */
-void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, cudaStream_t st);
+ * empty), all on the device (refit.cu).  requantise: the compressed nodes'
+ * grids and planes from the boxes too. */
+void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, bool requantise, cudaStream_t st);
 
 /* Traversal of a ray buffer (8 floats per ray) into hits or occlusion flags. */
 void launch_trace_closest(const DeviceScene &s, const float4 *rays, uint32_t n,

@@ -15,7 +15,7 @@
  *   2. face normals of meshes created without normals (the triangle that
  *      gathered the vertex last, as scene creation does);
  *   3. triangle lights {a, b - a, c - a} of their triangles;
- *   4. tree-node boxes, one launch per tree level from the deepest: a leaf
+ *   4. tree-node boxes, one launch that climbs from the leaves: a leaf
  *      is the union of its triangles' boxes (min(p1, min(p2, p3)) per axis,
  *      zeros made +0), an inner node the union of its two children.  With
  *      canonical zeros min and max are functions of the set of values, so
@@ -24,11 +24,10 @@
  *      triangle box of Submesh::bvh, include/mesh.hpp:48-78), the padded
  *      child boxes of the fast and wide nodes, and the walk-ordered
  *      triangle records.  Headers, links and references are not touched.
- * Every kernel is a grid-stride loop over independent items; nothing waits.
+ * Nothing waits: every other kernel is a loop over independent items.
  */
 #include <float.h>
 
-#include "kgr_cw8.h"
 #include "kgr_internal.h"
 #include "kgr_wavefront.h"
 
@@ -134,35 +133,57 @@ __device__ __forceinline__ void triangle_box(const uint4 *tris, const float4 *po
 	mx[2] = gmax_d(a.z, gmax_d(b.z, c.z));
 }
 
-__global__ void node_boxes_kernel(const uint32_t *__restrict__ ids, uint32_t n, const int4 *__restrict__ nodes,
-		const uint32_t *__restrict__ prim_order, const uint4 *__restrict__ tris, const float4 *__restrict__ pos,
-		float4 *boxes)
+/* All boxes of the tree in one launch: a thread takes a leaf, writes its box
+ * and climbs.  At each node the first of its two children to arrive ends there;
+ * the second finds both boxes written, unites them and goes on, so nothing
+ * waits.  Every refit adds two arrivals to a node, so the parity of the count
+ * tells first from second and nothing is reset.  The union takes the left child
+ * first whichever arrives last.
+ *
+ * Bound by the chain of an atomic and two box loads a level (27 levels on the
+ * 1.16M-triangle terrain) and the gathers of the vertices.  One launch a level,
+ * most of them far below a full GPU: 215 us; this one 110 (137 with a fence on
+ * each side of the atomic, which empties L1 more often). */
+__global__ void __launch_bounds__(REFIT_BLOCK) tree_boxes_kernel(const uint32_t *__restrict__ leaves, uint32_t n,
+		const int4 *__restrict__ nodes, const int32_t *__restrict__ parent, const uint32_t *__restrict__ prim_order,
+		const uint4 *__restrict__ tris, const float4 *__restrict__ pos, uint32_t *arrived, float4 *boxes)
 {
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-		uint32_t id = ids[i];
-		int4 nd = nodes[id];
-		float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-		if (nd.w > 0) {
-			for (int k = 0; k < nd.w; k++) {
-				float tmn[3], tmx[3];
-				triangle_box(tris, pos, prim_order[nd.z + k], tmn, tmx);
-				for (int a = 0; a < 3; a++) {
-					mn[a] = gmin_d(mn[a], tmn[a] + 0.0f); /* +0.0f: -0 -> +0 */
-					mx[a] = gmax_d(mx[a], tmx[a] + 0.0f);
-				}
-			}
-		} else {
-			float4 l0 = boxes[2 * (size_t)nd.x], l1 = boxes[2 * (size_t)nd.x + 1];
-			float4 r0 = boxes[2 * (size_t)nd.y], r1 = boxes[2 * (size_t)nd.y + 1];
-			mn[0] = gmin_d(l0.x, r0.x);
-			mn[1] = gmin_d(l0.y, r0.y);
-			mn[2] = gmin_d(l0.z, r0.z);
-			mx[0] = gmax_d(l1.x, r1.x);
-			mx[1] = gmax_d(l1.y, r1.y);
-			mx[2] = gmax_d(l1.z, r1.z);
+	uint32_t i = blockIdx.x * REFIT_BLOCK + threadIdx.x;
+	if (i >= n)
+		return;
+	int32_t id = (int32_t)leaves[i];
+	int4 nd = nodes[id];
+	float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+	for (int k = 0; k < nd.w; k++) {
+		float tmn[3], tmx[3];
+		triangle_box(tris, pos, prim_order[nd.z + k], tmn, tmx);
+		for (int a = 0; a < 3; a++) {
+			mn[a] = gmin_d(mn[a], tmn[a] + 0.0f); /* +0.0f: -0 -> +0 */
+			mx[a] = gmax_d(mx[a], tmx[a] + 0.0f);
 		}
-		boxes[2 * (size_t)id] = make_float4(mn[0], mn[1], mn[2], 0.0f);
-		boxes[2 * (size_t)id + 1] = make_float4(mx[0], mx[1], mx[2], 0.0f);
+	}
+	for (;;) {
+		__stcg(&boxes[2 * (size_t)id], make_float4(mn[0], mn[1], mn[2], 0.0f));
+		__stcg(&boxes[2 * (size_t)id + 1], make_float4(mx[0], mx[1], mx[2], 0.0f));
+		int32_t up = parent[id];
+		if (up < 0)
+			return;
+		/* releases this child's box and acquires the other one's */
+		uint32_t before;
+		asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(&arrived[up]) : "memory");
+		if ((before & 1u) == 0u)
+			return;
+		/* this child's box is at hand; the other one's comes from L2 */
+		nd = nodes[up];
+		const bool left = nd.x == id;
+		const size_t o = 2 * (size_t)(left ? nd.y : nd.x);
+		const float4 lo = __ldcg(&boxes[o]), hi = __ldcg(&boxes[o + 1]);
+		const float omn[3] = {lo.x, lo.y, lo.z}, omx[3] = {hi.x, hi.y, hi.z};
+		for (int a = 0; a < 3; a++) {
+			mn[a] = left ? gmin_d(mn[a], omn[a]) : gmin_d(omn[a], mn[a]);
+			mx[a] = left ? gmax_d(mx[a], omx[a]) : gmax_d(omx[a], mx[a]);
+		}
+		id = up;
 	}
 }
 
@@ -245,46 +266,102 @@ __global__ void wide_nodes_kernel(const int4 *__restrict__ kids, uint32_t nw, co
 	}
 }
 
-/* The compressed nodes requantised from their children's refitted boxes by
- * the host builder's own rules (kgr_cw8.h): same slots, same child and
- * triangle bases, new grid and planes. */
-__global__ void cw_nodes_kernel(const int32_t *__restrict__ kids, uint32_t nc, const float4 *__restrict__ boxes,
-		CwNode *nodes)
+/* The difference of two floats as a double holds it: d + e with |e| at most
+ * half an ulp of d, and e dropped where a double has no bit for it. */
+__device__ __forceinline__ void exact_diff(float a, float b, float &d, float &e)
 {
-	for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nc; c += gridDim.x * blockDim.x) {
-		float lo[8][3], hi[8][3];
-		uint32_t used = 0;
-		for (int j = 0; j < 8; j++) {
-			int32_t k = kids[8 * (size_t)c + j];
-			for (int a = 0; a < 3; a++) {
-				lo[j][a] = 0.0f;
-				hi[j][a] = 0.0f;
-			}
-			if (k < 0)
-				continue;
-			used |= 1u << j;
-			padded(boxes, k, lo[j], hi[j]);
-		}
-		CwNode n = nodes[c];
-		uint32_t imask = __float_as_uint(n.origin.w) >> 24;
-		cw_quantize(lo, hi, used, imask, n.origin, n.qa, n.qb, n.qc);
-		nodes[c] = n;
-	}
+	d = a - b;
+	float t = d - a;
+	e = (a - (d - t)) - (b + t);
+	if (fabsf(e) <= fabsf(d) * 5.5511151e-17f) /* 2^-54 */
+		e = 0.0f;
 }
 
-/* One slot of a cooperative node per thread: its child's padded box, and the
- * reference from the compressed node's topology. */
-__global__ void coop_nodes_kernel(const int32_t *__restrict__ kids, uint32_t slots, const float4 *__restrict__ boxes,
-		const CwNode *__restrict__ cw, CoopNode *__restrict__ out)
+__device__ __forceinline__ float pow2i(int k) { return ldexpf(1.0f, k); }
+
+/* cw_axis_grid of kgr_cw8.h: the same exponent and origin with all but one
+ * operation in single precision (the origin's rounding, which has to see the
+ * double). */
+__device__ __forceinline__ void axis_grid(float lo, float hi, int &e, float &p)
 {
-	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < slots; i += gridDim.x * blockDim.x) {
-		uint32_t c = i >> 3, j = i & 7u;
-		int32_t k = kids[i];
+	float d, r;
+	exact_diff(hi, lo, d, r);
+	int k = -126;
+	if (d > 0.0f) {
+		/* the least k with 253 2^k >= the extent */
+		int x;
+		frexpf(d, &x);
+		k = max(x - 9, -126);
+		while (k < 127) {
+			float m = 253.0f * pow2i(k);
+			if (d < m || (d == m && r <= 0.0f))
+				break;
+			k++;
+		}
+	}
+	for (; k < 127; k++) {
+		p = __double2float_rd((double)lo - (double)pow2i(k));
+		exact_diff(hi, p, d, r);
+		float m = 254.5f * pow2i(k);
+		if (d < m || (d == m && r <= 0.0f))
+			break;
+	}
+	if (k >= 127) {
+		k = 127;
+		p = __double2float_rd((double)lo - (double)pow2i(127));
+	}
+	e = k;
+}
+
+/* cw_qlo and cw_qhi: floor((plane - p) / 2^e - 1/2) and ceil(.. + 1/2), from the
+ * whole part f and the rest r (exact) of the quotient and the sign of what the
+ * difference lost. */
+__device__ __forceinline__ uint32_t plane_lo(float plane, float p, int e)
+{
+	float d, t;
+	exact_diff(plane, p, d, t);
+	float x = ldexpf(d, -e), f = floorf(x), r = x - f;
+	float q = (r > 0.5f || (r == 0.5f && t >= 0.0f)) ? f : f - 1.0f;
+	return (uint32_t)fminf(fmaxf(q, 0.0f), 255.0f);
+}
+
+__device__ __forceinline__ uint32_t plane_hi(float plane, float p, int e)
+{
+	float d, t;
+	exact_diff(plane, p, d, t);
+	float x = ldexpf(d, -e), f = floorf(x), r = x - f;
+	float q = (r > 0.5f || (r == 0.5f && t > 0.0f)) ? f + 2.0f : f + 1.0f;
+	return (uint32_t)fminf(fmaxf(q, 0.0f), 255.0f);
+}
+
+/* The slots of the eight-child nodes, one a thread, eight lanes a node: the
+ * cooperative node's padded box and reference (the reference from the
+ * compressed node's topology), and with QUANT the compressed node's grid and
+ * planes, requantised from its children's boxes by the host builder's rules
+ * (kgr_cw8.h): same slots, same child and triangle bases.
+ *
+ * Bound by the gathers of the boxes.  One thread a node in double precision,
+ * its eight boxes in local memory: 420 us for the 1.16M-triangle terrain's
+ * 196,000 nodes, and the cooperative nodes 20 us; this kernel 36 us for both. */
+template <bool QUANT>
+__global__ void __launch_bounds__(REFIT_BLOCK) slot_nodes_kernel(const int32_t *__restrict__ kids, uint32_t slots,
+		const float4 *__restrict__ boxes, CwNode *__restrict__ cw, CoopNode *__restrict__ out)
+{
+	const unsigned full = 0xffffffffu;
+	const int gs = threadIdx.x & 24;
+	const uint32_t stride = gridDim.x * REFIT_BLOCK;
+	/* whole warps iterate: the bound is the same for a warp's lanes */
+	for (uint32_t i = blockIdx.x * REFIT_BLOCK + threadIdx.x; (i & ~31u) < slots; i += stride) {
+		const bool in = i < slots;
+		const uint32_t c = i >> 3, j = i & 7u;
+		const int32_t k = in ? kids[i] : -1;
+		float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+		uint32_t imask = 0u;
+		if (in)
+			imask = __float_as_uint(cw[c].origin.w) >> 24;
 		float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = make_float4(0.0f, 0.0f, __int_as_float(KGR_WIDE_EMPTY), 0.0f);
 		if (k >= 0) {
-			float mn[3], mx[3];
 			padded(boxes, k, mn, mx);
-			uint32_t imask = __float_as_uint(cw[c].origin.w) >> 24;
 			uint4 base = cw[c].base;
 			int32_t ref;
 			if ((imask >> j) & 1u) {
@@ -296,8 +373,45 @@ __global__ void coop_nodes_kernel(const int32_t *__restrict__ kids, uint32_t slo
 			a = make_float4(mn[0], mx[0], mn[1], mx[1]);
 			b = make_float4(mn[2], mx[2], __int_as_float(ref), 0.0f);
 		}
-		out[c].slot[2u * j] = a;
-		out[c].slot[2u * j + 1u] = b;
+		if (in) {
+			out[c].slot[2u * j] = a;
+			out[c].slot[2u * j + 1u] = b;
+		}
+		if (!QUANT)
+			continue;
+		float lo[3], hi[3];
+		for (int x = 0; x < 3; x++) {
+			lo[x] = mn[x];
+			hi[x] = mx[x];
+			for (int o = 1; o < 8; o <<= 1) {
+				float l = __shfl_xor_sync(full, lo[x], o), h = __shfl_xor_sync(full, hi[x], o);
+				lo[x] = l < lo[x] ? l : lo[x];
+				hi[x] = h > hi[x] ? h : hi[x];
+			}
+			if (!(lo[x] <= hi[x]))
+				lo[x] = hi[x] = 0.0f; /* a node without children */
+		}
+		/* lanes 0, 1 and 2 of a group find the grid of one axis each */
+		int e;
+		float p;
+		axis_grid(j == 0u ? lo[0] : (j == 1u ? lo[1] : lo[2]), j == 0u ? hi[0] : (j == 1u ? hi[1] : hi[2]), e, p);
+		int ex[3];
+		float px[3];
+		for (int x = 0; x < 3; x++) {
+			ex[x] = __shfl_sync(full, e, gs + x);
+			px[x] = __shfl_sync(full, p, gs + x);
+		}
+		if (!in)
+			continue;
+		/* planes: lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, a byte a slot */
+		uint8_t *q = reinterpret_cast<uint8_t *>(&cw[c].qa) + j;
+		for (int x = 0; x < 3; x++) {
+			q[8 * x] = (uint8_t)(k >= 0 ? plane_lo(mn[x], px[x], ex[x]) : 255u);
+			q[24 + 8 * x] = (uint8_t)(k >= 0 ? plane_hi(mx[x], px[x], ex[x]) : 0u);
+		}
+		if (j == 0u)
+			cw[c].origin = make_float4(px[0], px[1], px[2], __uint_as_float((uint32_t)(ex[0] + 127) |
+				(uint32_t)(ex[1] + 127) << 8 | (uint32_t)(ex[2] + 127) << 16 | imask << 24));
 	}
 }
 
@@ -362,7 +476,11 @@ void upload_plan(kgr_scene *sc)
 	upload_vec(d.light_tri, pl.light_tri);
 	upload_vec(d.nodes, pl.nodes);
 	upload_vec(d.prim_order, pl.prim_order);
-	upload_vec(d.level_order, pl.level_order);
+	upload_vec(d.leaves, pl.leaves);
+	upload_vec(d.parent, pl.parent);
+	d.arrived.alloc(pl.nodes.size());
+	if (!pl.nodes.empty())
+		KGR_CUDA(cudaMemset(d.arrived.ptr, 0, d.arrived.bytes()));
 	upload_vec(d.rec_node, pl.rec_node);
 	upload_vec(d.fast_kids, pl.fast_kids);
 	upload_vec(d.wide_kids, pl.wide_kids);
@@ -373,7 +491,7 @@ void upload_plan(kgr_scene *sc)
 
 } /* namespace */
 
-void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, cudaStream_t st)
+void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, bool requantise, cudaStream_t st)
 {
 	static_assert(sizeof(CoopNode) == 256, "cooperative node size");
 	if (!sc->cw_node_count)
@@ -383,7 +501,8 @@ void coop_nodes(kgr_scene *sc, const int32_t *kids, const float4 *boxes, cudaStr
 	KGR_REQUIRE(((uintptr_t)sc->d_coop_nodes.ptr & 31) == 0, KGR_ERR_INTERNAL, "cooperative nodes misaligned");
 	size_t slots = 8 * (size_t)sc->cw_node_count;
 	KGR_REQUIRE(slots <= 0xffffffffu, KGR_ERR_UNSUPPORTED, "too many compressed nodes");
-	coop_nodes_kernel<<<grid_for(slots), REFIT_BLOCK, 0, st>>>(kids, (uint32_t)slots, boxes, sc->d_cw_nodes.ptr,
+	auto kernel = requantise ? slot_nodes_kernel<true> : slot_nodes_kernel<false>;
+	kernel<<<grid_for(slots), REFIT_BLOCK, 0, st>>>(kids, (uint32_t)slots, boxes, sc->d_cw_nodes.ptr,
 		sc->d_coop_nodes.ptr);
 	KGR_CUDA(cudaGetLastError());
 }
@@ -422,11 +541,10 @@ void refit_scene(kgr_scene *sc, int mode, const float *positions, const float *n
 		face_normals_kernel<<<grid_for(nv), REFIT_BLOCK, 0, st>>>(d.normal_src.ptr, tris, pos, nv, nrm);
 	if (nl)
 		lights_kernel<<<grid_for(nl), REFIT_BLOCK, 0, st>>>(d.light_tri.ptr, tris, pos, nl, sc->d_lights.ptr);
-	for (size_t l = 0; l + 1 < pl.level_begin.size(); l++) {
-		uint32_t b = pl.level_begin[l], e = pl.level_begin[l + 1];
-		if (e > b)
-			node_boxes_kernel<<<grid_for(e - b), REFIT_BLOCK, 0, st>>>(d.level_order.ptr + b, e - b,
-				d.nodes.ptr, d.prim_order.ptr, tris, pos, d.boxes.ptr);
+	if (!pl.leaves.empty()) {
+		uint32_t n = (uint32_t)pl.leaves.size();
+		tree_boxes_kernel<<<(n + REFIT_BLOCK - 1) / REFIT_BLOCK, REFIT_BLOCK, 0, st>>>(d.leaves.ptr, n, d.nodes.ptr,
+			d.parent.ptr, d.prim_order.ptr, tris, pos, d.arrived.ptr, d.boxes.ptr);
 	}
 	uint32_t nrec = (uint32_t)pl.rec_node.size();
 	if (nrec)
@@ -438,10 +556,7 @@ void refit_scene(kgr_scene *sc, int mode, const float *positions, const float *n
 	if (sc->wide_node_count)
 		wide_nodes_kernel<<<grid_for(sc->wide_node_count), REFIT_BLOCK, 0, st>>>(d.wide_kids.ptr,
 			sc->wide_node_count, d.boxes.ptr, sc->d_wide_nodes.ptr);
-	if (sc->cw_node_count)
-		cw_nodes_kernel<<<grid_for(sc->cw_node_count), REFIT_BLOCK, 0, st>>>(d.cw_kids.ptr, sc->cw_node_count,
-			d.boxes.ptr, sc->d_cw_nodes.ptr);
-	coop_nodes(sc, d.cw_kids.ptr, d.boxes.ptr, st);
+	coop_nodes(sc, d.cw_kids.ptr, d.boxes.ptr, true, st);
 	if (nt)
 		triangle_records_kernel<<<grid_for(nt), REFIT_BLOCK, 0, st>>>(nt, tris, pos, sc->d_fast_tris.ptr);
 	if (nt && sc->cw_node_count)
