@@ -6,42 +6,48 @@
  * BF16 or FP16 weights and activations, FP32 accumulation); this kernel is
  * an alternative to its mma.sync inference and computes the same function.
  *
- * A CTA of four warpgroups (512 threads) holds the weights once and runs
- * four independent chains, one a warpgroup, each walking tiles of 128 rows
- * (the MMA's M) with its own buffer, barriers and accumulator; two CTAs fit
- * an SM, so eight tiles move through the network on an SM at once and the
- * 512 TMEM columns are all in use:
+ * A CTA of five warpgroups (640 threads), one an SM, holds the weights once and
+ * runs five independent chains, one a warpgroup, each walking tiles of 128 rows
+ * (the MMA's M) with its own input buffer, barriers and accumulator:
  *   weights        the six layers (B operands, N x K) in shared memory in
  *                  the canonical K-major layout without swizzle: 8 x 8 core
  *                  matrices of 128 contiguous bytes, K neighbours 128 bytes
  *                  apart (leading byte offset), 8-row groups 1024 bytes apart
  *                  (stride byte offset);
- *   activations    one 128 x 64 tile (A operand) a chain in the K-major
- *                  layout with the 128-byte swizzle: row r at r x 128 bytes,
- *                  its 16-byte chunk c at chunk c ^ (r mod 8).  A tile
- *                  arrives by one TMA load (cp.async.bulk.tensor.2d, the
+ *   input          one 128 x 64 tile (the first layer's A operand) a chain in
+ *                  the K-major layout with the 128-byte swizzle: row r at r x
+ *                  128 bytes, its 16-byte chunk c at chunk c ^ (r mod 8).  A
+ *                  tile arrives by one TMA load (cp.async.bulk.tensor.2d, the
  *                  tensor map's 128-byte swizzle writes exactly this layout;
  *                  rows past the end read as zero); the chain's next tile is
- *                  loaded into the same buffer as soon as the last layer's
- *                  MMA has read it, while the outputs are read back;
- *   TMEM           a 128-lane x 64-column FP32 accumulator a chain (columns
- *                  64 c .. 64 c + 63), row i in lane i; a warp reads lanes
- *                  32 (warp mod 4) .. +31;
+ *                  loaded into the same buffer as soon as the first layer's
+ *                  MMA has read it, and arrives under the other five layers;
+ *   TMEM           96 columns a chain: the activations (32 columns, two halves
+ *                  a column, row i in lane i: the A operand of every layer
+ *                  after the first) and the FP32 accumulator (64 columns); a
+ *                  warp reads and writes lanes 32 (warp mod 4) .. +31;
  *   per layer      one thread of the chain issues four tcgen05.mma (K = 16
- *                  each; the A start address advances 32 bytes inside the
- *                  swizzled row) and a tcgen05.commit to the chain's
- *                  mbarrier; after it every warp of the chain reads its 32
- *                  lanes with tcgen05.ld (32x32b, two halves of 32 columns),
- *                  applies ReLU, rounds to half precision and writes the row
- *                  back into the tile, swizzled, as the next layer's A
- *                  operand; the chain's 128 threads meet at a named barrier
- *                  (1 + chain).
+ *                  each) and a tcgen05.commit to the chain's mbarrier; after it
+ *                  every warp of the chain reads its 32 lanes with tcgen05.ld,
+ *                  rounds to half precision, applies ReLU and writes the next
+ *                  layer's A operand with tcgen05.st; the chain's 128 threads
+ *                  meet at a named barrier (1 + chain).
+ *
+ * Activations in TMEM are what the five chains buy: written back to shared
+ * memory they cost a tile 16 KB of stores and 16 KB of operand reads a layer
+ * beside the weights' 8 KB, and that bandwidth was the limit (four chains in
+ * each of two CTAs an SM: 129 us for 2.07M rows; this kernel 81 us, 0.54 of the
+ * measured BF16 peak).  What is left is the latency of a layer (issue, MMA,
+ * commit, read, write, barrier), so every instruction on that path counts: a
+ * ReLU of its own beside the conversion 106 against 93 us, the six layers
+ * unrolled 102 -> 81 us; four chains 93 us.  Two MMAs of N = 32 a layer, the
+ * first half's epilogue under the second's MMA: 139 us.
  *
  * Every wait on an mbarrier is bounded.  A wait that runs out sets bit 0 of
- * the error word; the chain stops at the next layer boundary (the decision
- * is taken by all its threads together), waits (bounded) for its TMA load in
- * flight, and the block frees its TMEM and returns; the host reads the word with
- * kgr_mlp_check.  kgr_mlp_test_wait_timeout exercises that path: its launch
+ * the error word; the chain stops at the next layer boundary (the barrier there
+ * takes the decision for all its threads together), waits (bounded) for its TMA
+ * load in flight, and the block frees its TMEM and returns; the host reads the
+ * word with kgr_mlp_check.  kgr_mlp_test_wait_timeout exercises that path: its launch
  * withholds each block's first load, so the wait on it runs out (after
  * TC_WAIT_TEST_LIMIT polls) before any MMA was issued.
  */
@@ -67,14 +73,15 @@ namespace {
 #define TC_SBO 1024u                /* bytes between 8-row groups (64-wide K) */
 #define TC_LAYER_BYTES 8192u        /* 64 x 64 half-precision weights */
 #define TC_W_BYTES (5u * TC_LAYER_BYTES + 2048u)
-#define TC_CHAINS 4                 /* warpgroups a CTA, each walking tiles of its own */
+#define TC_CHAINS 5                 /* warpgroups a CTA, each walking tiles of its own */
 #define TC_THREADS (128 * TC_CHAINS)
 #define TC_X_OFF 43008u             /* = TC_W_BYTES, a multiple of 1024 (swizzle atom) */
 #define TC_X_BYTES (TC_ROWS * TC_W * 2u)
 #define TC_BAR_OFF (TC_X_OFF + TC_CHAINS * TC_X_BYTES)  /* per chain: MMA barrier, TMA barrier */
 #define TC_SLOT_OFF (TC_BAR_OFF + TC_CHAINS * 16u)
-#define TC_SMEM (TC_SLOT_OFF + 8u)  /* 108,616 bytes: two CTAs fit an SM */
-#define TC_TMEM_COLS 256u           /* 64 columns a chain, rounded up to a power of two */
+#define TC_SMEM (TC_SLOT_OFF + 8u)  /* 125,016 bytes: one CTA an SM */
+#define TC_CHAIN_COLS 96u           /* 32 of activations, 64 of accumulator */
+#define TC_TMEM_COLS 512u           /* 5 x 96, rounded up to a power of two */
 #define TC_WAIT_LIMIT (1u << 24)    /* mbarrier polls before a wait gives up */
 #define TC_WAIT_TEST_LIMIT (1u << 16) /* the same, in a launch that tests the give-up path */
 
@@ -83,13 +90,6 @@ namespace {
 __device__ __forceinline__ uint32_t core_off(uint32_t r, uint32_t k)
 {
 	return (r >> 3) * TC_SBO + (k >> 3) * TC_LBO + (r & 7u) * 16u + (k & 7u) * 2u;
-}
-
-/* Byte offset of the 16-byte chunk c of row r of a 128-byte-swizzled tile
- * (the activations). */
-__device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c)
-{
-	return r * 128u + ((c ^ (r & 7u)) << 4);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p)
@@ -132,13 +132,8 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-/* Barrier of one chain's 128 threads (named barrier 1 + chain; 0 is the
- * CTA's), and the same with an AND over a flag of every thread. */
-__device__ __forceinline__ void chain_sync(int chain)
-{
-	asm volatile("bar.sync %0, 128;" :: "r"(chain + 1) : "memory");
-}
-
+/* Barrier of one chain's 128 threads (named barrier 1 + chain; 0 is the CTA's)
+ * with an AND over a flag of every thread. */
 __device__ __forceinline__ bool chain_and(int chain, bool v)
 {
 	uint32_t r;
@@ -160,6 +155,17 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, ui
 		"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
 		"}"
 		:: "r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
+}
+
+/* The same with the A operand in tensor memory. */
+__device__ __forceinline__ void tc_mma_ts(uint32_t tmem, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+	asm volatile(
+		"{\n\t.reg .pred p;\n\t"
+		"setp.ne.b32 p, %4, 0;\n\t"
+		"tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+		"}"
+		:: "r"(tmem), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
 }
 
 __device__ __forceinline__ void tc_commit(uint32_t bar)
@@ -218,27 +224,36 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
 		: TC_R8(0), TC_R8(8) : "r"(taddr) : "memory");
 }
 
+#define TC_I8(i) "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]), "r"(v[i + 4]), "r"(v[i + 5]), \
+	"r"(v[i + 6]), "r"(v[i + 7])
+
+/* 32 consecutive 32-bit columns of this thread's TMEM lane, written. */
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32])
+{
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+		"{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+		"%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
+		:: TC_I8(0), TC_I8(8), TC_I8(16), TC_I8(24), "r"(taddr) : "memory");
+}
+
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+/* Two values rounded to half precision with ReLU, in one instruction: a NaN
+ * stays a NaN. */
 template <class T>
-__device__ __forceinline__ uint32_t pack_relu(uint32_t lo, uint32_t hi);
-
-template <>
-__device__ __forceinline__ uint32_t pack_relu<__nv_bfloat16>(uint32_t lo, uint32_t hi)
+__device__ __forceinline__ uint32_t pack_relu(uint32_t lo, uint32_t hi)
 {
-	__nv_bfloat162 h = __floats2bfloat162_rn(fmaxf(__uint_as_float(lo), 0.0f), fmaxf(__uint_as_float(hi), 0.0f));
-	return *reinterpret_cast<uint32_t *>(&h);
+	uint32_t r;
+	if (std::is_same<T, __nv_bfloat16>::value)
+		asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+	else
+		asm("cvt.rn.relu.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
+	return r;
 }
 
-template <>
-__device__ __forceinline__ uint32_t pack_relu<__half>(uint32_t lo, uint32_t hi)
-{
-	__half2 h = __floats2half2_rn(fmaxf(__uint_as_float(lo), 0.0f), fmaxf(__uint_as_float(hi), 0.0f));
-	return *reinterpret_cast<uint32_t *>(&h);
-}
-
-template <class T>
-__global__ void __launch_bounds__(TC_THREADS, 2) mlp_infer_tc_kernel(const T *__restrict__ wt_g,
+template <class T, int UNROLL>
+__global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__restrict__ wt_g,
 		const __grid_constant__ CUtensorMap xmap, uint32_t n, float4 *__restrict__ out,
 		const uint32_t *__restrict__ n_dev, uint32_t *__restrict__ err, uint32_t withhold_first)
 {
@@ -263,7 +278,24 @@ __global__ void __launch_bounds__(TC_THREADS, 2) mlp_infer_tc_kernel(const T *__
 	const uint32_t mbar = smem_addr(sm + TC_BAR_OFF + 16u * (uint32_t)chain), tbar = mbar + 8u;
 	uint32_t *slot = reinterpret_cast<uint32_t *>(sm + TC_SLOT_OFF);
 	const uint32_t tiles = (n + TC_ROWS - 1) / TC_ROWS;
+	/* tile t goes to CTA t mod grid: few tiles spread over the SMs */
+	const uint32_t stride = gridDim.x * TC_CHAINS;
+	uint32_t t = blockIdx.x + gridDim.x * (uint32_t)chain;
 
+	if (tid == 0) {
+		for (int i = 0; i < 2 * TC_CHAINS; i++)
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(sm + TC_BAR_OFF) + 8u * i),
+				"r"(1u) : "memory");
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+		/* the first chain's first tile comes in under the weights */
+		if (t < tiles && !withhold_first)
+			tma_tile(&xmap, smem_addr(sm + TC_X_OFF), tbar, (int)(t * TC_ROWS));
+	}
+	if (warp == 0) {
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+			:: "r"(smem_addr(slot)), "r"(TC_TMEM_COLS) : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+	}
 	/* weights: global [l][rows][64] row-major -> canonical layout */
 	for (int l = 0; l < TC_LAYERS; l++) {
 		int rows = l == TC_LAYERS - 1 ? TC_OUT : TC_W;
@@ -274,107 +306,133 @@ __global__ void __launch_bounds__(TC_THREADS, 2) mlp_infer_tc_kernel(const T *__
 			*reinterpret_cast<uint4 *>(dst + core_off(r, kb * 8u)) = __ldg(src + c);
 		}
 	}
-	if (tid == 0) {
-		for (int i = 0; i < 2 * TC_CHAINS; i++)
-			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_addr(sm + TC_BAR_OFF) + 8u * i),
-				"r"(1u) : "memory");
-		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-	}
-	if (warp == 0) {
-		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-			:: "r"(smem_addr(slot)), "r"(TC_TMEM_COLS) : "memory");
-		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-	}
 	fence_async_smem();
 	tc_before();
 	__syncthreads();
 	tc_after();
 	const uint32_t tmem_base = *slot;
-	const uint32_t tmem = tmem_base + 64u * (uint32_t)chain;
-	const uint32_t lane_addr = tmem + ((uint32_t)(cwarp * 32) << 16);
-	const uint32_t wbase = smem_addr(sm), xbase = smem_addr(sm + TC_X_OFF + (uint32_t)chain * TC_X_BYTES);
-	unsigned char *xs = sm + TC_X_OFF + (uint32_t)chain * TC_X_BYTES;
+	const uint32_t act = tmem_base + TC_CHAIN_COLS * (uint32_t)chain, acc = act + 32u;
+	const uint32_t my_lane = (uint32_t)(cwarp * 32) << 16;
+	const uint32_t xbase = smem_addr(sm + TC_X_OFF + (uint32_t)chain * TC_X_BYTES);
 	const uint32_t id_hidden = instr_desc(bf16, TC_W, TC_ROWS), id_out = instr_desc(bf16, TC_OUT, TC_ROWS);
+	/* the operands' descriptors; an offset within them adds to the address
+	 * field (16-byte units, all below 2^14).  Layout type 2: 128-byte swizzle */
+	const uint64_t x_desc = smem_desc(xbase, 16u, 1024u, 2u), w_desc = smem_desc(smem_addr(sm), TC_LBO, TC_SBO, 0u);
 	uint32_t parity = 0;
-	bool ok = true;
-	/* a TMA load issued and not yet waited for, and its parity */
+	bool ok = true;    /* the same in the chain's threads */
+	bool sound = true; /* this thread's waits */
+	/* thread 0 of the chain: a TMA load issued and not yet waited for, and how
+	 * many have been */
 	bool pending = false;
-	uint32_t pend_parity = 0;
-
-	const uint32_t stride = gridDim.x * TC_CHAINS;
-	uint32_t t = blockIdx.x * TC_CHAINS + (uint32_t)chain;
-	if (ctid == 0 && t < tiles && !withhold_first)
-		tma_tile(&xmap, xbase, tbar, (int)(t * TC_ROWS));
-	pending = t < tiles && !withhold_first;
-	for (uint32_t i = 0; ok && t < tiles; i++, t += stride) {
-		pend_parity = i & 1u;
-		bool got = bar_wait(tbar, i & 1u, limit);
-		ok = chain_and(chain, got);
-		if (!ok)
-			break;
+	uint32_t loads = 0;
+	auto load = [&](uint32_t tile) {
+		tma_tile(&xmap, xbase, tbar, (int)(tile * TC_ROWS));
+		pending = true;
+	};
+	auto loaded = [&]() -> bool {
+		if (!bar_wait(tbar, loads & 1u, limit))
+			return false;
+		loads++;
 		pending = false;
-		const uint64_t lo_sw = 2u; /* layout type: 128-byte swizzle */
-		for (int l = 0; l < TC_LAYERS; l++) {
+		return true;
+	};
+
+	if (ctid == 0 && t < tiles && !withhold_first) {
+		if (chain == 0)
+			pending = true; /* issued above */
+		else
+			load(t);
+	}
+	/* ReLU keeps a NaN here, and a NaN among a row's activations makes all of
+	 * the next layer's NaN, so a row that met one ends as NaN.  Such a tile is
+	 * done again with the ReLU that makes a NaN 0; every other row is the same
+	 * with either. */
+	bool nan_relu = false;
+	while (ok && t < tiles) {
+		bool again = false;
+#pragma unroll UNROLL
+		for (int l = 0; ok && l < TC_LAYERS; l++) {
 			const bool last = l == TC_LAYERS - 1;
 			if (ctid == 0) {
-				for (uint32_t kc = 0; kc < 4; kc++)
-					tc_mma(tmem, smem_desc(xbase + kc * 32u, 16u, 1024u, (uint32_t)lo_sw),
-						smem_desc(wbase + l * TC_LAYER_BYTES + kc * 256u, TC_LBO, TC_SBO, 0u),
-						last ? id_out : id_hidden, kc > 0 ? 1u : 0u);
+				if (l == 0) {
+					if (sound && loaded()) {
+#pragma unroll
+						for (uint32_t kc = 0; kc < 4; kc++)
+							tc_mma(acc, x_desc + ((kc * 32u) >> 4), w_desc + ((kc * 256u) >> 4), id_hidden,
+								kc > 0 ? 1u : 0u);
+					} else {
+						sound = false;
+					}
+				} else {
+					/* 16 halves of K are 8 columns */
+					const uint64_t wl = w_desc + (((uint32_t)l * TC_LAYER_BYTES) >> 4);
+#pragma unroll
+					for (uint32_t kc = 0; kc < 4; kc++)
+						tc_mma_ts(acc, act + kc * 8u, wl + ((kc * 256u) >> 4), last ? id_out : id_hidden,
+							kc > 0 ? 1u : 0u);
+				}
+				/* without an MMA the commit arrives at once */
 				tc_commit(mbar);
 			}
-			got = bar_wait(mbar, parity, limit);
+			sound = bar_wait(mbar, parity, limit) && sound;
 			parity ^= 1u;
-			ok = chain_and(chain, got);
 			tc_after();
-			if (!ok)
-				break;
-			uint32_t r = (uint32_t)(cwarp * 32 + lane);
+			/* the MMA has read the tile: the next one comes into the same
+			 * buffer under the other layers */
+			if (l == 0 && ctid == 0 && sound && t + stride < tiles)
+				load(t + stride);
+			bool good = sound;
 			if (!last) {
-				/* two halves of 32 columns: two CTAs of 512 threads leave
-				 * 64 registers a thread */
-#pragma unroll
-				for (uint32_t h = 0; h < 2; h++) {
-					uint32_t v[32];
-					tmem_ld32(lane_addr + 32u * h, v);
-					tmem_wait_ld();
-#pragma unroll
-					for (uint32_t kb = 0; kb < 4; kb++) {
-						uint4 p;
-						p.x = pack_relu<T>(v[8 * kb + 0], v[8 * kb + 1]);
-						p.y = pack_relu<T>(v[8 * kb + 2], v[8 * kb + 3]);
-						p.z = pack_relu<T>(v[8 * kb + 4], v[8 * kb + 5]);
-						p.w = pack_relu<T>(v[8 * kb + 6], v[8 * kb + 7]);
-						*reinterpret_cast<uint4 *>(xs + sw128_off(r, 4u * h + kb)) = p;
-					}
-				}
-				fence_async_smem();
-			} else {
-				/* the last MMA has read the tile: the next tile's load into
-				 * the same buffer runs while the outputs are read */
-				uint32_t tn = t + stride;
-				if (ctid == 0 && tn < tiles)
-					tma_tile(&xmap, xbase, tbar, (int)(tn * TC_ROWS));
-				pending = tn < tiles;
-				uint32_t v[16];
-				tmem_ld16(lane_addr, v);
+				uint32_t v[64], a[32];
+				tmem_ld64(acc + my_lane, v);
 				tmem_wait_ld();
-				size_t row = (size_t)t * TC_ROWS + r;
-				if (row < n)
-					out[row] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), 0.0f);
+				if (nan_relu) {
+#pragma unroll
+					for (int k = 0; k < 64; k++)
+						v[k] = __float_as_uint(fmaxf(__uint_as_float(v[k]), 0.0f));
+				}
+#pragma unroll
+				for (int k = 0; k < 32; k++)
+					a[k] = pack_relu<T>(v[2 * k], v[2 * k + 1]);
+				tmem_st32(act + my_lane, a);
+				tmem_wait_st();
+			} else {
+				uint32_t v[16];
+				tmem_ld16(acc + my_lane, v);
+				tmem_wait_ld();
+				const float y[3] = {__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2])};
+				size_t row = (size_t)t * TC_ROWS + (uint32_t)(cwarp * 32 + lane);
+				if (row < n && good) {
+					out[row] = make_float4(y[0], y[1], y[2], 0.0f);
+					good = nan_relu || (y[0] == y[0] && y[1] == y[1] && y[2] == y[2]);
+				}
 			}
 			tc_before();
-			chain_sync(chain);
+			ok = chain_and(chain, good);
+			if (last && !ok) {
+				ok = chain_and(chain, sound);
+				again = ok;
+			}
 			tc_after();
 		}
+		nan_relu = again;
+		if (!again)
+			t += stride;
+		else if (ctid == 0) {
+			/* the next tile is on its way into the buffer: let it arrive, then
+			 * fetch this one again */
+			sound = !pending || loaded();
+			if (sound)
+				load(t);
+		}
 	}
-	if (!ok) {
-		if (ctid == 0)
+	if (ctid == 0) {
+		if (!ok)
 			atomicOr(err, 1u);
 		/* a load may still be in flight: give it its (bounded) time before
 		 * the block frees its memory */
 		if (pending)
-			bar_wait(tbar, pend_parity, limit);
+			bar_wait(tbar, loads & 1u, limit);
 	}
 	tc_before();
 	__syncthreads();
@@ -778,6 +836,30 @@ void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint
 	KGR_CUDA(cudaGetLastError());
 }
 
+namespace {
+
+template <class T, int UNROLL>
+void launch_infer_unrolled(const MlpParams &mp, const CUtensorMap &map, uint32_t n, int grid, float4 *out,
+		const uint32_t *n_dev, uint32_t *err, bool withhold_first, cudaStream_t st)
+{
+	static bool once = (set_tc_smem(mlp_infer_tc_kernel<T, UNROLL>), true);
+	(void)once;
+	mlp_infer_tc_kernel<T, UNROLL><<<grid, TC_THREADS, TC_SMEM, st>>>(static_cast<const T *>(mp.wt), map, n, out, n_dev,
+		err, withhold_first ? 1u : 0u);
+}
+
+template <class T>
+void launch_infer(bool many, const MlpParams &mp, const CUtensorMap &map, uint32_t n, int grid, float4 *out,
+		const uint32_t *n_dev, uint32_t *err, bool withhold_first, cudaStream_t st)
+{
+	if (many)
+		launch_infer_unrolled<T, TC_LAYERS>(mp, map, n, grid, out, n_dev, err, withhold_first, st);
+	else
+		launch_infer_unrolled<T, 1>(mp, map, n, grid, out, n_dev, err, withhold_first, st);
+}
+
+} /* namespace */
+
 void mlp_infer_tc(const MlpParams &mp, const void *x, uint32_t n, float4 *out, uint32_t *err, cudaStream_t st,
 		const uint32_t *n_dev, bool withhold_first)
 {
@@ -796,23 +878,18 @@ void mlp_infer_tc(const MlpParams &mp, const void *x, uint32_t n, float4 *out, u
 		const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
 		CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
 	KGR_REQUIRE(r == CUDA_SUCCESS, KGR_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
-	/* two CTAs fit an SM (106 KB of shared memory, 256 TMEM columns and 512
-	 * threads at 64 registers each); a CTA walks TC_CHAINS tiles at a time */
+	/* one CTA an SM; fewer when there are fewer tiles than SMs */
 	long long tiles = ((long long)n + TC_ROWS - 1) / TC_ROWS;
-	long long blocks = (tiles + TC_CHAINS - 1) / TC_CHAINS;
-	long long cap = (long long)device_sm_count() * 2;
-	int grid = (int)(blocks < cap ? blocks : cap);
-	if (mp.dtype == KGR_MLP_BF16) {
-		static bool once = (set_tc_smem(mlp_infer_tc_kernel<__nv_bfloat16>), true);
-		(void)once;
-		mlp_infer_tc_kernel<__nv_bfloat16><<<grid, TC_THREADS, TC_SMEM, st>>>(
-			static_cast<const __nv_bfloat16 *>(mp.wt), map, n, out, n_dev, err, withhold_first ? 1u : 0u);
-	} else {
-		static bool once = (set_tc_smem(mlp_infer_tc_kernel<__half>), true);
-		(void)once;
-		mlp_infer_tc_kernel<__half><<<grid, TC_THREADS, TC_SMEM, st>>>(static_cast<const __half *>(mp.wt), map, n, out,
-			n_dev, err, withhold_first ? 1u : 0u);
-	}
+	long long cap = device_sm_count();
+	int grid = (int)(tiles < cap ? tiles : cap);
+	/* the unrolled layers are six times the code, which a call of few tiles
+	 * waits for: up to 20,000 rows about 13 us a call rolled and 14 unrolled,
+	 * most of it the launch; 200,000 rows 18.6 and 16.1 us, 2.07M 102 and 81 */
+	const bool many = tiles > 2 * cap;
+	if (mp.dtype == KGR_MLP_BF16)
+		launch_infer<__nv_bfloat16>(many, mp, map, n, grid, out, n_dev, err, withhold_first, st);
+	else
+		launch_infer<__half>(many, mp, map, n, grid, out, n_dev, err, withhold_first, st);
 	KGR_CUDA(cudaGetLastError());
 }
 

@@ -168,3 +168,25 @@ def test_tcgen05_training_lowers_loss_and_times_both_kernels():
     net.check()
     print(f"gradient pass + Adam over 2^16 rows: mma.sync {times['mma'] * 1e3:.1f} us, "
           f"tcgen05 {times['tcgen05'] * 1e3:.1f} us")
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("n", [1, 127, 129, 128 * 152 + 1, 128 * 761, 200001])
+def test_tile_counts_and_non_finite_rows(dtype, n):
+    """Tiles fewer than SMs, one more than a round of them, several a chain, a
+    ragged last one; rows with NaN and infinities give what mma.sync gives
+    (ReLU makes a NaN 0), in the first, the last and a middle tile."""
+    rng = np.random.default_rng(n)
+    x = mlp_ref.encode_inputs(rng, min(n, 4096), dtype)
+    x = np.tile(x, (-(-n // len(x)), 1))[:n]
+    x[0, 5], x[n // 2, 7], x[n - 1, 0] = np.nan, np.inf, -np.inf
+    xd = half_tensor(x, dtype)
+    net = kgr.Mlp(dtype, seed=3)
+    got = {}
+    for kernel in ("mma", "tcgen05"):
+        net.set_inference(kernel)
+        out = torch.full((n, 4), 7.0, device="cuda")
+        net.forward(xd.data_ptr(), n, out.data_ptr())
+        got[kernel] = out.cpu().numpy()
+    net.check()
+    np.testing.assert_allclose(got["tcgen05"], got["mma"], rtol=2e-2, atol=2e-2)
