@@ -255,14 +255,19 @@ __device__ __forceinline__ SurfaceHit receiver_prev(const DeviceScene &s, const 
 }
 
 /* Target function of sample s at receiver h: sum_rgb(f L_o) |n.w|. */
-__device__ __forceinline__ float gi_target(const SurfaceHit &h, const GiSample &s)
+__device__ __forceinline__ float gi_target(const SurfaceHit &h, const BrdfView &view, const GiSample &s)
 {
 	f3 D = s.xs - h.x;
 	float d = length(D);
 	f3 w = D / d;
-	f3 v = brdf(h, w) * s.Lo * fabsf(dot(h.n, w));
+	f3 v = brdf(h, view, w) * s.Lo * fabsf(dot(h.n, w));
 	float t = v.x + v.y + v.z;
 	return (t > 0.0f && t < 1e30f) ? t : 0.0f;
+}
+
+__device__ __forceinline__ float gi_target(const SurfaceHit &h, const GiSample &s)
+{
+	return gi_target(h, brdf_view(h), s);
 }
 
 /* Primary vertex: G-buffer, ReSTIR DI candidates for direct light, and the
@@ -305,6 +310,7 @@ __global__ void __launch_bounds__(128) gi_primary_kernel(DeviceScene s, PathBuff
 					dst[k] = __ldg(src + k);
 				float4 sv = pb.seed[p];
 				f3 seed = mk(sv.x, sv.y, sv.z);
+				const BrdfView view = brdf_view(sh);
 				/* ReSTIR DI candidates (amadeus_restir.cu:478-523), shaded directly */
 				f3 risseed = pixel_seed(p, fp.frame, KGR_GI_RIS_SALT);
 				float wsum = 0.0f;
@@ -321,7 +327,7 @@ __global__ void __launch_bounds__(128) gi_primary_kernel(DeviceScene s, PathBuff
 						float pdf = 1.0f / (l.area() * total);
 						f3 D = pt - sh.x;
 						float d = length(D);
-						f3 Li = direct_unoccluded(sh, l.intensity, l.normal(), D / d, d);
+						f3 Li = direct_unoccluded(sh, view, l.intensity, l.normal(), D / d, d);
 						float tgt = Li.x + Li.y + Li.z;
 						weight = (pdf > 0) ? tgt / pdf : 0;
 					}
@@ -342,7 +348,7 @@ __global__ void __launch_bounds__(128) gi_primary_kernel(DeviceScene s, PathBuff
 					f3 D = selp - sh.x;
 					float d = length(D);
 					f3 Dn = D / d;
-					f3 Li = direct_unoccluded(sh, l.intensity, l.normal(), Dn, d);
+					f3 Li = direct_unoccluded(sh, view, l.intensity, l.normal(), Dn, d);
 					float tgt = Li.x + Li.y + Li.z;
 					float dd = tgt * M;
 					float W = (dd > 0) ? wsum / dd : 0.0f;
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(128) gi_primary_kernel(DeviceScene s, PathBuff
 				/* GI direction (eval, brdf.cuh:573-589) */
 				f3 wi;
 				float pdf = 0.0f;
-				eval(sh, wi, pdf, seed);
+				eval(sh, view, wi, pdf, seed);
 				if (pdf > 0 && 0 < fp.max_depth) {
 					gb.gi_dir[p] = f4_of(wi, pdf);
 					pb.ray_o[p] = f4_of(sh.x, 0.0f);
@@ -460,11 +466,12 @@ __global__ void __launch_bounds__(128) gi_temporal_kernel(DeviceScene s, FramePa
 	GiRes C = load_gi(gb.res[cur], pix);
 	int32_t pM = P.M < fp.gi_mcap ? P.M : fp.gi_mcap;
 	SurfaceHit h = receiver(fp, gb, pix, g);
+	const BrdfView view = brdf_view(h);
 	GiMerge r;
 	r.init(pixel_seed(pix, fp.frame, KGR_GI_REUSE_SALT));
-	r.update(C.s, gi_target(h, C.s) * C.W * C.M, -1);
+	r.update(C.s, gi_target(h, view, C.s) * C.W * C.M, -1);
 	float J = gi_jacobian(g.x, gp.x, P.s, fp.gi_jmax);
-	float wp = gi_target(h, P.s) * J * P.W * pM;
+	float wp = gi_target(h, view, P.s) * J * P.W * pM;
 	r.update(P.s, wp, 0);
 	/* The history counts toward the normalisation whether or not its own
 	 * sample carries weight: an empty history reservoir (its GI ray found
@@ -473,7 +480,7 @@ __global__ void __launch_bounds__(128) gi_temporal_kernel(DeviceScene s, FramePa
 	 * sample's target is positive -- divides by too few candidates and
 	 * brightens pixels whose GI samples are often empty. */
 	int32_t M = C.M + pM;
-	float tq = gi_target(h, r.sel);
+	float tq = gi_target(h, view, r.sel);
 	float jp = gi_jacobian(gp.x, g.x, r.sel, fp.gi_jmax);
 	float tp = jp > 0.0f ? gi_target(receiver_prev(s, fp, gp), r.sel) * jp : 0.0f;
 	float D = (float)C.M * tq + (float)pM * tp;
@@ -530,8 +537,9 @@ __global__ void __launch_bounds__(128) gi_spatial_gather_kernel(FrameParams fp, 
 	}
 	float depth = length(g.x - v3(fp.center));
 	SurfaceHit h = receiver(fp, gb, pix, g);
+	const BrdfView view = brdf_view(h);
 	f3 seed = pixel_seed(pix, fp.frame, KGR_GI_REUSE_SALT + 1u + (uint32_t)iteration);
-	float wC = gi_target(h, C.s) * C.W * C.M;
+	float wC = gi_target(h, view, C.s) * C.W * C.M;
 	rand_uniform(seed);
 	int32_t Msum = C.M;
 	for (int k = 0; k < fp.gi_neighbors; k++) {
@@ -554,7 +562,7 @@ __global__ void __launch_bounds__(128) gi_spatial_gather_kernel(FrameParams fp, 
 				nb = make_int2(index0, cn);
 				Msum += cn;
 				float J = N.s.rc ? gi_jacobian(g.x, gn.x, N.s, fp.gi_jmax) : 0.0f;
-				wn = J > 0.0f ? gi_target(h, N.s) * J * N.W * cn : 0.0f;
+				wn = J > 0.0f ? gi_target(h, view, N.s) * J * N.W * cn : 0.0f;
 				rand_uniform(seed);
 			}
 		}

@@ -998,21 +998,6 @@ __device__ __forceinline__ float ggx_D(const f3 &n, const f3 &h, const Material 
 	return (alpha * alpha) / (KGR_PI_DEV * kpow4(c) * kpow2(alpha * alpha + tn * tn));
 }
 
-/* GGX::brdf (brdf.cuh:337-353) with shlick_F (:202-207) and G (:195-199) */
-__device__ __forceinline__ f3 ggx_brdf(const Material &mat, f3 n, const f3 &wi, const f3 &wo)
-{
-	if (dot(wo, n) <= 0.0f)
-		n = -n;
-	f3 h = normalize(wi + wo);
-	float k = kpow5(1 - dot(wi, h));
-	f3 f = mat.specular + (1.0f - mat.specular) * k;
-	float g = G1(n, wo, mat) * G1(n, wi, mat);
-	float d = ggx_D(n, h, mat);
-	f3 num = f * g * d;
-	float denom = 4 * dot(wi, n) * dot(wo, n);
-	return num / (denom + 1e-6f);
-}
-
 /* GGX::pdf (brdf.cuh:356-382) */
 __device__ __forceinline__ float ggx_pdf(const Material &mat, f3 n, const f3 &wi, const f3 &wo)
 {
@@ -1061,7 +1046,7 @@ __device__ __forceinline__ f3 ggx_sample(const Material &mat, f3 n, const f3 &wo
 	return rotate(v, n);
 }
 
-/* ggx_brdf and ggx_pdf of one direction pair together: the flipped normal,
+/* GGX::brdf and GGX::pdf of one direction pair together: the flipped normal,
  * the half vector and D are the same in both, so they are computed once
  * (the results are those of the two separate calls). */
 __device__ __forceinline__ void ggx_brdf_pdf(const Material &mat, f3 n, const f3 &wi, const f3 &wo, f3 &brdf_out,
@@ -1091,10 +1076,72 @@ __device__ __forceinline__ void ggx_brdf_pdf(const Material &mat, f3 n, const f3
 	pdf_out = (1 - t) * term1 + t * term2;
 }
 
+/* What brdf() of one surface has in common for every incoming direction: the
+ * flipped normal, its product with wo, G1 of wo (an arc cosine, a tangent, a
+ * square root and a division) and the diffuse term's three divisions.  A loop
+ * over light samples at one surface, or a vertex that evaluates its light
+ * sample and its continuation, makes it once; the operations and their order
+ * are those of brdf.cuh:337-353, 437-449, so the values are too. */
+struct BrdfView {
+	f3 n, kd;
+	float wo_n, g1;
+};
+
+__device__ __forceinline__ BrdfView brdf_view(const SurfaceHit &sh)
+{
+	BrdfView v;
+	v.n = sh.n;
+	if (dot(sh.wo, v.n) <= 0.0f)
+		v.n = -v.n;
+	v.wo_n = dot(sh.wo, v.n);
+	v.g1 = G1(v.n, sh.wo, sh.mat);
+	v.kd = sh.mat.diffuse / KGR_PI_DEV;
+	return v;
+}
+
+/* GGX::brdf (brdf.cuh:337-353) with shlick_F (:202-207) and G (:195-199), the
+ * half vector h and D at hand */
+__device__ __forceinline__ f3 ggx_brdf_of(const SurfaceHit &sh, const BrdfView &v, const f3 &wi, const f3 &h, float d)
+{
+	float k = kpow5(1 - dot(wi, h));
+	f3 f = sh.mat.specular + (1.0f - sh.mat.specular) * k;
+	float g = v.g1 * G1(v.n, wi, sh.mat);
+	f3 num = f * g * d;
+	float denom = 4 * dot(wi, v.n) * v.wo_n;
+	return num / (denom + 1e-6f);
+}
+
 /* brdf() (brdf.cuh:437-449), out = eDiffuse */
+__device__ __forceinline__ f3 brdf(const SurfaceHit &sh, const BrdfView &v, const f3 &wi)
+{
+	f3 h = normalize(wi + sh.wo);
+	return v.kd + ggx_brdf_of(sh, v, wi, h, ggx_D(v.n, h, sh.mat));
+}
+
 __device__ __forceinline__ f3 brdf(const SurfaceHit &sh, const f3 &wi)
 {
-	return sh.mat.diffuse / KGR_PI_DEV + ggx_brdf(sh.mat, sh.n, wi, sh.wo);
+	return brdf(sh, brdf_view(sh), wi);
+}
+
+/* brdf() and ggx_pdf() of one direction: the half vector and D once. */
+__device__ __forceinline__ f3 brdf_pdf(const SurfaceHit &sh, const BrdfView &v, const f3 &wi, float &pdf)
+{
+	f3 h = normalize(wi + sh.wo);
+	float d = ggx_D(v.n, h, sh.mat);
+	f3 f = v.kd + ggx_brdf_of(sh, v, wi, h, d);
+	if (dot(wi, v.n) <= 0.0f) {
+		pdf = 0.0f;
+		return f;
+	}
+	float avg_Kd = (sh.mat.diffuse.x + sh.mat.diffuse.y + sh.mat.diffuse.z) / 3.0f;
+	float avg_Ks = (sh.mat.specular.x + sh.mat.specular.y + sh.mat.specular.z) / 3.0f;
+	float t = 1.0f;
+	if (avg_Kd + avg_Ks > 0.0f)
+		t = kmax(avg_Ks / (avg_Kd + avg_Ks), 0.25f);
+	float term1 = dot(v.n, wi) / KGR_PI_DEV;
+	float term2 = d * dot(v.n, h) / (4.0f * dot(wi, h));
+	pdf = (1 - t) * term1 + t * term2;
+	return f;
 }
 
 /* A ReSTIR GI secondary vertex whose outgoing radiance may be reused toward
@@ -1110,7 +1157,7 @@ __device__ __forceinline__ bool gi_reconnectable(const Material &m)
 
 /* eval() (brdf.cuh:573-589): GGX, or Glass::sample (:154-175) for
  * transmissive materials; pdf = 0 for a degenerate direction. */
-__device__ __forceinline__ f3 eval(const SurfaceHit &sh, f3 &wi, float &pdf, f3 &seed)
+__device__ __forceinline__ f3 eval(const SurfaceHit &sh, const BrdfView &v, f3 &wi, float &pdf, f3 &seed)
 {
 	if (sh.mat.type & KGR_SHADING_TRANSMISSION) {
 		float eta = sh.mat.refraction;
@@ -1138,8 +1185,12 @@ __device__ __forceinline__ f3 eval(const SurfaceHit &sh, f3 &wi, float &pdf, f3 
 		pdf = 0.0f;
 		return mk(0.0f);
 	}
-	pdf = ggx_pdf(sh.mat, sh.n, wi, sh.wo);
-	return brdf(sh, wi);
+	return brdf_pdf(sh, v, wi, pdf);
+}
+
+__device__ __forceinline__ f3 eval(const SurfaceHit &sh, f3 &wi, float &pdf, f3 &seed)
+{
+	return eval(sh, brdf_view(sh), wi, pdf, seed);
 }
 
 /* --------------------------------------------------------------- lights -- */
@@ -1181,10 +1232,10 @@ __device__ __forceinline__ f3 sample_area_light(const TriLight &light, f3 &seed)
 #define KGR_OFFSET_EPS 1e-3f /* amadeus_common.cuh:22 */
 
 /* direct_unoccluded (amadeus_common.cuh:380-397) for a triangle light */
-__device__ __forceinline__ f3 direct_unoccluded(const SurfaceHit &sh, const f3 &Le, const f3 &normal,
+__device__ __forceinline__ f3 direct_unoccluded(const SurfaceHit &sh, const BrdfView &v, const f3 &Le, const f3 &normal,
 		const f3 &D, float d)
 {
-	f3 rho = brdf(sh, D);
+	f3 rho = brdf(sh, v, D);
 	float geometric = fabsf(dot(sh.n, D));
 	float ldot = fabsf(dot(normal, D));
 	geometric *= ldot / (d * d);
@@ -1317,10 +1368,10 @@ __device__ __forceinline__ int sample_direct(const DeviceScene &s, const f3 &x, 
 
 /* direct_unoccluded (amadeus_common.cuh:380-397) for any light type: the
  * environment (type 2) drops the light's cosine and 1/d^2 */
-__device__ __forceinline__ f3 direct_unoccluded_typed(const SurfaceHit &sh, const f3 &Le, const f3 &normal,
-		int type, const f3 &D, float d)
+__device__ __forceinline__ f3 direct_unoccluded_typed(const SurfaceHit &sh, const BrdfView &v, const f3 &Le,
+		const f3 &normal, int type, const f3 &D, float d)
 {
-	f3 rho = brdf(sh, D);
+	f3 rho = brdf(sh, v, D);
 	float geometric = fabsf(dot(sh.n, D));
 	if (type != 2) {
 		float ldot = fabsf(dot(normal, D));

@@ -33,6 +33,7 @@ __device__ __forceinline__ void shade_surface(const DeviceScene &s, const FrameP
 	float sgn = sh.mat.type == KGR_SHADING_TRANSMISSION ? -1.0f : 1.0f;
 	sh.x = sh.x + sgn * n3 * KGR_OFFSET_EPS;
 	out.vertex(sh.x, n3, sh.mat);
+	const BrdfView view = brdf_view(sh);
 	unsigned int total_count = s.quad_count + s.light_count + (s.has_env ? 1u : 0u);
 	if (total_count == 0) {
 		f3 direct = sh.mat.emission + mk(0.0f);
@@ -62,7 +63,7 @@ __device__ __forceinline__ void shade_surface(const DeviceScene &s, const FrameP
 			}
 			wi = normalize(lpos - sh.x);
 			float R = length(lpos - sh.x);
-			f3 f = brdf(sh, wi);
+			f3 f = brdf(sh, view, wi);
 			float ldot = fabsf(dot(lnormal, wi));
 			float geometric = ldot * fabsf(dot(sh.n, wi)) / (R * R);
 			contr = f * Le * geometric;
@@ -75,7 +76,7 @@ __device__ __forceinline__ void shade_surface(const DeviceScene &s, const FrameP
 			env_uv(wi, u, v);
 			f3 Li = env_fetch(s, u, v);
 			light_pdf = (float)(1.0 / (4.0 * KGR_PI_D));
-			f3 f = brdf(sh, wi) * fabsf(dot(sh.n, wi));
+			f3 f = brdf(sh, view, wi) * fabsf(dot(sh.n, wi));
 			contr = f * Li;
 			tmax = KGR_WORLD_RADIUS - KGR_SHADOW_EPS;
 		}
@@ -91,7 +92,7 @@ __device__ __forceinline__ void shade_surface(const DeviceScene &s, const FrameP
 	if (depth < last || final_seed) {
 		f3 wi;
 		float pdf = 0.0f;
-		f3 f = eval(sh, wi, pdf, seed);
+		f3 f = eval(sh, view, wi, pdf, seed);
 		if (pdf > 0) {
 			f3 T = f * fabsf(dot(wi, n3)) / pdf;
 			beta = beta * T;

@@ -107,7 +107,8 @@ __device__ __forceinline__ void store_res(const ReservoirBuffers &rb, uint32_t i
 
 
 /* target (amadeus_restir.cu:147-161) */
-__device__ __forceinline__ float target(const DeviceScene &s, const Sample &smp, const SurfaceHit &hit)
+__device__ __forceinline__ float target(const DeviceScene &s, const Sample &smp, const SurfaceHit &hit,
+		const BrdfView &view)
 {
 	if (!has_light(smp))
 		return 0.0f;
@@ -115,7 +116,7 @@ __device__ __forceinline__ float target(const DeviceScene &s, const Sample &smp,
 	int type = emitter(s, smp, Le, ln);
 	f3 D = smp.point - hit.x;
 	float d = length(D);
-	f3 Li = direct_unoccluded_typed(hit, Le, ln, type, D / d, d);
+	f3 Li = direct_unoccluded_typed(hit, view, Le, ln, type, D / d, d);
 	return Li.x + Li.y + Li.z;
 }
 
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(128) primary_kernel(DeviceScene s, PathBuffers
 				pb.aov_p[p] = f4_of(sh.x, 0.0f);
 				float4 sv = pb.seed[p];
 				f3 seed = mk(sv.x, sv.y, sv.z);
+				const BrdfView view = brdf_view(sh);
 				Reservoir res;
 				res.init(pixel_seed(p, fp.frame, KGR_RIS_SALT));
 				for (int c = 0; c < fp.candidates; c++) {
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(128) primary_kernel(DeviceScene s, PathBuffers
 						pdf = lp.pdf;
 						f3 D = smp.point - sh.x;
 						float d = length(D);
-						f3 Li = direct_unoccluded_typed(sh, lp.Le, lp.normal, lp.type, D / d, d);
+						f3 Li = direct_unoccluded_typed(sh, view, lp.Le, lp.normal, lp.type, D / d, d);
 						tgt = Li.x + Li.y + Li.z;
 					} else {
 						smp.light = -1;
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(128) primary_kernel(DeviceScene s, PathBuffers
 					f3 D = res.data.point - sh.x;
 					float d = length(D);
 					f3 Dn = D / d;
-					f3 Li = direct_unoccluded_typed(sh, Le, ln, type, Dn, d);
+					f3 Li = direct_unoccluded_typed(sh, view, Le, ln, type, Dn, d);
 					tgt = Li.x + Li.y + Li.z;
 					pb.sh_o[p] = f4_of(sh.x, 0.0f);
 					pb.sh_d[p] = f4_of(Dn, d - KGR_SHADOW_EPS);
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(128) primary_kernel(DeviceScene s, PathBuffers
 				/* continuation (:531-558) */
 				f3 wi;
 				float pdf = 0.0f;
-				f3 f = eval(sh, wi, pdf, seed);
+				f3 f = eval(sh, view, wi, pdf, seed);
 				if (pdf > 0) {
 					f3 T = f * fabsf(dot(wi, n3)) / pdf;
 					float4 bv = pb.beta[p];
@@ -391,7 +393,8 @@ __global__ void __launch_bounds__(128) temporal_gather_kernel(DeviceScene s, Fra
 		return;
 	SurfaceHit hit = gbuffer_hit(fp, rb, out, pix);
 	int pindex = reproject(fp, (int)pix, hit.x);
-	float t_current = target(s, cs, hit);
+	const BrdfView view = brdf_view(hit);
+	float t_current = target(s, cs, hit, view);
 	rb.targets[pix] = t_current;
 	/* +0 stays +0 whatever the ray; anything else is traced */
 	bool ray = __float_as_uint(t_current) != 0u;
@@ -405,7 +408,7 @@ __global__ void __launch_bounds__(128) temporal_gather_kernel(DeviceScene s, Fra
 		float pw, pW;
 		load_res(P, (uint32_t)pindex, ps, pw, pW, pM);
 		if (pM > 0) {
-			float t_previous = target(s, ps, hit);
+			float t_previous = target(s, ps, hit, view);
 			rb.targets[fp.npix + pix] = t_previous;
 			bool pray = __float_as_uint(t_previous) != 0u;
 			if (pray)
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(128) temporal_merge_kernel(DeviceScene s, Fram
 		}
 	}
 	merged.M = N;
-	float t_merged = target(s, merged.data, hit);
+	float t_merged = target(s, merged.data, hit, brdf_view(hit));
 	merged.resample(t_merged);
 	store_res(C, pix, merged.data, merged.w, merged.W, merged.M);
 }
@@ -507,6 +510,7 @@ __global__ void __launch_bounds__(128) restir_gather_kernel(DeviceScene s, Frame
 	if (cM <= 0)
 		return;
 	SurfaceHit hit = gbuffer_hit(fp, rb, out, pix);
+	const BrdfView view = brdf_view(hit);
 	f3 from = f3_of(out.position[pix]);
 	float4 av = rb.auxiliary[pix];
 	f3 seed = mk(av.x, av.y, av.z);
@@ -522,7 +526,7 @@ __global__ void __launch_bounds__(128) restir_gather_kernel(DeviceScene s, Frame
 		bool ray = false;
 		if (nM > 0) {
 			if (has_light(ns)) {
-				t = target(s, ns, hit);
+				t = target(s, ns, hit, view);
 				/* +0 stays +0 whatever the ray; -0 would become +0 if blocked */
 				ray = __float_as_uint(t) != 0u;
 			}
@@ -557,7 +561,7 @@ __global__ void __launch_bounds__(128) restir_resample_kernel(DeviceScene s, Fra
 	float4 av = rb.auxiliary[pix];
 	Reservoir merged;
 	merged.init(mk(av.x, av.y, av.z));
-	float t_current = target(s, cs, hit);
+	float t_current = target(s, cs, hit, brdf_view(hit));
 	merged.update(cs, t_current * cW * cM);
 	int K = fp.spatial_neighbors;
 	int32_t count = 0;
@@ -585,7 +589,7 @@ __global__ void __launch_bounds__(128) restir_resample_kernel(DeviceScene s, Fra
 			SurfaceHit h0 = gbuffer_hit(fp, rb, out, (uint32_t)nb.x);
 			h0.wo = hit.wo;
 			h0.entering = true;
-			t = target(s, merged.data, h0);
+			t = target(s, merged.data, h0, brdf_view(h0));
 		}
 		rb.targets[slot] = t;
 		if (t > 0.0f)
@@ -627,7 +631,8 @@ __global__ void __launch_bounds__(128) restir_finish_kernel(DeviceScene s, Frame
 			if (vis_target(rb, slot) > 0.0f)
 				Z += size;
 		}
-		float t_merged = target(s, data, hit);
+		const BrdfView view = brdf_view(hit);
+		float t_merged = target(s, data, hit, view);
 		float denominator = t_merged * Z;
 		float W = (denominator > 0.0f) ? w / denominator : 0.0f;
 		f3 lighting = mk(0.0f);
@@ -637,7 +642,7 @@ __global__ void __launch_bounds__(128) restir_finish_kernel(DeviceScene s, Frame
 			f3 D = data.point - hit.x;
 			float d = length(D);
 			f3 Dn = D / d;
-			lighting = direct_unoccluded_typed(hit, Le, ln, type, Dn, d);
+			lighting = direct_unoccluded_typed(hit, view, Le, ln, type, Dn, d);
 		}
 		direct = hit.mat.emission + lighting * W;
 		store_res(OUT, pix, data, w, W, M);
