@@ -40,8 +40,8 @@ __global__ void __launch_bounds__(256) batch_generate_kernel(PathBuffers pb, con
 		pb.counters[CNT_Q0] = total;
 		pb.counters[CNT_Q1] = 0;
 		pb.counters[CNT_SHADOW] = 0;
-		pb.counters[CNT_BOUNCE_TOTAL] = 0;
-		pb.counters[CNT_SHADOW_TOTAL] = 0;
+		for (int k = CNT_BOUNCE_TOTAL; k < CNT_COUNT; k++)
+			pb.counters[k] = 0;
 	}
 	for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
 		const BatchJob &J = jobs[find_job<false>(jobs, njobs, p)];
@@ -109,8 +109,6 @@ void batch_frame(const DeviceScene &s, const PathBuffers &pb, const FrameParams 
 		pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
 		for (int d = 0; d <= fp.max_depth; d++) {
 			int q = d & 1;
-			if (d > 0)
-				reset_counters(pb, (1 << (q ^ 1)) | (1 << CNT_SHADOW), st);
 			pt_shade(s, pb, fp, d, q, st);
 			KGR_CUDA(cudaEventRecord(side.shaded, st));
 			KGR_CUDA(cudaStreamWaitEvent(side.stream, side.shaded, 0));
@@ -123,8 +121,6 @@ void batch_frame(const DeviceScene &s, const PathBuffers &pb, const FrameParams 
 	} else {
 		for (int d = 0; d <= fp.max_depth; d++) {
 			int q = d & 1;
-			if (d > 0)
-				reset_counters(pb, (1 << (q ^ 1)) | (1 << CNT_SHADOW), st);
 			pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 			pt_shade(s, pb, fp, d, q, st);
 			pt_shadow_resolve(s, pb, fp.layout, fp.tune, st);

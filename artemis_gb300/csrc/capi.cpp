@@ -1244,10 +1244,6 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 		m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 		for (int d = 0; d <= last; d++) {
 			int q = d & 1;
-			if (d > 0) {
-				reset_counters(pb, (1 << (q ^ 1)) | (1 << CNT_SHADOW), st);
-				m = att->mark(-1, st);
-			}
 			pt_shade(s, pb, fp, d, q, st);
 			m = att->mark(STAGE_SHADE, st, m);
 			KGR_CUDA(cudaEventRecord(att->ev_shaded, st));
@@ -1267,10 +1263,6 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 	} else {
 		for (int d = 0; d <= last; d++) {
 			int q = d & 1;
-			if (d > 0) {
-				reset_counters(pb, (1 << (q ^ 1)) | (1 << CNT_SHADOW), st);
-				m = att->mark(-1, st);
-			}
 			pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 			m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 			pt_shade(s, pb, fp, d, q, st);
@@ -1347,7 +1339,9 @@ void render_restir_di(kgr_attachment *att, const kgr_launch_info *info, const kg
 	/* with an environment map one more bounce is traced for its misses */
 	for (int d = 1; d <= fp.max_depth; d++) {
 		int q = d & 1;
-		reset_counters(pb, (1 << (q ^ 1)) | (1 << CNT_SHADOW), st);
+		/* the primary vertex's queue; shade empties the later ones */
+		if (d == 1)
+			reset_counters(pb, 1 << CNT_Q0, st);
 		att->mark(-1, st);
 		pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 		att->mark(STAGE_TRACE_CLOSEST, st);
@@ -1573,7 +1567,6 @@ void render_pt_cached(kgr_attachment *att, const kgr_launch_info *info, const kg
 		KGR_CUDA(cudaEventRecord(att->ev_infer, st));
 	if (overlap)
 		KGR_CUDA(cudaStreamWaitEvent(st, att->ev_shadowed, 0));
-	reset_counters(pb, (1 << CNT_Q0) | (1 << CNT_SHADOW), st);
 	cache_apply(pb, 1, att->q_out.ptr, att->q_le.ptr, st);
 	m = att->mark(STAGE_CACHE_INFER, st, m);
 	pt_accumulate(pb, fp, out, st);
@@ -1669,7 +1662,9 @@ void render_restir_gi(kgr_attachment *att, const kgr_launch_info *info, const kg
 	launches += 2 + KGR_GI_PRIMARY_LAUNCHES; /* generate, closest hit, primary vertex, its shadow rays */
 	for (int d = 1; d <= fp.max_depth; d++) {
 		int q = d & 1;
-		reset_counters(pb, (1 << (q ^ 1)) | (1 << CNT_SHADOW), st);
+		/* the primary vertex's queue; shade empties the later ones */
+		if (d == 1)
+			reset_counters(pb, 1 << CNT_Q0, st);
 		att->mark(-1, st);
 		pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 		att->mark(STAGE_TRACE_CLOSEST, st);

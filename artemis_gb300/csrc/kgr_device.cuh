@@ -1464,6 +1464,16 @@ __device__ __forceinline__ void queue_append(uint32_t *queue, uint32_t *counter,
 		queue[base + __popc(ballot & ((1u << lane) - 1u))] = value;
 }
 
+/* True in one lane of the launch: the last warp of the grid to get here.  The
+ * counter is 0 again afterwards.  A kernel ends with it to put back the
+ * counters that its launch has used up -- every other warp has read them by
+ * then -- so that no memset lies between two launches (about 2 us each). */
+__device__ __forceinline__ bool last_warp(uint32_t *done)
+{
+	const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+	return (threadIdx.x & 31) == 0 && atomicInc(done, warps - 1u) == warps - 1u;
+}
+
 /* Visit entries 0..n-1 of a queue in batches of 32 a warp: lane 0 takes the
  * next batch from *fetch when the warp is done with its last, so warps that
  * drew short rays take more batches and none is left with a fixed share of

@@ -24,7 +24,12 @@ enum Counter {
 	CNT_SHADOW_TOTAL = 4,
 	CNT_FETCH_CLOSEST = 5, /* next queue entry of the persistent closest-hit kernel */
 	CNT_FETCH_SHADOW = 6,  /* next queue entry of the persistent shadow kernel */
-	CNT_COUNT = 8
+	/* warps of the running closest-hit, shadow and shade launch that are done
+	 * (last_warp); 0 between launches, as the two fetch counters are */
+	CNT_DONE_CLOSEST = 7,
+	CNT_DONE_SHADOW = 8,
+	CNT_DONE_SHADE = 9,
+	CNT_COUNT = 10
 };
 
 struct PathBuffers {

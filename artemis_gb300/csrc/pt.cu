@@ -48,8 +48,8 @@ __global__ void generate_kernel(PathBuffers pb, FrameParams fp)
 		pb.counters[CNT_Q0] = fp.paths;
 		pb.counters[CNT_Q1] = 0;
 		pb.counters[CNT_SHADOW] = 0;
-		pb.counters[CNT_BOUNCE_TOTAL] = 0;
-		pb.counters[CNT_SHADOW_TOTAL] = 0;
+		for (int k = CNT_BOUNCE_TOTAL; k < CNT_COUNT; k++)
+			pb.counters[k] = 0;
 	}
 	if (p >= fp.paths)
 		return;
@@ -104,6 +104,26 @@ __global__ void __launch_bounds__(128) trace_closest_kernel(DeviceScene s, PathB
 	}
 	if (COUNT)
 		add_visits(pb.visits, cnt);
+}
+
+/* The end of an any-hit walk: its fetch counter back to 0, and the queue's
+ * count too unless the blocked flags' reader still needs it. */
+__device__ __forceinline__ void end_shadow(const PathBuffers &pb)
+{
+	__syncwarp();
+	if (last_warp(pb.counters + CNT_DONE_SHADOW)) {
+		pb.counters[CNT_FETCH_SHADOW] = 0;
+		if (!pb.shadow_flags)
+			pb.counters[CNT_SHADOW] = 0;
+	}
+}
+
+/* The end of a closest-hit walk. */
+__device__ __forceinline__ void end_closest(const PathBuffers &pb)
+{
+	__syncwarp();
+	if (last_warp(pb.counters + CNT_DONE_CLOSEST))
+		pb.counters[CNT_FETCH_CLOSEST] = 0;
 }
 
 /* Writes one shaded vertex into the path state of path p. */
@@ -211,6 +231,10 @@ __global__ void __launch_bounds__(SHADE_BLOCK) shade_kernel(DeviceScene s, PathB
 			return p;
 		},
 		[&](uint32_t p, float4 hv) { shade_hit(s, pb, fp, depth, final_seed, next_queue, out_counter, p, hv); });
+	/* this bounce's queue is used up: empty, it takes the next but one */
+	__syncwarp();
+	if (last_warp(pb.counters + CNT_DONE_SHADE))
+		pb.counters[q == 0 ? CNT_Q0 : CNT_Q1] = 0;
 }
 
 /* is_occluded for every queued shadow ray, then Ld = contr / pdf and
@@ -262,6 +286,7 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) shadow_reso
 	}
 	if (COUNT)
 		add_visits(pb.visits + 2, cnt);
+	end_shadow(pb);
 }
 
 /* Shadow-ray resolve: L holds L + beta * (Le + 0) already (the blocked
@@ -321,6 +346,7 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) fast_persis
 				load(i, a, b);
 				return true;
 			}, done);
+		ANY ? end_shadow(pb) : end_closest(pb);
 		return;
 	}
 	int32_t local_stack[KGR_STACK_DEPTH - SHORT];
@@ -341,6 +367,7 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) fast_persis
 		}, done);
 	if (COUNT)
 		add_visits(pb.visits + (ANY ? 2 : 0), cnt);
+	ANY ? end_shadow(pb) : end_closest(pb);
 }
 
 /* The persistent traversal over the compressed eight-child layout: the
@@ -404,6 +431,7 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) cw_persiste
 	}
 	if (COUNT)
 		add_visits(pb.visits + (ANY ? 2 : 0), cnt);
+	ANY ? end_shadow(pb) : end_closest(pb);
 }
 
 template <class K>
@@ -564,7 +592,6 @@ void pt_trace_closest(const DeviceScene &s, const PathBuffers &pb, int q, int la
 		else
 			trace_closest_kernel<KGR_LAYOUT_THREADED, false><<<grid, 128, 0, st>>>(s, pb, q);
 	} else {
-		KGR_CUDA(cudaMemsetAsync(pb.counters + CNT_FETCH_CLOSEST, 0, sizeof(uint32_t), st));
 		if (layout == KGR_LAYOUT_CW8) {
 			if (c)
 				launch_cw_persistent<false, true, 128>(s, pb, q, st);
@@ -619,7 +646,6 @@ void pt_shadow_resolve(const DeviceScene &s, const PathBuffers &pb, int layout, 
 		else
 			launch_shadow_grid<true, KGR_LAYOUT_FAST, 128>(s, pb, st);
 	} else if (tune.shadow == TRACE_PERSISTENT) {
-		KGR_CUDA(cudaMemsetAsync(pb.counters + CNT_FETCH_SHADOW, 0, sizeof(uint32_t), st));
 		if (layout == KGR_LAYOUT_CW8)
 			launch_cw_persistent_tuned<true>(s, pb, 0, tune, st);
 		else if (layout == KGR_LAYOUT_WIDE)
