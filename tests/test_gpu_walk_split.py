@@ -63,3 +63,28 @@ def test_small_counts_on_every_tree(scene, max_leaf):
     ref = sc.trace_closest_host(rays, kgr.LAYOUT_THREADED)
     assert np.array_equal(sc.trace_closest_host(rays).view(np.uint32), ref.view(np.uint32))
     assert np.array_equal(sc.trace_any_host(rays), sc.trace_any_host(rays, kgr.LAYOUT_THREADED))
+
+
+@pytest.mark.parametrize("side", [48, 176, 256, 288])
+@pytest.mark.parametrize("plugin", ["restir_di", "restir_gi"])
+def test_restir_bounces_overlapped_or_not(plugin, side):
+    """Bounces whose shadow rays run beside the next closest hits, at path
+    counts on each side of the cooperative walk's limits: the same bits as
+    one after the other."""
+    torch = pytest.importorskip("torch")
+    g, sc, _ = helpers.both("box64", 5)
+    cam = kgr.camera(g.eye, g.target, g.fov, 1.0)
+    images = []
+    for overlap in (False, True):
+        bufs = helpers.device_buffers(torch, side * side)
+        att = kgr.Attachment(plugin)
+        att.attach(side, side)
+        att.load()
+        att.set_option("trace_overlap", overlap)
+        for frame in range(2):
+            att.render(helpers.launch(cam, side, side, bufs, frame=frame, max_depth=3), sc)
+        torch.cuda.synchronize()
+        images.append(bufs[0].cpu().numpy())
+        att.close()
+    assert images[0][:, :3].mean() > 0.0
+    assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
