@@ -1,8 +1,8 @@
 /*
  * kgr_mlp.h -- the radiance-cache MLP (mlp.cu) and the device buffers of one
  * network: FP32 master weights W[6][64][64] ([in][out]; the last layer's
- * outputs 3..63 unused), Adam moments, and half-precision copies
- * wn[l] = [in][cols] and wt[l] = [cols][in] (cols = 64, or 16 for the last).
+ * outputs 3..63 unused), Adam moments, and a half-precision copy
+ * wt[l] = [cols][in] (cols = 64, or 16 for the last).
  */
 #ifndef KGR_MLP_H_
 #define KGR_MLP_H_
@@ -17,7 +17,7 @@ namespace kgr {
 struct MlpParams {
 	int dtype; /* KGR_MLP_BF16 or KGR_MLP_FP16 */
 	float *master, *m, *v;
-	void *wn, *wt;
+	void *wt;
 	float *partial;     /* per-block gradient slices [partial_blocks][6][64][64] */
 	int partial_blocks;
 	int infer;          /* KGR_MLP_INFER_MMA or KGR_MLP_INFER_TCGEN05 */
@@ -63,11 +63,11 @@ struct kgr_mlp {
 	int infer = KGR_MLP_INFER_TCGEN05;
 	int train = KGR_MLP_TRAIN_TCGEN05;
 	kgr::DevBuf<float> master, m, v, grad, loss, partial;
-	kgr::DevBuf<uint16_t> wn, wt;
+	kgr::DevBuf<uint16_t> wt;
 	kgr::DevBuf<uint32_t> tc_err;
 	kgr::MlpParams params()
 	{
-		return kgr::MlpParams{dtype, master.ptr, m.ptr, v.ptr, wn.ptr, wt.ptr, partial.ptr, partial_blocks, infer,
+		return kgr::MlpParams{dtype, master.ptr, m.ptr, v.ptr, wt.ptr, partial.ptr, partial_blocks, infer,
 			tc_err.ptr, train};
 	}
 };

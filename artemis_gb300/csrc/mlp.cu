@@ -82,27 +82,17 @@ struct HalfOps<__half> {
 	}
 };
 
-/* Stage the half-precision weights in shared memory, transposed (forward)
- * and/or as stored (backward). */
+/* Stage the half-precision weights ([out][in]) in shared memory. */
 template <class T>
-__device__ __forceinline__ void stage_weights(const T *__restrict__ wt_g, T *wt_s, const T *__restrict__ wn_g,
-		T *wn_s)
+__device__ __forceinline__ void stage_weights(const T *__restrict__ wt_g, T *wt_s)
 {
-	/* global layout: per layer a dense [rows][64] block; layer 5 has 16 rows
-	 * in the transposed copy and 64 x 16 in the plain copy */
+	/* global layout: per layer a dense [rows][64] block; layer 5 has 16 rows */
 	for (int l = 0; l < MLP_LAYERS; l++) {
 		int rows_t = l == MLP_LAYERS - 1 ? MLP_OUT_PAD : MLP_W;
 		const T *src = wt_g + (size_t)l * MLP_W * MLP_W;
 		T *dst = wt_s + (size_t)l * MLP_W * MLP_STRIDE;
 		for (int i = threadIdx.x; i < rows_t * MLP_W; i += blockDim.x)
 			dst[(i / MLP_W) * MLP_STRIDE + (i % MLP_W)] = src[i];
-		if (wn_s) {
-			int cols_n = l == MLP_LAYERS - 1 ? MLP_OUT_PAD : MLP_W;
-			const T *s2 = wn_g + (size_t)l * MLP_W * MLP_W;
-			T *d2 = wn_s + (size_t)l * MLP_W * MLP_STRIDE;
-			for (int i = threadIdx.x; i < MLP_W * cols_n; i += blockDim.x)
-				d2[(i / cols_n) * MLP_STRIDE + (i % cols_n)] = s2[i];
-		}
 	}
 }
 
@@ -202,7 +192,7 @@ __global__ void __launch_bounds__(128) mlp_infer_kernel(const T *__restrict__ wt
 	}
 	extern __shared__ __align__(16) unsigned char smem_raw[];
 	T *wt_s = reinterpret_cast<T *>(smem_raw);
-	stage_weights<T>(wt_g, wt_s, nullptr, nullptr);
+	stage_weights<T>(wt_g, wt_s);
 	__syncthreads();
 	int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	int g = lane >> 2, t = lane & 3;
@@ -287,7 +277,7 @@ __global__ void __launch_bounds__(128) mlp_train_kernel(const T *__restrict__ wt
 	T *act = wt_s + (size_t)MLP_LAYERS * MLP_W * MLP_STRIDE;             /* 6 x [64][72] */
 	T *dlt = act + (size_t)MLP_LAYERS * TRAIN_ROWS * MLP_STRIDE;          /* [64][72] */
 	float *gacc = reinterpret_cast<float *>(dlt + (size_t)TRAIN_ROWS * MLP_STRIDE); /* [6][64][64] */
-	stage_weights<T>(wt_g, wt_s, nullptr, nullptr);
+	stage_weights<T>(wt_g, wt_s);
 	for (int i = threadIdx.x; i < MLP_LAYERS * MLP_W * MLP_W / 4; i += blockDim.x)
 		reinterpret_cast<float4 *>(gacc)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	__syncthreads();
@@ -478,11 +468,10 @@ __global__ void reduce_partials_kernel(const float *__restrict__ partial, int bl
 	grad[k] = s;
 }
 
-/* Adam on the FP32 master weights, then the half-precision copies in both
- * layouts (plain [l][in][out] and transposed [l][out][in]). */
+/* Adam on the FP32 master weights, then the half-precision copy [l][out][in]. */
 template <class T>
 __global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
-		const float *__restrict__ grad, T *__restrict__ wn, T *__restrict__ wt, float lr, float b1, float b2,
+		const float *__restrict__ grad, T *__restrict__ wt, float lr, float b1, float b2,
 		float eps, float c1, float c2, int update)
 {
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -504,12 +493,8 @@ __global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float 
 		w[i] = wi;
 	}
 	T h = HalfOps<T>::from_float(wi);
-	/* plain copy: layer l block [in][cols], cols = 64 or 16 */
-	int cols = l == MLP_LAYERS - 1 ? MLP_OUT_PAD : MLP_W;
-	if (out < cols)
-		wn[(size_t)l * MLP_W * MLP_W + in * cols + out] = h;
-	/* transposed copy: [out][in], rows = 64 or 16 */
-	if (out < cols)
+	/* [out][in], rows = 64 or 16 */
+	if (out < (l == MLP_LAYERS - 1 ? MLP_OUT_PAD : MLP_W))
 		wt[(size_t)l * MLP_W * MLP_W + out * MLP_W + in] = h;
 }
 
@@ -597,11 +582,11 @@ void mlp_adam(const MlpParams &mp, const float *grad, float lr, int step, cudaSt
 	int n = MLP_LAYERS * MLP_W * MLP_W;
 	if (mp.dtype == KGR_MLP_BF16)
 		adam_kernel<__nv_bfloat16><<<(n + 255) / 256, 256, 0, st>>>(mp.master, mp.m, mp.v, grad,
-			static_cast<__nv_bfloat16 *>(mp.wn), static_cast<__nv_bfloat16 *>(mp.wt), lr, b1, b2, eps, c1, c2,
+			static_cast<__nv_bfloat16 *>(mp.wt), lr, b1, b2, eps, c1, c2,
 			update);
 	else
 		adam_kernel<__half><<<(n + 255) / 256, 256, 0, st>>>(mp.master, mp.m, mp.v, grad,
-			static_cast<__half *>(mp.wn), static_cast<__half *>(mp.wt), lr, b1, b2, eps, c1, c2, update);
+			static_cast<__half *>(mp.wt), lr, b1, b2, eps, c1, c2, update);
 	KGR_CUDA(cudaGetLastError());
 }
 

@@ -48,7 +48,6 @@ void alloc_all(kgr_mlp *m)
 	m->v.alloc(KGR_MLP_PARAMS);
 	m->grad.alloc(KGR_MLP_PARAMS);
 	m->loss.alloc(1);
-	m->wn.alloc(KGR_MLP_PARAMS);
 	m->wt.alloc(KGR_MLP_PARAMS);
 	m->partial_blocks = kgr::device_sm_count();
 	m->partial.alloc((size_t)m->partial_blocks * KGR_MLP_PARAMS);
@@ -56,7 +55,6 @@ void alloc_all(kgr_mlp *m)
 	KGR_CUDA(cudaMemset(m->tc_err.ptr, 0, sizeof(uint32_t)));
 	KGR_CUDA(cudaMemset(m->m.ptr, 0, KGR_MLP_PARAMS * 4));
 	KGR_CUDA(cudaMemset(m->v.ptr, 0, KGR_MLP_PARAMS * 4));
-	KGR_CUDA(cudaMemset(m->wn.ptr, 0, KGR_MLP_PARAMS * 2));
 	KGR_CUDA(cudaMemset(m->wt.ptr, 0, KGR_MLP_PARAMS * 2));
 }
 

@@ -445,95 +445,124 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__
 /* ------------------------------------------------------------ training -- */
 
 /* Training (forward, loss, backward) on the fifth-generation tensor cores.
- * One CTA of 128 threads per SM (225 KB of shared memory, 512 TMEM
- * columns) walks tiles of 128 rows; every operand sits in shared memory in
- * the canonical K-major layout without swizzle (8 x 8 core matrices of 128
- * contiguous bytes, K neighbours 128 bytes apart, 8-row groups K/8 x 128
- * bytes apart):
- *   WT   the six layers' weights as [out][in] (forward B operands, 42 KB)
- *   WN   layers 1..5 as [in][out] (the delta's B operands, 34 KB)
- *   X    the tile's input of the current layer [128][64] (forward A operand)
- *   AT   every layer's input transposed, [64][128] (A operands of dW)
- *   D    the delta of the current layer's output [128][cols] (A operand)
- *   DT   the same transposed, [cols][128] (B operand of dW)
- * Per tile: six forward MMAs (M = 128) whose epilogue applies ReLU, rounds
- * to half precision and writes X and AT; the loss and the output delta;
- * then for each layer from the last, dW += AT^T-shaped MMA (M = 64: the
- * layer's 64 inputs, N = its outputs, K = the 128 rows), accumulated in
- * TMEM over every tile of the block, and the delta of the layer input
- * (M = 128, N = 64, K = outputs) masked by ReLU'.  With M = 64 the
- * accumulator's rows 16q..16q+15 are TMEM lanes 32q..32q+15.  At the end
+ * One CTA an SM: two chains of 128 threads, each walking tiles of 128 rows
+ * (thread = row = TMEM lane), and a warp that issues every MMA.  All operands
+ * are in the canonical layout without swizzle (8 x 8 core matrices of 128
+ * contiguous bytes, column neighbours 128 bytes apart, 8-row groups 1024), and
+ * each is stored once and read both ways, K-major or, with the descriptor's
+ * offsets exchanged and the instruction's transpose bit, MN-major:
+ *   W    the six layers' weights [out][in] (42 KB): the forward's B operand
+ *        as it is, the delta's transposed;
+ *   A    a layer's input [128][64]: the forward's A operand as it is, dW's
+ *        transposed;
+ *   D    the delta of a layer's output: the A operand of the delta of its
+ *        input as it is, dW's B operand transposed.
+ * A chain has five tiles of 16 KB and one [128][16] for the output's delta.
+ * With A(l) the input of layer l, tile b(i) holds X = A(0) and then A(1) for
+ * i = 0, else A(i + 1).  Twelve stages a tile, every one MMAs and then the
+ * chain's epilogue of their result:
+ *   forward l = 0..5    A(l) x W(l); ReLU, rounded, is A(l + 1) in b(l); the
+ *                       last epilogue is the loss and the output's delta D(5);
+ *   backward l = 5..0   dW(l) += A(l)^T D(l) (M = 64 inputs, N = outputs, K =
+ *                       the 128 rows) and, but for l = 0, D(l) x W(l)^T; masked
+ *                       by A(l) > 0 and rounded it is D(l - 1), which takes
+ *                       A(l)'s place in b(l - 1).
+ * X, overwritten by A(1), comes back into b(4) when stage 4 has read it, and
+ * the next tile's X into b(3) when stage 3 has: the next tile counts its tiles
+ * from there.  Both come by asynchronous copies under the other stages.
+ *
+ * The chains need not meet at any barrier: a thread writes its own row only,
+ * and a chain's `ready` mbarrier (one arrival a warp) releases the issuer,
+ * whose commit releases the chain (`done`).  The issuer takes the chains in
+ * turn, stage by stage, so one chain's epilogue runs under the other's MMAs,
+ * and dW, which both add to in tensor memory, is summed in the order of the
+ * block's tiles.  TMEM: 64 columns of accumulator a chain, 64 a dW (16 for the
+ * last; with M = 64 its rows 16q..16q+15 are lanes 32q..32q+15).  At the end
  * the block writes its dW to its slice of `partial`, which the host sums in
- * block order; the rounding points are those of mlp_train_kernel. */
+ * block order; the rounding points are those of mlp_train_kernel.
+ *
+ * What bounds it is the latency of a stage (arrive, issue, MMA, commit, read,
+ * convert, store), which the second chain hides half of; the tensor cores are
+ * busy for about a quarter of the time.  Operands stored a second time,
+ * transposed two bytes at a time with bank conflicts, the weights in both
+ * layouts, one chain of 128 threads and a barrier on either side of every
+ * stage: 114 us for 65,536 rows of FP16, this kernel 34 (a training step 125
+ * and 53 us).
+ *
+ * Every wait is bounded; a warp whose wait runs out leaves, so that every
+ * later wait of its chain and of the issuer runs out too, and bit 0 of the
+ * error word is set. */
 #define TT_ROWS 128
-#define TT_SBO16 256u
-#define TT_SBO64 1024u
-#define TT_SBO128 2048u
-#define TT_WN_OFF TC_W_BYTES                      /* 43,008 */
-#define TT_WN_BYTES (4u * TC_LAYER_BYTES + 2048u) /* layers 1..4, then layer 5 (K = 16) */
-#define TT_X_OFF (TT_WN_OFF + TT_WN_BYTES)        /* 77,824 */
+#define TT_CHAINS 2
+#define TT_THREADS (128 * TT_CHAINS + 32)
 #define TT_TILE_BYTES (TT_ROWS * TC_W * 2u)       /* 16 KB */
-#define TT_AT_OFF (TT_X_OFF + TT_TILE_BYTES)
-#define TT_D_OFF (TT_AT_OFF + 6u * TT_TILE_BYTES)
-#define TT_DT_OFF (TT_D_OFF + TT_TILE_BYTES)
-#define TT_BAR_OFF (TT_DT_OFF + TT_TILE_BYTES)    /* 225,280 */
-#define TT_SLOT_OFF (TT_BAR_OFF + 8u)
-#define TT_SMEM (TT_SLOT_OFF + 8u)
+#define TT_BUFS 5u
+#define TT_CHAIN_OFF TC_W_BYTES                   /* 43,008 */
+#define TT_CHAIN_BYTES (TT_BUFS * TT_TILE_BYTES + TT_ROWS * TC_OUT * 2u)
+#define TT_BAR_OFF (TT_CHAIN_OFF + TT_CHAINS * TT_CHAIN_BYTES) /* per chain: ready, done */
+#define TT_SLOT_OFF (TT_BAR_OFF + TT_CHAINS * 16u)
+#define TT_SMEM (TT_SLOT_OFF + 8u)              /* 215,080 bytes */
 #define TT_TMEM_COLS 512u
-#define TT_DW_COL(l) (64u + 64u * (uint32_t)(l))   /* dW of layer l (layer 5: 16 columns) */
+#define TT_WAIT_LIMIT (1u << 18)    /* mbarrier polls before a wait gives up */
+#define TT_DW_COL(l) (64u * TT_CHAINS + 64u * (uint32_t)(l))   /* dW of layer l (layer 5: 16 columns) */
+#define TT_TRANSPOSE_A (1u << 15)                 /* instruction descriptor: MN-major operands */
+#define TT_TRANSPOSE_B (1u << 16)
 
-__device__ __forceinline__ uint32_t kmaj_off(uint32_t r, uint32_t k, uint32_t sbo)
+/* 16 bytes from global to shared memory without a register; zeros if !valid
+ * (src must be readable memory all the same). */
+__device__ __forceinline__ void copy16(uint32_t dst, const void *src, bool valid)
 {
-	return (r >> 3) * sbo + (k >> 3) * 128u + (r & 7u) * 16u + (k & 7u) * 2u;
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(valid ? 16u : 0u)
+		: "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+/* Rows 8g..8g+7 of a [rows][64] matrix by one warp: eight lanes write a core
+ * matrix (no bank conflict), four read a row's half (whole sectors). */
+template <class T>
+__device__ __forceinline__ void copy_rows8(uint32_t dst, const T *src, uint32_t g, uint32_t lane, bool valid)
+{
+	const uint32_t r = lane & 7u, c = lane >> 3;
+#pragma unroll
+	for (uint32_t h = 0; h < 2; h++)
+		copy16(dst + g * TC_SBO + (c + 4u * h) * TC_LBO + r * 16u,
+			src + (valid ? (size_t)(8u * g + r) * TC_W + (c + 4u * h) * 8u : 0), valid);
 }
 
-__device__ __forceinline__ uint32_t wn_off(int l)
+/* Two values rounded to half precision. */
+template <class T>
+__device__ __forceinline__ uint32_t pack2(float lo, float hi)
 {
-	return TT_WN_OFF + (l < TC_LAYERS - 1 ? (uint32_t)(l - 1) * TC_LAYER_BYTES : 4u * TC_LAYER_BYTES);
+	uint32_t r;
+	if (std::is_same<T, __nv_bfloat16>::value)
+		asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+	else
+		asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+	return r;
+}
+
+/* ReLU of two halves: a NaN and a negative zero are +0. */
+template <class T>
+__device__ __forceinline__ uint32_t relu2(uint32_t v)
+{
+	uint32_t r;
+	if (std::is_same<T, __nv_bfloat16>::value)
+		asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
+	else
+		asm("max.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0u));
+	return r;
+}
+
+/* 0xFFFF in each half of two ReLU outputs (no sign, no NaN) that is not zero. */
+__device__ __forceinline__ uint32_t positive2(uint32_t a)
+{
+	uint32_t r;
+	asm("prmt.b32 %0, %1, %2, 0xBB99;" : "=r"(r) : "r"(a + 0x7FFF7FFFu), "r"(0u));
+	return r;
 }
 
 template <class T>
-__device__ __forceinline__ T half_bits(uint16_t b)
-{
-	T h;
-	*reinterpret_cast<uint16_t *>(&h) = b;
-	return h;
-}
-
-template <class T>
-__device__ __forceinline__ uint16_t bits_of(T h)
-{
-	return *reinterpret_cast<uint16_t *>(&h);
-}
-
-template <class T>
-__device__ __forceinline__ float half_to_float(T h);
-template <>
-__device__ __forceinline__ float half_to_float<__nv_bfloat16>(__nv_bfloat16 h) { return __bfloat162float(h); }
-template <>
-__device__ __forceinline__ float half_to_float<__half>(__half h) { return __half2float(h); }
-
-template <class T>
-__device__ __forceinline__ T float_to_half(float f);
-template <>
-__device__ __forceinline__ __nv_bfloat16 float_to_half<__nv_bfloat16>(float f) { return __float2bfloat16_rn(f); }
-template <>
-__device__ __forceinline__ __half float_to_half<__half>(float f) { return __float2half_rn(f); }
-
-/* A row of 8 halves (one 16-byte chunk) from 8 values. */
-template <class T>
-__device__ __forceinline__ uint4 pack8(const uint16_t (&h)[8])
-{
-	uint4 p;
-	p.x = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
-	p.y = (uint32_t)h[2] | ((uint32_t)h[3] << 16);
-	p.z = (uint32_t)h[4] | ((uint32_t)h[5] << 16);
-	p.w = (uint32_t)h[6] | ((uint32_t)h[7] << 16);
-	return p;
-}
-
-template <class T>
-__global__ void __launch_bounds__(128, 1) mlp_train_tc_kernel(const T *__restrict__ wt_g, const T *__restrict__ wn_g,
+__global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__restrict__ wt_g,
 		const T *__restrict__ x, const float4 *__restrict__ target, uint32_t n, float *__restrict__ partial,
 		float *__restrict__ loss_sum, const uint32_t *__restrict__ n_dev, uint32_t *__restrict__ err)
 {
@@ -542,33 +571,36 @@ __global__ void __launch_bounds__(128, 1) mlp_train_tc_kernel(const T *__restric
 		n = c < n ? c : n;
 	}
 	extern __shared__ __align__(1024) unsigned char sm[];
-	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+	const int tid = threadIdx.x, warp = tid >> 5;
+	const uint32_t lane = (uint32_t)tid & 31u;
+	const int chain = warp >> 2; /* TT_CHAINS: the issuer */
+	const uint32_t cwarp = (uint32_t)warp & 3u;
 	const bool bf16 = std::is_same<T, __nv_bfloat16>::value;
-	const uint32_t bar = smem_addr(sm + TT_BAR_OFF);
+	const uint32_t base = smem_addr(sm), bars = base + TT_BAR_OFF;
 	uint32_t *slot = reinterpret_cast<uint32_t *>(sm + TT_SLOT_OFF);
 	const uint32_t tiles = (n + TT_ROWS - 1) / TT_ROWS;
+	const uint32_t tile0 = base + TT_CHAIN_OFF + (uint32_t)chain * TT_CHAIN_BYTES;
 
-	/* weights: forward [out][in], then layers 1..5 as [in][out] */
-	for (int l = 0; l < TC_LAYERS; l++) {
-		int rows = l == TC_LAYERS - 1 ? TC_OUT : TC_W;
-		const uint4 *src = reinterpret_cast<const uint4 *>(wt_g + (size_t)l * TC_W * TC_W);
-		unsigned char *dst = sm + l * TC_LAYER_BYTES;
-		for (int c = tid; c < rows * 8; c += 128) {
-			uint32_t r = (uint32_t)c >> 3, kb = (uint32_t)c & 7u;
-			*reinterpret_cast<uint4 *>(dst + kmaj_off(r, kb * 8u, TT_SBO64)) = __ldg(src + c);
+	/* this warp's 32 rows of X of a tile */
+	auto copy_x = [&](uint32_t buf, uint32_t tile) {
+#pragma unroll
+		for (uint32_t g = 0; g < 4; g++) {
+			const uint32_t row = 32u * cwarp + 8u * g + (lane & 7u);
+			const bool valid = (size_t)tile * TT_ROWS + row < n;
+			copy_rows8(tile0 + buf * TT_TILE_BYTES, valid ? x + (size_t)tile * TT_ROWS * TC_W : x, 4u * cwarp + g,
+				lane, valid);
 		}
-	}
-	for (int l = 1; l < TC_LAYERS; l++) {
-		uint32_t cols = l == TC_LAYERS - 1 ? TC_OUT : TC_W, chunks = cols / 8u, sbo = chunks * 128u;
-		const uint4 *src = reinterpret_cast<const uint4 *>(wn_g + (size_t)l * TC_W * TC_W);
-		unsigned char *dst = sm + wn_off(l);
-		for (uint32_t c = (uint32_t)tid; c < TC_W * chunks; c += 128u) {
-			uint32_t r = c / chunks, kb = c % chunks;
-			*reinterpret_cast<uint4 *>(dst + kmaj_off(r, kb * 8u, sbo)) = __ldg(src + c);
-		}
-	}
+	};
+	uint32_t t = blockIdx.x + gridDim.x * (uint32_t)chain;
+	const uint32_t stride = gridDim.x * TT_CHAINS;
+	if (chain < TT_CHAINS && t < tiles)
+		copy_x(0, t);
+	for (uint32_t g = (uint32_t)warp; g < 42u; g += TT_THREADS / 32) /* 5 x 8 groups of rows, 2 of the last layer */
+		copy_rows8(base, wt_g, g, lane, true);
 	if (tid == 0) {
-		asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(1u) : "memory");
+		for (uint32_t i = 0; i < 2u * TT_CHAINS; i++)
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bars + 8u * i), "r"(i & 1u ? 1u : 4u)
+				: "memory");
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
 	if (warp == 0) {
@@ -576,202 +608,223 @@ __global__ void __launch_bounds__(128, 1) mlp_train_tc_kernel(const T *__restric
 			:: "r"(smem_addr(slot)), "r"(TT_TMEM_COLS) : "memory");
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 	}
+	copy_wait();
 	fence_async_smem();
 	tc_before();
 	__syncthreads();
 	tc_after();
 	const uint32_t tmem = *slot;
-	const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
-	const uint32_t base = smem_addr(sm);
-	const uint32_t id_hidden = instr_desc(bf16, TC_W, TT_ROWS), id_out = instr_desc(bf16, TC_OUT, TT_ROWS);
-	const uint32_t id_dw = instr_desc(bf16, TC_W, 64), id_dw_out = instr_desc(bf16, TC_OUT, 64);
-	const uint32_t r = (uint32_t)tid; /* this thread's row of the tile, and its TMEM lane */
-	unsigned char *xs = sm + TT_X_OFF, *ds = sm + TT_D_OFF, *dts = sm + TT_DT_OFF;
-	uint32_t parity = 0;
-	bool ok = true, first = true;
+	bool ok = true;
 	float lsum = 0.0f;
 
-	/* wait for the committed MMAs, then make the epilogue's view current */
-	auto mma_wait = [&]() -> bool {
-		bool got = bar_wait(bar, parity, TC_WAIT_LIMIT);
-		parity ^= 1u;
-		bool all = __syncthreads_and(got) != 0;
-		tc_after();
-		return all;
-	};
-	/* make this thread's shared-memory writes visible to the MMAs */
-	auto publish = [&]() {
-		fence_async_smem();
-		tc_before();
-		__syncthreads();
-		tc_after();
-	};
-
-	for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-		const size_t gr = (size_t)t * TT_ROWS + r;
-		/* ---- the tile's input: X (row r) and AT[0] (column r) ---- */
-		{
-			uint4 c[8];
-			const uint4 *src = reinterpret_cast<const uint4 *>(x + gr * TC_W);
+	if (chain == TT_CHAINS) {
+		/* ---- the issuer ---- */
+		if (lane == 0) {
+			const uint32_t id_hidden = instr_desc(bf16, TC_W, TT_ROWS), id_out = instr_desc(bf16, TC_OUT, TT_ROWS);
+			const uint32_t id_dw = instr_desc(bf16, TC_W, 64) | TT_TRANSPOSE_A | TT_TRANSPOSE_B;
+			const uint32_t id_dw_out = instr_desc(bf16, TC_OUT, 64) | TT_TRANSPOSE_A | TT_TRANSPOSE_B;
+			const uint32_t id_delta = id_hidden | TT_TRANSPOSE_B;
+			/* a [][64] matrix as it is and transposed, a [][16] one the same; an
+			 * address adds to the address field (16-byte units, all below 2^14) */
+			const uint64_t k64 = smem_desc(0u, TC_LBO, TC_SBO, 0u), m64 = smem_desc(0u, TC_SBO, TC_LBO, 0u);
+			const uint64_t k16 = smem_desc(0u, 128u, 256u, 0u), m16 = smem_desc(0u, 256u, 128u, 0u);
+			uint32_t phase = 0, start = 0;
+			for (uint32_t b = blockIdx.x; ok && b < tiles; b += stride) {
+				const uint32_t chains = b + gridDim.x < tiles ? 2u : 1u;
+				for (int s = 0; ok && s < 2 * TC_LAYERS; s++) {
+					const bool backward = s >= TC_LAYERS;
+					const uint32_t l = backward ? 2u * TC_LAYERS - 1u - (uint32_t)s : (uint32_t)s;
+					const bool last = l == TC_LAYERS - 1;
+					/* the tiles of A(l) (l > 0) and of D(l) (l < 5) */
+					uint32_t ia = start + (l > 0 ? l - 1u : backward ? 4u : 0u), id = start + l;
+					ia -= ia >= TT_BUFS ? TT_BUFS : 0u;
+					id -= id >= TT_BUFS ? TT_BUFS : 0u;
+					const uint32_t w = (base + l * TC_LAYER_BYTES) >> 4;
+					for (uint32_t c = 0; ok && c < chains; c++) {
+						const uint32_t bar = bars + 16u * c, buf0 = base + TT_CHAIN_OFF + c * TT_CHAIN_BYTES;
+						const uint32_t a = (buf0 + ia * TT_TILE_BYTES) >> 4;
+						const uint32_t d = (buf0 + (last ? TT_BUFS : id) * TT_TILE_BYTES) >> 4;
+						const uint32_t acc = tmem + 64u * c;
+						/* X of the first tile came before the CTA's barrier, of a
+						 * later one with the last D(0) */
+						if (s > 0 && !(ok = bar_wait(bar, phase, TT_WAIT_LIMIT)))
+							break;
+						tc_after();
+						if (!backward) {
 #pragma unroll
-			for (int kb = 0; kb < 8; kb++)
-				c[kb] = gr < n ? __ldg(src + kb) : make_uint4(0u, 0u, 0u, 0u);
-			unsigned char *at = sm + TT_AT_OFF;
+							for (uint32_t kc = 0; kc < 4; kc++)
+								tc_mma(acc, k64 + a + kc * 16u, k64 + w + kc * 16u, last ? id_out : id_hidden,
+									kc > 0 ? 1u : 0u);
+						} else {
+							const uint32_t sum = b != blockIdx.x || c > 0 ? 1u : 0u;
 #pragma unroll
-			for (int kb = 0; kb < 8; kb++) {
-				*reinterpret_cast<uint4 *>(xs + kmaj_off(r, kb * 8u, TT_SBO64)) = c[kb];
-				const uint32_t w4[4] = {c[kb].x, c[kb].y, c[kb].z, c[kb].w};
+							for (uint32_t kc = 0; kc < 8; kc++)
+								tc_mma(tmem + TT_DW_COL(l), m64 + a + kc * 128u,
+									last ? m16 + d + kc * 32u : m64 + d + kc * 128u, last ? id_dw_out : id_dw,
+									kc > 0 ? 1u : sum);
+							if (last) {
+								tc_mma(acc, k16 + d, m64 + w, id_delta, 0u);
+							} else if (l > 0) {
 #pragma unroll
-				for (int e = 0; e < 8; e++) {
-					uint16_t h = (uint16_t)(w4[e >> 1] >> (16 * (e & 1)));
-					*reinterpret_cast<uint16_t *>(at + kmaj_off((uint32_t)(kb * 8 + e), r, TT_SBO128)) = h;
+								for (uint32_t kc = 0; kc < 4; kc++)
+									tc_mma(acc, k64 + d + kc * 16u, m64 + w + kc * 128u, id_delta, kc > 0 ? 1u : 0u);
+							}
+						}
+						/* nobody waits for a tile's last stage but the end */
+						if (s < 2 * TC_LAYERS - 1 || b + gridDim.x * c + stride >= tiles)
+							tc_commit(bar + 8u);
+					}
+					if (s > 0)
+						phase ^= 1u;
 				}
+				start = start >= 2u ? start - 2u : start + 3u;
 			}
 		}
-		publish();
-		/* ---- forward ---- */
-		for (int l = 0; l < TC_LAYERS && ok; l++) {
-			const bool last = l == TC_LAYERS - 1;
-			if (tid == 0) {
-				for (uint32_t kc = 0; kc < 4; kc++)
-					tc_mma(tmem, smem_desc(base + TT_X_OFF + kc * 256u, TC_LBO, TT_SBO64, 0u),
-						smem_desc(base + l * TC_LAYER_BYTES + kc * 256u, TC_LBO, TT_SBO64, 0u),
-						last ? id_out : id_hidden, kc > 0 ? 1u : 0u);
-				tc_commit(bar);
-			}
-			ok = mma_wait();
-			if (!ok)
-				break;
-			if (!last) {
+		ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+	} else {
+		/* ---- a chain ---- */
+		const uint32_t ready = bars + 16u * (uint32_t)chain, done = ready + 8u;
+		const uint32_t acc = tmem + 64u * (uint32_t)chain + ((32u * cwarp) << 16);
+		const uint32_t row = 32u * cwarp + lane;
+		unsigned char *mine = sm + TT_CHAIN_OFF + (uint32_t)chain * TT_CHAIN_BYTES + (row >> 3) * TC_SBO + (row & 7u) * 16u;
+		uint32_t phase = 0, start = 0;
+		auto at = [&](uint32_t i) -> uint32_t {
+			i += start;
+			return i >= TT_BUFS ? i - TT_BUFS : i;
+		};
+		/* wait for the committed MMAs */
+		auto wait = [&]() -> bool {
+			bool got = bar_wait(done, phase, TT_WAIT_LIMIT);
+			phase ^= 1u;
+			got = __all_sync(0xffffffffu, got) != 0;
+			tc_after();
+			return got;
+		};
+		/* this warp's rows are written and its lanes read */
+		auto publish = [&]() {
+			fence_async_smem();
+			tc_before();
+			__syncwarp();
+			if (lane == 0)
+				asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(ready) : "memory");
+		};
+		while (ok && t < tiles) {
+			const size_t gr = (size_t)t * TT_ROWS + row;
+			const float4 tg = gr < n ? __ldg(target + gr) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+			/* ---- forward ---- */
+			for (uint32_t l = 0; l < TC_LAYERS - 1; l++) {
+				ok = wait();
+				if (!ok)
+					break;
 				uint32_t v[64];
-				tmem_ld64(lane_addr, v);
+				tmem_ld64(acc, v);
 				tmem_wait_ld();
-				unsigned char *at = sm + TT_AT_OFF + (uint32_t)(l + 1) * TT_TILE_BYTES;
+				unsigned char *dst = mine + at(l) * TT_TILE_BYTES;
 #pragma unroll
-				for (uint32_t kb = 0; kb < 8; kb++) {
-					uint16_t h[8];
+				for (int kb = 0; kb < 8; kb++) {
+					uint32_t h[4];
 #pragma unroll
-					for (int e = 0; e < 8; e++) {
-						h[e] = bits_of<T>(float_to_half<T>(fmaxf(__uint_as_float(v[8 * kb + e]), 0.0f)));
-						*reinterpret_cast<uint16_t *>(at + kmaj_off(8u * kb + (uint32_t)e, r, TT_SBO128)) = h[e];
-					}
-					*reinterpret_cast<uint4 *>(xs + kmaj_off(r, kb * 8u, TT_SBO64)) = pack8<T>(h);
+					for (int e = 0; e < 4; e++)
+						h[e] = relu2<T>(pack2<T>(__uint_as_float(v[8 * kb + 2 * e]), __uint_as_float(v[8 * kb + 2 * e + 1])));
+					*reinterpret_cast<uint4 *>(dst + kb * TC_LBO) = make_uint4(h[0], h[1], h[2], h[3]);
 				}
-			} else {
-				/* the loss and the output delta (columns 0..15, 0..2 non-zero) */
+				publish();
+			}
+			if (!ok || !(ok = wait()))
+				break;
+			/* ---- the loss and the output's delta (columns 0..2 of 16) ---- */
+			{
 				uint32_t v[16];
-				tmem_ld16(lane_addr, v);
+				tmem_ld16(acc, v);
 				tmem_wait_ld();
-				float4 tg = gr < n ? target[gr] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 				const float tv[3] = {tg.x, tg.y, tg.z};
-				uint16_t h[16];
+				float d[3] = {0.0f, 0.0f, 0.0f};
+				if (gr < n) {
 #pragma unroll
-				for (int col = 0; col < 16; col++) {
-					float d = 0.0f;
-					if (col < 3 && gr < n) {
+					for (int col = 0; col < 3; col++) {
 						float y = __uint_as_float(v[col]);
 						float diff = y - tv[col];
 						float den = y * y + 0.01f;
 						lsum += diff * diff / den;
-						d = 2.0f * diff / den / (float)n;
+						d[col] = 2.0f * diff / den / (float)n;
 					}
-					h[col] = bits_of<T>(float_to_half<T>(d));
-					*reinterpret_cast<uint16_t *>(dts + kmaj_off((uint32_t)col, r, TT_SBO128)) = h[col];
 				}
-				uint16_t lo[8], hi[8];
-#pragma unroll
-				for (int e = 0; e < 8; e++) {
-					lo[e] = h[e];
-					hi[e] = h[8 + e];
-				}
-				*reinterpret_cast<uint4 *>(ds + kmaj_off(r, 0u, TT_SBO16)) = pack8<T>(lo);
-				*reinterpret_cast<uint4 *>(ds + kmaj_off(r, 8u, TT_SBO16)) = pack8<T>(hi);
+				unsigned char *dst = sm + TT_CHAIN_OFF + (uint32_t)chain * TT_CHAIN_BYTES + TT_BUFS * TT_TILE_BYTES
+					+ (row >> 3) * 256u + (row & 7u) * 16u;
+				*reinterpret_cast<uint4 *>(dst) = make_uint4(pack2<T>(d[0], d[1]), pack2<T>(d[2], 0.0f), 0u, 0u);
+				*reinterpret_cast<uint4 *>(dst + 128u) = make_uint4(0u, 0u, 0u, 0u);
 			}
 			publish();
-		}
-		/* ---- backward ---- */
-		for (int l = TC_LAYERS - 1; l >= 0 && ok; l--) {
-			const uint32_t cols = l == TC_LAYERS - 1 ? TC_OUT : TC_W;
-			const uint32_t sbo_d = cols / 8u * 128u;
-			if (tid == 0) {
-				/* dW[l] (+)= AT[l] x DT: M = 64 inputs, N = cols outputs, K = 128 rows */
-				for (uint32_t kc = 0; kc < 8; kc++)
-					tc_mma(tmem + TT_DW_COL(l),
-						smem_desc(base + TT_AT_OFF + (uint32_t)l * TT_TILE_BYTES + kc * 256u, TC_LBO, TT_SBO128, 0u),
-						smem_desc(base + TT_DT_OFF + kc * 256u, TC_LBO, TT_SBO128, 0u),
-						l == TC_LAYERS - 1 ? id_dw_out : id_dw, (!first || kc > 0) ? 1u : 0u);
-				/* the delta of the layer input: D x WN[l], M = 128, N = 64, K = cols */
-				if (l > 0)
-					for (uint32_t kc = 0; kc < cols / 16u; kc++)
-						tc_mma(tmem, smem_desc(base + TT_D_OFF + kc * 256u, TC_LBO, sbo_d, 0u),
-							smem_desc(base + wn_off(l) + kc * 256u, TC_LBO, sbo_d, 0u), id_hidden,
-							kc > 0 ? 1u : 0u);
-				tc_commit(bar);
-			}
-			ok = mma_wait();
-			if (!ok || l == 0)
-				break;
-			uint32_t v[64];
-			tmem_ld64(lane_addr, v);
-			tmem_wait_ld();
-			const unsigned char *at = sm + TT_AT_OFF + (uint32_t)l * TT_TILE_BYTES;
+			/* ---- backward ---- */
+			for (uint32_t l = TC_LAYERS - 1; l > 0; l--) {
+				ok = wait();
+				if (!ok)
+					break;
+				if (l == 4)
+					copy_x(at(4), t);
+				if (l == 3 && t + stride < tiles)
+					copy_x(at(3), t + stride);
+				uint32_t v[64];
+				tmem_ld64(acc, v);
+				tmem_wait_ld();
+				unsigned char *dst = mine + at(l - 1) * TT_TILE_BYTES;
 #pragma unroll
-			for (uint32_t kb = 0; kb < 8; kb++) {
-				uint16_t h[8];
+				for (int kb = 0; kb < 8; kb++) {
+					uint4 *p = reinterpret_cast<uint4 *>(dst + kb * TC_LBO);
+					const uint4 a = *p;
+					const uint32_t m[4] = {a.x, a.y, a.z, a.w};
+					uint32_t h[4];
 #pragma unroll
-				for (int e = 0; e < 8; e++) {
-					uint32_t i = 8u * kb + (uint32_t)e;
-					float av = half_to_float<T>(half_bits<T>(*reinterpret_cast<const uint16_t *>(
-						at + kmaj_off(i, r, TT_SBO128))));
-					float d = av > 0.0f ? __uint_as_float(v[i]) : 0.0f;
-					h[e] = bits_of<T>(float_to_half<T>(d));
-					*reinterpret_cast<uint16_t *>(dts + kmaj_off(i, r, TT_SBO128)) = h[e];
+					for (int e = 0; e < 4; e++)
+						h[e] = pack2<T>(__uint_as_float(v[8 * kb + 2 * e]), __uint_as_float(v[8 * kb + 2 * e + 1])) & positive2(m[e]);
+					*p = make_uint4(h[0], h[1], h[2], h[3]);
 				}
-				*reinterpret_cast<uint4 *>(ds + kmaj_off(r, kb * 8u, TT_SBO64)) = pack8<T>(h);
+				if (l == 1) /* X is back, and the next tile's is there: the issuer goes on without another arrival */
+					copy_wait();
+				publish();
 			}
-			publish();
+			if (ok && t + stride >= tiles)
+				ok = wait();
+			start = start >= 2u ? start - 2u : start + 3u;
+			t += stride;
 		}
-		first = false;
+		copy_wait();
 	}
+	tc_before();
+	ok = __syncthreads_and(ok) != 0;
+	tc_after();
 	if (!ok && tid == 0)
 		atomicOr(err, 1u);
-	tc_before();
-	__syncthreads();
-	tc_after();
-	/* this block's dW: lanes 32w..32w+15 hold rows 16w..16w+15 */
-	float *dst = partial + (size_t)blockIdx.x * TC_LAYERS * TC_W * TC_W;
-	for (int l = 0; l < TC_LAYERS; l++) {
-		const uint32_t cols = l == TC_LAYERS - 1 ? TC_OUT : TC_W;
-		const uint32_t i = 16u * (uint32_t)warp + (uint32_t)lane;
-		uint32_t v[64];
-		if (cols == TC_W) {
-			tmem_ld64(lane_addr + TT_DW_COL(l), v);
-		} else {
-			uint32_t w16[16];
-			tmem_ld16(lane_addr + TT_DW_COL(l), w16);
+	/* this block's dW: lanes 32q..32q+15 hold rows 16q..16q+15 of 64 */
+	if (chain < TT_CHAINS) {
+		float *dst = partial + (size_t)blockIdx.x * TC_LAYERS * TC_W * TC_W + (size_t)(16u * cwarp + (lane & 15u)) * TC_W;
+		const bool valid = ok && blockIdx.x < tiles;
+		for (int l = chain; l < TC_LAYERS; l += TT_CHAINS) {
+			uint32_t v[64];
+			const uint32_t col = tmem + ((32u * cwarp) << 16) + TT_DW_COL(l);
+			if (l < TC_LAYERS - 1) {
+				tmem_ld64(col, v);
+			} else {
+				uint32_t w16[16];
+				tmem_ld16(col, w16);
 #pragma unroll
-			for (int j = 0; j < 16; j++)
-				v[j] = w16[j];
+				for (int j = 0; j < 64; j++)
+					v[j] = j < 16 ? w16[j & 15] : 0u;
+			}
+			tmem_wait_ld();
+			if (lane < 16) {
+				float *out = dst + (size_t)l * TC_W * TC_W;
 #pragma unroll
-			for (int j = 16; j < 64; j++)
-				v[j] = 0u;
+				for (int j = 0; j < 64; j += 4)
+					*reinterpret_cast<uint4 *>(out + j) = valid ? make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3])
+						: make_uint4(0u, 0u, 0u, 0u);
+			}
 		}
-		tmem_wait_ld();
-		if (lane < 16) {
-			float *row = dst + (size_t)l * TC_W * TC_W + (size_t)i * TC_W;
-			const bool valid = ok && !first;
-#pragma unroll
-			for (int j = 0; j < 64; j += 4)
-				*reinterpret_cast<float4 *>(row + j) = valid
-					? make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]),
-						__uint_as_float(v[j + 3]))
-					: make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-		}
+		for (int off = 16; off > 0; off >>= 1)
+			lsum += __shfl_down_sync(0xffffffffu, lsum, off);
+		if (lane == 0)
+			atomicAdd(loss_sum, lsum);
 	}
-	for (int off = 16; off > 0; off >>= 1)
-		lsum += __shfl_down_sync(0xffffffffu, lsum, off);
-	if (lane == 0)
-		atomicAdd(loss_sum, lsum);
 	tc_before();
 	__syncthreads();
 	tc_after();
@@ -823,15 +876,13 @@ void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint
 	if (mp.dtype == KGR_MLP_BF16) {
 		static bool once = (set_train_smem(mlp_train_tc_kernel<__nv_bfloat16>), true);
 		(void)once;
-		mlp_train_tc_kernel<__nv_bfloat16><<<grid, 128, TT_SMEM, st>>>(static_cast<const __nv_bfloat16 *>(mp.wt),
-			static_cast<const __nv_bfloat16 *>(mp.wn), static_cast<const __nv_bfloat16 *>(x), target, n, mp.partial,
-			loss, n_dev, mp.tc_err);
+		mlp_train_tc_kernel<__nv_bfloat16><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const __nv_bfloat16 *>(mp.wt),
+			static_cast<const __nv_bfloat16 *>(x), target, n, mp.partial, loss, n_dev, mp.tc_err);
 	} else {
 		static bool once = (set_train_smem(mlp_train_tc_kernel<__half>), true);
 		(void)once;
-		mlp_train_tc_kernel<__half><<<grid, 128, TT_SMEM, st>>>(static_cast<const __half *>(mp.wt),
-			static_cast<const __half *>(mp.wn), static_cast<const __half *>(x), target, n, mp.partial, loss, n_dev,
-			mp.tc_err);
+		mlp_train_tc_kernel<__half><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const __half *>(mp.wt),
+			static_cast<const __half *>(x), target, n, mp.partial, loss, n_dev, mp.tc_err);
 	}
 	KGR_CUDA(cudaGetLastError());
 }

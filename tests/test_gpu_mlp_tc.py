@@ -190,3 +190,27 @@ def test_tile_counts_and_non_finite_rows(dtype, n):
         got[kernel] = out.cpu().numpy()
     net.check()
     np.testing.assert_allclose(got["tcgen05"], got["mma"], rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("tiles,rest", [(1, -127), (1, 1), (152, 1), (304, 0), (304, 1), (456, -1), (608, 130)])
+def test_training_tile_counts(dtype, tiles, rest):
+    """Tiles at the edges of the chains' split on 152 SMs (one chain, both,
+    two and three tiles a chain, a ragged last): the mma.sync gradients within
+    1e-2 of each layer's norm, and the same bits on a second pass."""
+    n = 128 * tiles + rest
+    rng = np.random.default_rng(n)
+    x = np.tile(mlp_ref.encode_inputs(rng, min(n, 4096), dtype), (-(-n // 4096), 1))[:n]
+    t = np.zeros((n, 4), np.float32)
+    t[:, :3] = rng.uniform(0, 2, (n, 3))
+    xd, td = half_tensor(x, dtype), torch.from_numpy(t).cuda()
+    net = kgr.Mlp(dtype, seed=9)
+    loss_tc, g_tc = gradients(net, "tcgen05", xd, td, n)
+    loss_mma, g_mma = gradients(net, "mma", xd, td, n)
+    assert abs(loss_tc - loss_mma) <= 1e-3 * abs(loss_mma)
+    for l in range(6):
+        a, c = g_tc[l], g_mma[l]
+        assert np.linalg.norm(a - c) <= 1e-2 * np.linalg.norm(c) + 1e-9, l
+    _, again = gradients(net, "tcgen05", xd, td, n)
+    assert np.array_equal(np.asarray(g_tc).view(np.uint32), np.asarray(again).view(np.uint32))
+    net.check()
