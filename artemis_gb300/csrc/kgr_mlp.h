@@ -13,6 +13,9 @@ namespace kgr {
 
 #define KGR_MLP_PARAMS (6 * 64 * 64)
 #define KGR_MLP_INPUTS 64
+/* a slice of the gradient scratch: the loss of its block, among the unused
+ * outputs of the last layer */
+#define MLP_LOSS_SLOT (5 * 64 * 64 + 16)
 
 struct MlpParams {
 	int dtype; /* KGR_MLP_BF16 or KGR_MLP_FP16 */
@@ -36,10 +39,11 @@ void mlp_infer(const MlpParams &mp, const void *x, uint32_t n, float4 *out, cuda
 void mlp_infer_tc(const MlpParams &mp, const void *x, uint32_t n, float4 *out, uint32_t *err, cudaStream_t st,
 		const uint32_t *n_dev = nullptr, bool withhold_first = false);
 /* The gradient pass of mlp_gradients on the tensor cores (mlp_tc.cu):
- * grid blocks write their slices of mp.partial (tiles of 128 rows) and add
- * their loss into *loss; sets bit 0 of *mp.tc_err if a wait ran out. */
-void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, float *loss,
-		cudaStream_t st, const uint32_t *n_dev);
+ * grid blocks write their slices of mp.partial (tiles of 128 rows), each with
+ * its loss in the slice's MLP_LOSS_SLOT and nothing in the other unused
+ * outputs; sets bit 0 of *mp.tc_err if a wait ran out. */
+void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, cudaStream_t st,
+		const uint32_t *n_dev);
 /* grad (FP32, [6][64][64]) = d loss / d W over n rows; loss = sum of the
  * relative L2 terms (not divided by n).  Uses mp.partial as scratch; the
  * result does not depend on block scheduling.  max_blocks > 0 caps the grid
@@ -52,6 +56,10 @@ void mlp_gradients(const MlpParams &mp, const void *x, const float4 *target, uin
 void mlp_adam(const MlpParams &mp, const float *grad, float lr, int step, cudaStream_t st);
 
 int device_sm_count();
+
+/* mlp_gradients and mlp_adam as one: a training step. */
+void mlp_train_step(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, float *grad, float *loss,
+		float lr, int step, cudaStream_t st);
 
 } /* namespace kgr */
 

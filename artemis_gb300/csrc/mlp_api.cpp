@@ -148,9 +148,9 @@ kgr_status kgr_mlp_train_step(kgr_mlp *m, const void *x, const float *targets, u
 		KGR_REQUIRE(m && (n == 0 || (x && targets)), KGR_ERR_INVALID_ARGUMENT, "NULL argument");
 		DeviceGuard g(m->device);
 		cudaStream_t st = (cudaStream_t)stream;
-		mlp_gradients(m->params(), x, reinterpret_cast<const float4 *>(targets), n, m->grad.ptr, m->loss.ptr, st);
+		mlp_train_step(m->params(), x, reinterpret_cast<const float4 *>(targets), n, m->grad.ptr, m->loss.ptr, lr,
+			m->step + 1, st);
 		m->step++;
-		mlp_adam(m->params(), m->grad.ptr, lr, m->step, st);
 	});
 }
 

@@ -561,10 +561,18 @@ __device__ __forceinline__ uint32_t positive2(uint32_t a)
 	return r;
 }
 
+/* Eight words to 32 aligned bytes of global memory (zeros if !valid). */
+__device__ __forceinline__ void store32(float *dst, const uint32_t *v, bool valid)
+{
+	asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+		:: "l"(dst), "r"(valid ? v[0] : 0u), "r"(valid ? v[1] : 0u), "r"(valid ? v[2] : 0u), "r"(valid ? v[3] : 0u),
+		"r"(valid ? v[4] : 0u), "r"(valid ? v[5] : 0u), "r"(valid ? v[6] : 0u), "r"(valid ? v[7] : 0u) : "memory");
+}
+
 template <class T>
 __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__restrict__ wt_g,
 		const T *__restrict__ x, const float4 *__restrict__ target, uint32_t n, float *__restrict__ partial,
-		float *__restrict__ loss_sum, const uint32_t *__restrict__ n_dev, uint32_t *__restrict__ err)
+		const uint32_t *__restrict__ n_dev, uint32_t *__restrict__ err)
 {
 	if (n_dev) {
 		uint32_t c = *n_dev;
@@ -796,38 +804,46 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 	if (!ok && tid == 0)
 		atomicOr(err, 1u);
 	/* this block's dW: lanes 32q..32q+15 hold rows 16q..16q+15 of 64 */
+	float *slice = partial + (size_t)blockIdx.x * TC_LAYERS * TC_W * TC_W;
+	float *warp_loss = reinterpret_cast<float *>(sm); /* the weights are done with */
 	if (chain < TT_CHAINS) {
-		float *dst = partial + (size_t)blockIdx.x * TC_LAYERS * TC_W * TC_W + (size_t)(16u * cwarp + (lane & 15u)) * TC_W;
+		float *dst = slice + (size_t)(16u * cwarp + (lane & 15u)) * TC_W;
 		const bool valid = ok && blockIdx.x < tiles;
-		for (int l = chain; l < TC_LAYERS; l += TT_CHAINS) {
+		for (int l = chain; l < TC_LAYERS - 1; l += TT_CHAINS) {
 			uint32_t v[64];
-			const uint32_t col = tmem + ((32u * cwarp) << 16) + TT_DW_COL(l);
-			if (l < TC_LAYERS - 1) {
-				tmem_ld64(col, v);
-			} else {
-				uint32_t w16[16];
-				tmem_ld16(col, w16);
-#pragma unroll
-				for (int j = 0; j < 64; j++)
-					v[j] = j < 16 ? w16[j & 15] : 0u;
-			}
+			tmem_ld64(tmem + ((32u * cwarp) << 16) + TT_DW_COL(l), v);
 			tmem_wait_ld();
 			if (lane < 16) {
-				float *out = dst + (size_t)l * TC_W * TC_W;
 #pragma unroll
-				for (int j = 0; j < 64; j += 4)
-					*reinterpret_cast<uint4 *>(out + j) = valid ? make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3])
-						: make_uint4(0u, 0u, 0u, 0u);
+				for (int j = 0; j < 64; j += 8)
+					store32(dst + (size_t)l * TC_W * TC_W + j, v + j, valid);
+			}
+		}
+		if (chain == TT_CHAINS - 1) {
+			uint32_t v[16];
+			tmem_ld16(tmem + ((32u * cwarp) << 16) + TT_DW_COL(TC_LAYERS - 1), v);
+			tmem_wait_ld();
+			if (lane < 16) {
+#pragma unroll
+				for (int j = 0; j < 16; j += 8)
+					store32(dst + (size_t)(TC_LAYERS - 1) * TC_W * TC_W + j, v + j, valid);
 			}
 		}
 		for (int off = 16; off > 0; off >>= 1)
 			lsum += __shfl_down_sync(0xffffffffu, lsum, off);
 		if (lane == 0)
-			atomicAdd(loss_sum, lsum);
+			warp_loss[warp] = lsum;
 	}
 	tc_before();
 	__syncthreads();
 	tc_after();
+	if (tid == 0) {
+		float sum = 0.0f;
+		for (int w = 0; w < 4 * TT_CHAINS; w++)
+			sum += warp_loss[w];
+		slice[MLP_LOSS_SLOT] = sum;
+	}
+	__syncwarp();
 	if (warp == 0)
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(TT_TMEM_COLS)
 			: "memory");
@@ -869,20 +885,20 @@ void set_train_smem(K kernel)
 
 } /* namespace */
 
-void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, float *loss,
-		cudaStream_t st, const uint32_t *n_dev)
+void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, cudaStream_t st,
+		const uint32_t *n_dev)
 {
 	KGR_REQUIRE(((uintptr_t)x & 15u) == 0, KGR_ERR_INVALID_ARGUMENT, "inputs must be 16-byte aligned");
 	if (mp.dtype == KGR_MLP_BF16) {
 		static bool once = (set_train_smem(mlp_train_tc_kernel<__nv_bfloat16>), true);
 		(void)once;
 		mlp_train_tc_kernel<__nv_bfloat16><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const __nv_bfloat16 *>(mp.wt),
-			static_cast<const __nv_bfloat16 *>(x), target, n, mp.partial, loss, n_dev, mp.tc_err);
+			static_cast<const __nv_bfloat16 *>(x), target, n, mp.partial, n_dev, mp.tc_err);
 	} else {
 		static bool once = (set_train_smem(mlp_train_tc_kernel<__half>), true);
 		(void)once;
 		mlp_train_tc_kernel<__half><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const __half *>(mp.wt),
-			static_cast<const __half *>(x), target, n, mp.partial, loss, n_dev, mp.tc_err);
+			static_cast<const __half *>(x), target, n, mp.partial, n_dev, mp.tc_err);
 	}
 	KGR_CUDA(cudaGetLastError());
 }
