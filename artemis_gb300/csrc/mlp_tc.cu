@@ -471,42 +471,53 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__
  * the next tile's X into b(3) when stage 3 has: the next tile counts its tiles
  * from there.  Both come by asynchronous copies under the other stages.
  *
- * The chains need not meet at any barrier: a thread writes its own row only,
- * and a chain's `ready` mbarrier (one arrival a warp) releases the issuer,
- * whose commit releases the chain (`done`).  The issuer takes the chains in
- * turn, stage by stage, so one chain's epilogue runs under the other's MMAs,
- * and dW, which both add to in tensor memory, is summed in the order of the
- * block's tiles.  TMEM: 64 columns of accumulator a chain, 64 a dW (16 for the
- * last; with M = 64 its rows 16q..16q+15 are lanes 32q..32q+15).  At the end
- * the block writes its dW to its slice of `partial`, which the host sums in
- * block order; the rounding points are those of mlp_train_kernel.
+ * The chains need not meet at any barrier: a thread writes its own row only.  A
+ * chain's `ready` mbarrier (one arrival a warp) releases the warp that issues
+ * its forward and delta MMAs, whose commit releases the chain (`done`).  The dW
+ * have a pair of barriers of their own and a third issuing warp, which takes
+ * the chains in turn, stage by stage, so that a dW, which both chains add to in
+ * tensor memory, is summed in the order of the block's tiles; they run under
+ * the delta's epilogue, which waits for its dW only before it stores.  TMEM: 64
+ * columns of accumulator a chain, 64 a dW (16 for the last; with M = 64 its
+ * rows 16q..16q+15 are lanes 32q..32q+15).  At the end the block writes its dW
+ * to its slice of `partial`, which the host sums in block order; the rounding
+ * points are those of mlp_train_kernel.
  *
  * What bounds it is the latency of a stage (arrive, issue, MMA, commit, read,
  * convert, store), which the second chain hides half of; the tensor cores are
  * busy for about a quarter of the time.  Operands stored a second time,
  * transposed two bytes at a time with bank conflicts, the weights in both
  * layouts, one chain of 128 threads and a barrier on either side of every
- * stage: 114 us for 65,536 rows of FP16, this kernel 34 (a training step 125
- * and 53 us).
+ * stage: 114 us for 65,536 rows of FP16; one issuing warp 34, this kernel 32 (a
+ * training step 125, now 39
+ * us; one tile an SM 27).
  *
  * Every wait is bounded; a warp whose wait runs out leaves, so that every
  * later wait of its chain and of the issuer runs out too, and bit 0 of the
  * error word is set. */
 #define TT_ROWS 128
 #define TT_CHAINS 2
-#define TT_THREADS (128 * TT_CHAINS + 32)
+#define TT_WARPS (5 * TT_CHAINS + 1)            /* four a chain, its issuer, the issuer of dW */
+#define TT_THREADS (32 * TT_WARPS)
 #define TT_TILE_BYTES (TT_ROWS * TC_W * 2u)       /* 16 KB */
 #define TT_BUFS 5u
 #define TT_CHAIN_OFF TC_W_BYTES                   /* 43,008 */
 #define TT_CHAIN_BYTES (TT_BUFS * TT_TILE_BYTES + TT_ROWS * TC_OUT * 2u)
-#define TT_BAR_OFF (TT_CHAIN_OFF + TT_CHAINS * TT_CHAIN_BYTES) /* per chain: ready, done */
-#define TT_SLOT_OFF (TT_BAR_OFF + TT_CHAINS * 16u)
-#define TT_SMEM (TT_SLOT_OFF + 8u)              /* 215,080 bytes */
+#define TT_BAR_OFF (TT_CHAIN_OFF + TT_CHAINS * TT_CHAIN_BYTES) /* per chain: ready, done, the same for dW */
+#define TT_SLOT_OFF (TT_BAR_OFF + TT_CHAINS * 32u)
+#define TT_SMEM (TT_SLOT_OFF + 8u)              /* 215,112 bytes */
 #define TT_TMEM_COLS 512u
 #define TT_WAIT_LIMIT (1u << 18)    /* mbarrier polls before a wait gives up */
 #define TT_DW_COL(l) (64u * TT_CHAINS + 64u * (uint32_t)(l))   /* dW of layer l (layer 5: 16 columns) */
 #define TT_TRANSPOSE_A (1u << 15)                 /* instruction descriptor: MN-major operands */
 #define TT_TRANSPOSE_B (1u << 16)
+
+/* Tile i of a chain whose b(0) is tile `start`. */
+__device__ __forceinline__ uint32_t tile_at(uint32_t start, uint32_t i)
+{
+	i += start;
+	return i >= TT_BUFS ? i - TT_BUFS : i;
+}
 
 /* 16 bytes from global to shared memory without a register; zeros if !valid
  * (src must be readable memory all the same). */
@@ -581,7 +592,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 	extern __shared__ __align__(1024) unsigned char sm[];
 	const int tid = threadIdx.x, warp = tid >> 5;
 	const uint32_t lane = (uint32_t)tid & 31u;
-	const int chain = warp >> 2; /* TT_CHAINS: the issuer */
+	const int chain = warp >> 2; /* TT_CHAINS: the issuers */
 	const uint32_t cwarp = (uint32_t)warp & 3u;
 	const bool bf16 = std::is_same<T, __nv_bfloat16>::value;
 	const uint32_t base = smem_addr(sm), bars = base + TT_BAR_OFF;
@@ -603,10 +614,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 	const uint32_t stride = gridDim.x * TT_CHAINS;
 	if (chain < TT_CHAINS && t < tiles)
 		copy_x(0, t);
-	for (uint32_t g = (uint32_t)warp; g < 42u; g += TT_THREADS / 32) /* 5 x 8 groups of rows, 2 of the last layer */
+	for (uint32_t g = (uint32_t)warp; g < 42u; g += TT_WARPS) /* 5 x 8 groups of rows, 2 of the last layer */
 		copy_rows8(base, wt_g, g, lane, true);
 	if (tid == 0) {
-		for (uint32_t i = 0; i < 2u * TT_CHAINS; i++)
+		for (uint32_t i = 0; i < 4u * TT_CHAINS; i++)
 			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bars + 8u * i), "r"(i & 1u ? 1u : 4u)
 				: "memory");
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -625,97 +636,124 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 	bool ok = true;
 	float lsum = 0.0f;
 
-	if (chain == TT_CHAINS) {
-		/* ---- the issuer ---- */
+	/* a [][64] matrix as it is and transposed, a [][16] one the same; an
+	 * address adds to the address field (16-byte units, all below 2^14) */
+	const uint64_t k64 = smem_desc(0u, TC_LBO, TC_SBO, 0u), m64 = smem_desc(0u, TC_SBO, TC_LBO, 0u);
+	const uint64_t k16 = smem_desc(0u, 128u, 256u, 0u), m16 = smem_desc(0u, 256u, 128u, 0u);
+	const uint32_t id_hidden = instr_desc(bf16, TC_W, TT_ROWS);
+	if (warp == 5 * TT_CHAINS) {
+		/* ---- the issuer of dW: both chains', stage by stage ---- */
 		if (lane == 0) {
-			const uint32_t id_hidden = instr_desc(bf16, TC_W, TT_ROWS), id_out = instr_desc(bf16, TC_OUT, TT_ROWS);
 			const uint32_t id_dw = instr_desc(bf16, TC_W, 64) | TT_TRANSPOSE_A | TT_TRANSPOSE_B;
 			const uint32_t id_dw_out = instr_desc(bf16, TC_OUT, 64) | TT_TRANSPOSE_A | TT_TRANSPOSE_B;
-			const uint32_t id_delta = id_hidden | TT_TRANSPOSE_B;
-			/* a [][64] matrix as it is and transposed, a [][16] one the same; an
-			 * address adds to the address field (16-byte units, all below 2^14) */
-			const uint64_t k64 = smem_desc(0u, TC_LBO, TC_SBO, 0u), m64 = smem_desc(0u, TC_SBO, TC_LBO, 0u);
-			const uint64_t k16 = smem_desc(0u, 128u, 256u, 0u), m16 = smem_desc(0u, 256u, 128u, 0u);
 			uint32_t phase = 0, start = 0;
 			for (uint32_t b = blockIdx.x; ok && b < tiles; b += stride) {
 				const uint32_t chains = b + gridDim.x < tiles ? 2u : 1u;
-				for (int s = 0; ok && s < 2 * TC_LAYERS; s++) {
-					const bool backward = s >= TC_LAYERS;
-					const uint32_t l = backward ? 2u * TC_LAYERS - 1u - (uint32_t)s : (uint32_t)s;
-					const bool last = l == TC_LAYERS - 1;
-					/* the tiles of A(l) (l > 0) and of D(l) (l < 5) */
-					uint32_t ia = start + (l > 0 ? l - 1u : backward ? 4u : 0u), id = start + l;
-					ia -= ia >= TT_BUFS ? TT_BUFS : 0u;
-					id -= id >= TT_BUFS ? TT_BUFS : 0u;
-					const uint32_t w = (base + l * TC_LAYER_BYTES) >> 4;
+				for (int l = TC_LAYERS - 1; ok && l >= 0; l--) {
+					/* the tiles of A(l) and of D(l) (l < 5) */
+					const uint32_t ia = tile_at(start, l > 0 ? (uint32_t)l - 1u : 4u), id = tile_at(start, (uint32_t)l);
 					for (uint32_t c = 0; ok && c < chains; c++) {
-						const uint32_t bar = bars + 16u * c, buf0 = base + TT_CHAIN_OFF + c * TT_CHAIN_BYTES;
-						const uint32_t a = (buf0 + ia * TT_TILE_BYTES) >> 4;
-						const uint32_t d = (buf0 + (last ? TT_BUFS : id) * TT_TILE_BYTES) >> 4;
-						const uint32_t acc = tmem + 64u * c;
-						/* X of the first tile came before the CTA's barrier, of a
-						 * later one with the last D(0) */
-						if (s > 0 && !(ok = bar_wait(bar, phase, TT_WAIT_LIMIT)))
+						const uint32_t bar = bars + 32u * c + 16u, buf0 = base + TT_CHAIN_OFF + c * TT_CHAIN_BYTES;
+						const uint64_t a = m64 + ((buf0 + ia * TT_TILE_BYTES) >> 4);
+						const uint32_t d = (buf0 + (l == TC_LAYERS - 1 ? TT_BUFS : id) * TT_TILE_BYTES) >> 4;
+						const uint32_t sum = b != blockIdx.x || c > 0 ? 1u : 0u, dw = tmem + TT_DW_COL(l);
+						ok = bar_wait(bar, phase, TT_WAIT_LIMIT);
+						if (!ok)
 							break;
 						tc_after();
-						if (!backward) {
-#pragma unroll
-							for (uint32_t kc = 0; kc < 4; kc++)
-								tc_mma(acc, k64 + a + kc * 16u, k64 + w + kc * 16u, last ? id_out : id_hidden,
-									kc > 0 ? 1u : 0u);
-						} else {
-							const uint32_t sum = b != blockIdx.x || c > 0 ? 1u : 0u;
+						if (l == TC_LAYERS - 1) {
 #pragma unroll
 							for (uint32_t kc = 0; kc < 8; kc++)
-								tc_mma(tmem + TT_DW_COL(l), m64 + a + kc * 128u,
-									last ? m16 + d + kc * 32u : m64 + d + kc * 128u, last ? id_dw_out : id_dw,
-									kc > 0 ? 1u : sum);
-							if (last) {
-								tc_mma(acc, k16 + d, m64 + w, id_delta, 0u);
-							} else if (l > 0) {
+								tc_mma(dw, a + kc * 128u, m16 + d + kc * 32u, id_dw_out, kc > 0 ? 1u : sum);
+						} else {
 #pragma unroll
-								for (uint32_t kc = 0; kc < 4; kc++)
-									tc_mma(acc, k64 + d + kc * 16u, m64 + w + kc * 128u, id_delta, kc > 0 ? 1u : 0u);
-							}
+							for (uint32_t kc = 0; kc < 8; kc++)
+								tc_mma(dw, a + kc * 128u, m64 + d + kc * 128u, id_dw, kc > 0 ? 1u : sum);
 						}
-						/* nobody waits for a tile's last stage but the end */
-						if (s < 2 * TC_LAYERS - 1 || b + gridDim.x * c + stride >= tiles)
-							tc_commit(bar + 8u);
+						tc_commit(bar + 8u);
 					}
-					if (s > 0)
-						phase ^= 1u;
+					phase ^= 1u;
 				}
-				start = start >= 2u ? start - 2u : start + 3u;
+				start = tile_at(start, 3u);
+			}
+		}
+		ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+	} else if (chain >= TT_CHAINS) {
+		/* ---- the issuer of a chain's forward and delta ---- */
+		if (lane == 0) {
+			const uint32_t c = (uint32_t)warp - 4u * TT_CHAINS;
+			const uint32_t id_out = instr_desc(bf16, TC_OUT, TT_ROWS), id_delta = id_hidden | TT_TRANSPOSE_B;
+			const uint32_t bar = bars + 32u * c, buf0 = base + TT_CHAIN_OFF + c * TT_CHAIN_BYTES;
+			const uint32_t acc = tmem + 64u * c;
+			uint32_t phase = 1, start = 0;
+			/* X of the first tile came before the CTA's barrier, of a later one
+			 * with the last D(0) */
+			bool first = true;
+			auto next = [&]() -> bool {
+				phase ^= 1u;
+				ok = first || bar_wait(bar, phase, TT_WAIT_LIMIT);
+				if (first)
+					phase ^= 1u;
+				first = false;
+				tc_after();
+				return ok;
+			};
+			for (uint32_t b = blockIdx.x + gridDim.x * c; ok && b < tiles; b += stride) {
+				for (uint32_t l = 0; l < TC_LAYERS && next(); l++) {
+					const uint64_t a = k64 + ((buf0 + tile_at(start, l > 0 ? l - 1u : 0u) * TT_TILE_BYTES) >> 4);
+					const uint64_t w = k64 + ((base + l * TC_LAYER_BYTES) >> 4);
+					const uint32_t id = l == TC_LAYERS - 1 ? id_out : id_hidden;
+#pragma unroll
+					for (uint32_t kc = 0; kc < 4; kc++)
+						tc_mma(acc, a + kc * 16u, w + kc * 16u, id, kc > 0 ? 1u : 0u);
+					tc_commit(bar + 8u);
+				}
+				if (!ok || !next())
+					break;
+				tc_mma(acc, k16 + ((buf0 + TT_BUFS * TT_TILE_BYTES) >> 4),
+					m64 + ((base + (TC_LAYERS - 1) * TC_LAYER_BYTES) >> 4), id_delta, 0u);
+				tc_commit(bar + 8u);
+				for (uint32_t l = TC_LAYERS - 2; l > 0 && next(); l--) {
+					const uint64_t d = k64 + ((buf0 + tile_at(start, l) * TT_TILE_BYTES) >> 4);
+					const uint64_t w = m64 + ((base + l * TC_LAYER_BYTES) >> 4);
+#pragma unroll
+					for (uint32_t kc = 0; kc < 4; kc++)
+						tc_mma(acc, d + kc * 16u, w + kc * 128u, id_delta, kc > 0 ? 1u : 0u);
+					tc_commit(bar + 8u);
+				}
+				start = tile_at(start, 3u);
 			}
 		}
 		ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
 	} else {
 		/* ---- a chain ---- */
-		const uint32_t ready = bars + 16u * (uint32_t)chain, done = ready + 8u;
+		const uint32_t ready = bars + 32u * (uint32_t)chain, done = ready + 8u, dw_ready = ready + 16u, dw_done = ready + 24u;
 		const uint32_t acc = tmem + 64u * (uint32_t)chain + ((32u * cwarp) << 16);
 		const uint32_t row = 32u * cwarp + lane;
 		unsigned char *mine = sm + TT_CHAIN_OFF + (uint32_t)chain * TT_CHAIN_BYTES + (row >> 3) * TC_SBO + (row & 7u) * 16u;
-		uint32_t phase = 0, start = 0;
-		auto at = [&](uint32_t i) -> uint32_t {
-			i += start;
-			return i >= TT_BUFS ? i - TT_BUFS : i;
-		};
-		/* wait for the committed MMAs */
-		auto wait = [&]() -> bool {
-			bool got = bar_wait(done, phase, TT_WAIT_LIMIT);
-			phase ^= 1u;
+		uint32_t phase = 0, dw_phase = 0, start = 0;
+		/* wait for the committed MMAs: the chain's, a dW's */
+		auto wait_for = [&](uint32_t bar, uint32_t &parity) -> bool {
+			bool got = bar_wait(bar, parity, TT_WAIT_LIMIT);
+			parity ^= 1u;
 			got = __all_sync(0xffffffffu, got) != 0;
 			tc_after();
 			return got;
 		};
+		auto wait = [&]() -> bool { return wait_for(done, phase); };
+		auto wait_dw = [&]() -> bool { return wait_for(dw_done, dw_phase); };
 		/* this warp's rows are written and its lanes read */
-		auto publish = [&]() {
+		auto publish = [&](bool dw) {
 			fence_async_smem();
 			tc_before();
 			__syncwarp();
-			if (lane == 0)
+			if (lane == 0) {
 				asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(ready) : "memory");
+				if (dw)
+					asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(dw_ready) : "memory");
+			}
 		};
+		bool dw0 = false; /* the last tile's dW(0) is not waited for */
 		while (ok && t < tiles) {
 			const size_t gr = (size_t)t * TT_ROWS + row;
 			const float4 tg = gr < n ? __ldg(target + gr) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -727,7 +765,10 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 				uint32_t v[64];
 				tmem_ld64(acc, v);
 				tmem_wait_ld();
-				unsigned char *dst = mine + at(l) * TT_TILE_BYTES;
+				unsigned char *dst = mine + tile_at(start, l) * TT_TILE_BYTES;
+				/* dW(0) reads the tiles that A(2) and A(3) will take */
+				if (l == 1 && dw0 && !(ok = wait_dw()))
+					break;
 #pragma unroll
 				for (int kb = 0; kb < 8; kb++) {
 					uint32_t h[4];
@@ -736,7 +777,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 						h[e] = relu2<T>(pack2<T>(__uint_as_float(v[8 * kb + 2 * e]), __uint_as_float(v[8 * kb + 2 * e + 1])));
 					*reinterpret_cast<uint4 *>(dst + kb * TC_LBO) = make_uint4(h[0], h[1], h[2], h[3]);
 				}
-				publish();
+				publish(false);
 			}
 			if (!ok || !(ok = wait()))
 				break;
@@ -762,40 +803,47 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 				*reinterpret_cast<uint4 *>(dst) = make_uint4(pack2<T>(d[0], d[1]), pack2<T>(d[2], 0.0f), 0u, 0u);
 				*reinterpret_cast<uint4 *>(dst + 128u) = make_uint4(0u, 0u, 0u, 0u);
 			}
-			publish();
+			publish(true);
 			/* ---- backward ---- */
 			for (uint32_t l = TC_LAYERS - 1; l > 0; l--) {
 				ok = wait();
 				if (!ok)
 					break;
-				if (l == 4)
-					copy_x(at(4), t);
-				if (l == 3 && t + stride < tiles)
-					copy_x(at(3), t + stride);
-				uint32_t v[64];
+				uint32_t v[64], h[32];
 				tmem_ld64(acc, v);
 				tmem_wait_ld();
-				unsigned char *dst = mine + at(l - 1) * TT_TILE_BYTES;
+				unsigned char *dst = mine + tile_at(start, l - 1) * TT_TILE_BYTES;
 #pragma unroll
 				for (int kb = 0; kb < 8; kb++) {
-					uint4 *p = reinterpret_cast<uint4 *>(dst + kb * TC_LBO);
-					const uint4 a = *p;
+					const uint4 a = *reinterpret_cast<const uint4 *>(dst + kb * TC_LBO);
 					const uint32_t m[4] = {a.x, a.y, a.z, a.w};
-					uint32_t h[4];
 #pragma unroll
 					for (int e = 0; e < 4; e++)
-						h[e] = pack2<T>(__uint_as_float(v[8 * kb + 2 * e]), __uint_as_float(v[8 * kb + 2 * e + 1])) & positive2(m[e]);
-					*p = make_uint4(h[0], h[1], h[2], h[3]);
+						h[4 * kb + e] = pack2<T>(__uint_as_float(v[8 * kb + 2 * e]), __uint_as_float(v[8 * kb + 2 * e + 1]))
+							& positive2(m[e]);
 				}
-				if (l == 1) /* X is back, and the next tile's is there: the issuer goes on without another arrival */
+				/* dW(l) reads A(l), whose place D(l - 1) takes */
+				ok = wait_dw();
+				if (!ok)
+					break;
+#pragma unroll
+				for (int kb = 0; kb < 8; kb++)
+					*reinterpret_cast<uint4 *>(dst + kb * TC_LBO) =
+						make_uint4(h[4 * kb], h[4 * kb + 1], h[4 * kb + 2], h[4 * kb + 3]);
+				if (l == 4)
+					copy_x(tile_at(start, 4u), t);
+				if (l == 3 && t + stride < tiles)
+					copy_x(tile_at(start, 3u), t + stride);
+				if (l == 1) /* X is back, and the next tile's is there: the issuer takes it up with D(0) */
 					copy_wait();
-				publish();
+				publish(true);
 			}
-			if (ok && t + stride >= tiles)
-				ok = wait();
-			start = start >= 2u ? start - 2u : start + 3u;
+			dw0 = true;
+			start = tile_at(start, 3u);
 			t += stride;
 		}
+		if (ok && dw0)
+			ok = wait_dw();
 		copy_wait();
 	}
 	tc_before();
