@@ -506,6 +506,49 @@ __device__ __forceinline__ int gi_neighbor(const FrameParams &fp, int index, f3 
 	return x0 + y0 * width;
 }
 
+/* Pairs (a lane's pixel, one of its neighbours) that a warp has found and not
+ * yet worked on: add() takes at most one more of each lane and, with 32 or more
+ * at hand, gives the latest 32 to work(valid, lane, k, neighbour), one a lane;
+ * finish() gives it the rest.  The whole warp calls both, and work() with all
+ * its lanes, so that it can fetch the pair's pixel from lane `lane` by shuffles. */
+struct WarpPairs {
+	uint2 *list; /* 64 in shared memory, the warp's own */
+	uint32_t count;
+	template <class F>
+	__device__ __forceinline__ void add(bool found, int k, uint32_t neighbour, F work)
+	{
+		const uint32_t lane = threadIdx.x & 31u;
+		const uint32_t mask = __ballot_sync(0xffffffffu, found);
+		if (found)
+			list[count + __popc(mask & ((1u << lane) - 1u))] = make_uint2(lane | (uint32_t)k << 5, neighbour);
+		count += __popc(mask);
+		__syncwarp();
+		if (count >= 32u) {
+			count -= 32u;
+			const uint2 e = list[count + lane];
+			__syncwarp();
+			work(true, (int)(e.x & 31u), (int)(e.x >> 5), e.y);
+		}
+	}
+	template <class F>
+	__device__ __forceinline__ void finish(F work)
+	{
+		const uint32_t lane = threadIdx.x & 31u;
+		if (!count)
+			return;
+		const uint2 e = lane < count ? list[lane] : make_uint2(lane, 0u);
+		work(lane < count, (int)(e.x & 31u), (int)(e.x >> 5), e.y);
+	}
+};
+
+__device__ __forceinline__ f3 from_lane(const f3 &v, int lane)
+{
+	return mk(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane),
+		__shfl_sync(0xffffffffu, v.z, lane));
+}
+
+__device__ __forceinline__ float from_lane(float v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
 /* Spatial reuse as a wavefront of five launches per iteration.  The
  * visibility rays of one resampling step -- one per weighted candidate, one
  * per neighbour domain of the balance-heuristic denominator -- are queued
@@ -522,55 +565,102 @@ __device__ __forceinline__ int gi_neighbor(const FrameParams &fp, int index, f3 
  * weights w_i = p^_q(y_i) |J_i| W_i M_i, and a visibility ray queued for
  * each positive weight.  The pixel's random stream advances as the
  * resampling will draw it: one uniform for the centre, three for each
- * neighbour's offset, one for each neighbour that is resampled. */
+ * neighbour's offset, one for each neighbour that is resampled.
+ *
+ * A lane tests one neighbour after the other; the weights, most of the work,
+ * are made for the neighbours that pass, gathered over the warp so that every
+ * lane has one.  Inside the loop they ran with 12.6 lanes of a warp.  Bound by
+ * issued instructions (0.65 of the cycles): 1920x1080, 8 neighbours, 327 -> 271
+ * us on the terrain, and the rays queued together start nearer each other (the
+ * visibility launches after it 200 -> 171 us). */
 __global__ void __launch_bounds__(128) gi_spatial_gather_kernel(FrameParams fp, GiFrameBuffers gb, int in, int out,
 		int iteration)
 {
-	uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-	if (pix >= fp.npix)
-		return;
-	GiRes C = load_gi(gb.res[in], pix);
-	GBuf g = gbuf(gb.position, gb.normal, pix);
-	if (!g.hit) {
-		store_gi(gb.res[out], pix, C.s, C.W, C.M);
-		return;
+	__shared__ uint2 lists[4][64];
+	const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+	WarpPairs pairs{lists[threadIdx.x >> 5], 0u};
+	bool here = pix < fp.npix;
+	GiRes C{};
+	GBuf g{};
+	if (here) {
+		C = load_gi(gb.res[in], pix);
+		g = gbuf(gb.position, gb.normal, pix);
+		here = g.hit;
+		if (!here)
+			store_gi(gb.res[out], pix, C.s, C.W, C.M);
 	}
-	float depth = length(g.x - v3(fp.center));
-	SurfaceHit h = receiver(fp, gb, pix, g);
-	const BrdfView view = brdf_view(h);
-	f3 seed = pixel_seed(pix, fp.frame, KGR_GI_REUSE_SALT + 1u + (uint32_t)iteration);
-	float wC = gi_target(h, view, C.s) * C.W * C.M;
-	rand_uniform(seed);
+	if (!__any_sync(0xffffffffu, here))
+		return;
+	float depth = 0.0f, wC = 0.0f;
+	SurfaceHit h{};
+	BrdfView view{};
+	f3 seed = mk(0.0f);
+	if (here) {
+		depth = length(g.x - v3(fp.center));
+		h = receiver(fp, gb, pix, g);
+		view = brdf_view(h);
+		seed = pixel_seed(pix, fp.frame, KGR_GI_REUSE_SALT + 1u + (uint32_t)iteration);
+		wC = gi_target(h, view, C.s) * C.W * C.M;
+		rand_uniform(seed);
+	}
+	auto weigh = [&](bool valid, int from, int k, uint32_t index0) {
+		/* the receiver, as far as the target needs it */
+		SurfaceHit q;
+		BrdfView qv;
+		q.x = from_lane(h.x, from);
+		q.n = from_lane(h.n, from);
+		q.wo = from_lane(h.wo, from);
+		q.mat.specular = from_lane(h.mat.specular, from);
+		q.mat.roughness = from_lane(h.mat.roughness, from);
+		qv.n = from_lane(view.n, from);
+		qv.kd = from_lane(view.kd, from);
+		qv.wo_n = from_lane(view.wo_n, from);
+		qv.g1 = from_lane(view.g1, from);
+		const int32_t CM = __shfl_sync(0xffffffffu, C.M, from);
+		float wn = 0.0f;
+		if (valid) {
+			const GiRes N = load_gi(gb.res[in], index0);
+			int32_t cn = fp.gi_confidence_rule && CM < N.M ? CM : N.M;
+			float J = N.s.rc ? gi_jacobian(q.x, f3_of(gb.position[index0]), N.s, fp.gi_jmax) : 0.0f;
+			wn = J > 0.0f ? gi_target(q, qv, N.s) * J * N.W * cn : 0.0f;
+		}
+		const uint32_t slot = (uint32_t)k * fp.npix + (pix - lane + (uint32_t)from);
+		if (valid)
+			gb.weights[slot] = wn;
+		queue_append(gb.vis_queue[0], gi_vis_n(gb, 0), slot, wn > 0.0f, gb.ray_total);
+	};
 	int32_t Msum = C.M;
 	for (int k = 0; k < fp.gi_neighbors; k++) {
-		int index0 = gi_neighbor(fp, (int)pix, seed);
-		uint32_t slot = (uint32_t)k * fp.npix + pix;
-		int2 nb = make_int2(-1, 0);
-		float wn = 0.0f;
-		GBuf gn = gbuf(gb.position, gb.normal, (uint32_t)index0);
-		if (similar(g, depth, gn, length(gn.x - v3(fp.center)))) {
-			GiRes N = load_gi(gb.res[in], (uint32_t)index0);
-			if (N.M > 0) {
-				/* confidence of the neighbour's domain (option
-				 * gi_neighbor_confidence, on by default): at most the
-				 * centre's M.  Any positive confidences keep the balance
-				 * heuristic's weights summing to one; with a neighbour's M
-				 * far above the centre's, a sample the centre can barely
-				 * see would be shaded with the ratio M_n / M_c (up to 255
-				 * where a disocclusion meets reused neighbours) */
-				int32_t cn = fp.gi_confidence_rule && C.M < N.M ? C.M : N.M;
-				nb = make_int2(index0, cn);
-				Msum += cn;
-				float J = N.s.rc ? gi_jacobian(g.x, gn.x, N.s, fp.gi_jmax) : 0.0f;
-				wn = J > 0.0f ? gi_target(h, view, N.s) * J * N.W * cn : 0.0f;
-				rand_uniform(seed);
+		bool found = false;
+		int index0 = 0;
+		if (here) {
+			index0 = gi_neighbor(fp, (int)pix, seed);
+			int2 nb = make_int2(-1, 0);
+			GBuf gn = gbuf(gb.position, gb.normal, (uint32_t)index0);
+			if (similar(g, depth, gn, length(gn.x - v3(fp.center)))) {
+				const int32_t NM = unpack_m(__float_as_uint(gb.res[in].a[index0].w));
+				if (NM > 0) {
+					/* confidence of the neighbour's domain (option
+					 * gi_neighbor_confidence, on by default): at most the
+					 * centre's M.  Any positive confidences keep the balance
+					 * heuristic's weights summing to one; with a neighbour's M
+					 * far above the centre's, a sample the centre can barely
+					 * see would be shaded with the ratio M_n / M_c (up to 255
+					 * where a disocclusion meets reused neighbours) */
+					int32_t cn = fp.gi_confidence_rule && C.M < NM ? C.M : NM;
+					nb = make_int2(index0, cn);
+					Msum += cn;
+					rand_uniform(seed);
+					found = true;
+				}
 			}
+			gb.neighbours[(size_t)((uint32_t)k * fp.npix + pix)] = nb;
 		}
-		gb.neighbours[slot] = nb;
-		gb.weights[slot] = wn;
-		queue_append(gb.vis_queue[0], gi_vis_n(gb, 0), slot, wn > 0.0f, gb.ray_total);
+		pairs.add(found, k, (uint32_t)index0, weigh);
 	}
-	gb.selection[pix] = make_float4(wC, 0.0f, __int_as_float(Msum), 0.0f);
+	pairs.finish(weigh);
+	if (here)
+		gb.selection[pix] = make_float4(wC, 0.0f, __int_as_float(Msum), 0.0f);
 }
 
 /* The receiver of neighbour slot `slot`'s selected sample (second round):
@@ -612,55 +702,74 @@ __global__ void __launch_bounds__(128) gi_visibility_kernel(DeviceScene s, Frame
 /* resample: the weighted reservoir over the centre and the neighbours with
  * their visibility-tested weights (GiMerge's rule, the same draws), then
  * the selected sample shifted back to every neighbour receiver,
- * p^_i(y) |J_q->i|, with a visibility ray queued for each positive one. */
+ * p^_i(y) |J_q->i|, with a visibility ray queued for each positive one.  The
+ * shifts are gathered over the warp like gather's weights (in the loop they
+ * ran with 8.6 lanes): 311 -> 163 us. */
 __global__ void __launch_bounds__(128) gi_spatial_resample_kernel(FrameParams fp, GiFrameBuffers gb, int in,
 		int iteration)
 {
-	uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-	if (pix >= fp.npix)
-		return;
-	GBuf g = gbuf(gb.position, gb.normal, pix);
-	if (!g.hit)
-		return;
-	float4 st = gb.selection[pix];
-	GiMerge r;
-	r.init(pixel_seed(pix, fp.frame, KGR_GI_REUSE_SALT + 1u + (uint32_t)iteration));
-	bool chosen = r.take(st.x);
-	for (int k = 0; k < fp.gi_neighbors; k++) {
-		rand_uniform_3f(r.seed);
-		uint32_t slot = (uint32_t)k * fp.npix + pix;
-		if (gb.neighbours[slot].x < 0)
-			continue;
-		if (r.take(gb.weights[slot])) {
-			r.src = k;
-			chosen = true;
-		}
+	__shared__ uint2 lists[4][64];
+	const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+	WarpPairs pairs{lists[threadIdx.x >> 5], 0u};
+	bool here = pix < fp.npix;
+	GBuf g{};
+	if (here) {
+		g = gbuf(gb.position, gb.normal, pix);
+		here = g.hit;
 	}
-	int32_t domain = chosen ? r.src : -2;
+	if (!__any_sync(0xffffffffu, here))
+		return;
 	GiSample sel;
-	if (chosen) {
-		sel = load_gi(gb.res[in], selected_from(gb, fp.npix, pix, domain)).s;
-	} else {
-		sel.xs = sel.ns = sel.Lo = mk(0.0f);
-		sel.valid = false;
-		sel.rc = true;
-	}
-	SurfaceHit h = receiver(fp, gb, pix, g);
-	float target = gi_target(h, sel);
-	if (target > 0.0f && sel.rc) {
+	sel.xs = sel.ns = sel.Lo = mk(0.0f);
+	sel.valid = false;
+	sel.rc = true;
+	bool shifts = false;
+	if (here) {
+		float4 st = gb.selection[pix];
+		GiMerge r;
+		r.init(pixel_seed(pix, fp.frame, KGR_GI_REUSE_SALT + 1u + (uint32_t)iteration));
+		bool chosen = r.take(st.x);
 		for (int k = 0; k < fp.gi_neighbors; k++) {
+			rand_uniform_3f(r.seed);
 			uint32_t slot = (uint32_t)k * fp.npix + pix;
-			int2 nb = gb.neighbours[slot];
-			if (nb.x < 0)
+			if (gb.neighbours[slot].x < 0)
 				continue;
-			GBuf gn = gbuf(gb.position, gb.normal, (uint32_t)nb.x);
-			float jn = gi_jacobian(gn.x, g.x, sel, fp.gi_jmax);
-			float tn = jn > 0.0f ? gi_target(receiver(fp, gb, (uint32_t)nb.x, gn), sel) * jn : 0.0f;
-			gb.weights[slot] = tn;
-			queue_append(gb.vis_queue[1], gi_vis_n(gb, 1), slot, tn > 0.0f, gb.ray_total);
+			if (r.take(gb.weights[slot])) {
+				r.src = k;
+				chosen = true;
+			}
 		}
+		int32_t domain = chosen ? r.src : -2;
+		if (chosen)
+			sel = load_gi(gb.res[in], selected_from(gb, fp.npix, pix, domain)).s;
+		SurfaceHit h = receiver(fp, gb, pix, g);
+		float target = gi_target(h, sel);
+		shifts = target > 0.0f && sel.rc;
+		gb.selection[pix] = make_float4(r.w, __int_as_float(domain), st.z, target);
 	}
-	gb.selection[pix] = make_float4(r.w, __int_as_float(domain), st.z, target);
+	auto shift = [&](bool valid, int from, int k, uint32_t index0) {
+		GiSample y;
+		y.xs = from_lane(sel.xs, from);
+		y.ns = from_lane(sel.ns, from);
+		y.Lo = from_lane(sel.Lo, from);
+		const f3 x = from_lane(g.x, from);
+		const uint32_t slot = (uint32_t)k * fp.npix + (pix - lane + (uint32_t)from);
+		float tn = 0.0f;
+		if (valid) {
+			GBuf gn = gbuf(gb.position, gb.normal, index0);
+			float jn = gi_jacobian(gn.x, x, y, fp.gi_jmax);
+			tn = jn > 0.0f ? gi_target(receiver(fp, gb, index0, gn), y) * jn : 0.0f;
+			gb.weights[slot] = tn;
+		}
+		queue_append(gb.vis_queue[1], gi_vis_n(gb, 1), slot, tn > 0.0f, gb.ray_total);
+	};
+	if (!__any_sync(0xffffffffu, shifts))
+		return;
+	for (int k = 0; k < fp.gi_neighbors; k++) {
+		const int32_t index0 = shifts ? gb.neighbours[(size_t)((uint32_t)k * fp.npix + pix)].x : -1;
+		pairs.add(index0 >= 0, k, (uint32_t)index0, shift);
+	}
+	pairs.finish(shift);
 }
 
 /* finish: the balance-heuristic weight W = p^<-j(y) w_sum / (p^_q(y) D),

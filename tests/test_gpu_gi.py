@@ -63,3 +63,27 @@ def test_restir_gi_matches_oracle(layout, neighbors):
     assert np.all(rel_ok(rb, state.arrays["res_b"]), axis=1).mean() >= 0.999
     assert color[:, :3].mean() > 0.01
     att.close()
+
+
+@pytest.mark.parametrize("W,H,neighbors", [(31, 7, 1), (33, 5, 3), (64, 2, 16), (97, 41, 8)])
+def test_spatial_reuse_on_partial_warps(W, H, neighbors):
+    """The passing neighbours are gathered over a warp: images whose last warp
+    is partial, one neighbour, the most there are -- reservoirs and colour as
+    the oracle's, with the tolerances of the test above."""
+    g, sc, osc = helpers.both("box4k", 1)
+    bufs = helpers.device_buffers(torch, W * H)
+    att = kgr.Attachment("restir_gi")
+    att.attach(W, H)
+    att.load()
+    att.set_option("gi_neighbors", neighbors)
+    state = pyoracle.GiState(W * H, temporal=True, mcap=30, iterations=3, neighbors=neighbors, radius=30)
+    ocolor = np.zeros((W * H, 4), np.float32)
+    cam = kgr.camera(g.eye, g.target, g.fov, W / H)
+    att.render(helpers.launch(cam, W, H, bufs, frame=0, max_depth=2), sc)
+    pyoracle.render_gi(osc, pyoracle.render_params(W, H, kgr.camera_dict(cam), max_depth=2, frame=0), state, ocolor)
+    torch.cuda.synchronize()
+    color = bufs[0].cpu().numpy()
+    ra = att.debug_copy("gi_reservoir_a", np.zeros((W * H, 4), np.float32))
+    att.close()
+    assert np.all(rel_ok(color, ocolor), axis=1).mean() >= 0.999
+    assert np.all(ra.view(np.uint32) == state.arrays["res_a"].view(np.uint32), axis=1).mean() >= 0.999
