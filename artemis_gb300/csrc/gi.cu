@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(128) gi_spatial_gather_kernel(FrameParams fp, 
 		const uint32_t slot = (uint32_t)k * fp.npix + (pix - lane + (uint32_t)from);
 		if (valid)
 			gb.weights[slot] = wn;
-		queue_append(gb.vis_queue[0], gi_vis_n(gb, 0), slot, wn > 0.0f, gb.ray_total);
+		queue_append(gb.vis_queue[0], gi_vis_n(gb, 0), slot, wn > 0.0f);
 	};
 	int32_t Msum = C.M;
 	for (int k = 0; k < fp.gi_neighbors; k++) {
@@ -671,32 +671,93 @@ __device__ __forceinline__ uint32_t selected_from(const GiFrameBuffers &gb, uint
 	return domain < 0 ? pix : (uint32_t)gb.neighbours[(size_t)domain * npix + pix].x;
 }
 
-/* visibility of queued slots, one ray per thread; a blocked ray's weight
- * becomes 0.  Round 0: from the pixel's receiver to the neighbour's
- * sample.  Round 1: from the neighbour's receiver to the pixel's selected
- * sample.  (These rays are short and two per neighbour: writing them out
- * for the tuned walk cost more than the walk saved.) */
+/* The visibility ray of a queued slot, {from} and to - from.  Round 0: from
+ * the pixel's receiver to the neighbour's sample.  Round 1: from the
+ * neighbour's receiver to the pixel's selected sample. */
+__device__ __forceinline__ void visibility_ends(const FrameParams &fp, const GiFrameBuffers &gb, int in, int round,
+		uint32_t slot, f3 &from, f3 &to)
+{
+	uint32_t pix = slot % fp.npix;
+	uint32_t idx = (uint32_t)gb.neighbours[slot].x;
+	if (round == 0) {
+		from = f3_of(gb.position[pix]);
+		to = f3_of(gb.res[in].a[idx]);
+	} else {
+		int32_t domain = __float_as_int(gb.selection[pix].y);
+		from = f3_of(gb.position[idx]);
+		to = f3_of(gb.res[in].a[selected_from(gb, fp.npix, pix, domain)]);
+	}
+}
+
+/* visibility of queued slots; a blocked ray's weight becomes 0.  The launch
+ * also adds the round's rays to the frame's.  (These rays are short and two per
+ * neighbour: writing them out for the tuned walk cost more than the walk
+ * saved.)  This kernel, one ray per thread, for the layouts that have no walk with
+ * refill. */
 __global__ void __launch_bounds__(128) gi_visibility_kernel(DeviceScene s, FrameParams fp, GiFrameBuffers gb, int in,
 		int round)
 {
 	const uint32_t *queue = gb.vis_queue[round];
 	uint32_t *n = gi_vis_n(gb, round);
+	if (blockIdx.x == 0 && threadIdx.x == 0)
+		atomicAdd(gb.ray_total, *n);
 	for_each_queued(*n, n + (CNT_FETCH_SHADOW - CNT_SHADOW), [&](uint32_t i) {
-		uint32_t slot = queue[i];
-		uint32_t pix = slot % fp.npix;
-		uint32_t idx = (uint32_t)gb.neighbours[slot].x;
+		const uint32_t slot = queue[i];
 		f3 from, to;
-		if (round == 0) {
-			from = f3_of(gb.position[pix]);
-			to = f3_of(gb.res[in].a[idx]);
-		} else {
-			int32_t domain = __float_as_int(gb.selection[pix].y);
-			from = f3_of(gb.position[idx]);
-			to = f3_of(gb.res[in].a[selected_from(gb, fp.npix, pix, domain)]);
-		}
+		visibility_ends(fp, gb, in, round, slot, from, to);
 		if (!visible(s, fp.layout, from, to))
 			gb.weights[slot] = 0.0f;
 	});
+}
+
+/* The same with lanes that take the next ray of their block as they finish one
+ * (persistent_walk), the rays handed out in order by a counter in shared
+ * memory.  Block b owns the runs b, b + grid, ... of GI_VIS_RUN entries.  1920 x
+ * 1080 on the terrain, a launch: 171 us with one ray per thread (10.8 lanes of a
+ * warp), 154 with this; the frame 7.86 -> 7.70 ms, box scene at 960x540 4.67 ->
+ * 4.54, and at most 0.6% either way below that. */
+#define GI_VIS_RUN 64u
+#define GI_VIS_REFILL 24
+template <int LAYOUT>
+__global__ void __launch_bounds__(128) gi_visibility_walk_kernel(DeviceScene s, FrameParams fp, GiFrameBuffers gb,
+		int in, int round)
+{
+	__shared__ uint32_t taken;
+	const uint32_t n = *gi_vis_n(gb, round);
+	if (threadIdx.x == 0) {
+		taken = 0;
+		if (blockIdx.x == 0)
+			atomicAdd(gb.ray_total, n);
+	}
+	__syncthreads();
+	const uint32_t lane = threadIdx.x & 31u;
+	int32_t entries[KGR_STACK_DEPTH];
+	LocalStack stack(nullptr, entries);
+	uint32_t slot = 0;
+	persistent_walk<true, false, LAYOUT>(s, stack, GI_VIS_REFILL, nullptr,
+		[&](bool need, float4 &a, float4 &b) {
+			const uint32_t m = __ballot_sync(0xffffffffu, need);
+			const int leader = __ffs(m) - 1;
+			uint32_t base = 0;
+			if ((int)lane == leader)
+				base = atomicAdd(&taken, (uint32_t)__popc(m));
+			base = __shfl_sync(0xffffffffu, base, leader) + (uint32_t)__popc(m & ((1u << lane) - 1u));
+			const uint64_t at = ((uint64_t)(base / GI_VIS_RUN) * gridDim.x + blockIdx.x) * GI_VIS_RUN + base % GI_VIS_RUN;
+			if (!need || at >= n)
+				return false;
+			slot = gb.vis_queue[round][at];
+			f3 from, to;
+			visibility_ends(fp, gb, in, round, slot, from, to);
+			const f3 D = to - from;
+			const float d = length(D);
+			a = f4_of(from, 0.0f);
+			b = f4_of(D / d, d - KGR_SHADOW_EPS);
+			return true;
+		},
+		[&](const kgr_hit &, bool occ) {
+			if (occ)
+				gb.weights[slot] = 0.0f;
+		});
 }
 
 /* resample: the weighted reservoir over the centre and the neighbours with
@@ -761,7 +822,7 @@ __global__ void __launch_bounds__(128) gi_spatial_resample_kernel(FrameParams fp
 			tn = jn > 0.0f ? gi_target(receiver(fp, gb, index0, gn), y) * jn : 0.0f;
 			gb.weights[slot] = tn;
 		}
-		queue_append(gb.vis_queue[1], gi_vis_n(gb, 1), slot, tn > 0.0f, gb.ray_total);
+		queue_append(gb.vis_queue[1], gi_vis_n(gb, 1), slot, tn > 0.0f);
 	};
 	if (!__any_sync(0xffffffffu, shifts))
 		return;
@@ -938,11 +999,21 @@ void gi_spatial(const DeviceScene &s, const FrameParams &fp, const GiFrameBuffer
 {
 	unsigned grid = (fp.npix + 127) / 128;
 	gi_vis_clear(gb, st);
-	int vis_grid = device_sm_count() * 8;
+	auto visibility = [&](int round) {
+		if (fp.layout == KGR_LAYOUT_THREADED || fp.layout == KGR_LAYOUT_CW8) {
+			gi_visibility_kernel<<<device_sm_count() * 8, 128, 0, st>>>(s, fp, gb, in, round);
+		} else if (fp.layout == KGR_LAYOUT_WIDE) {
+			static const int resident = resident_blocks(gi_visibility_walk_kernel<KGR_LAYOUT_WIDE>, 128);
+			gi_visibility_walk_kernel<KGR_LAYOUT_WIDE><<<resident, 128, 0, st>>>(s, fp, gb, in, round);
+		} else {
+			static const int resident = resident_blocks(gi_visibility_walk_kernel<KGR_LAYOUT_FAST>, 128);
+			gi_visibility_walk_kernel<KGR_LAYOUT_FAST><<<resident, 128, 0, st>>>(s, fp, gb, in, round);
+		}
+	};
 	gi_spatial_gather_kernel<<<grid, 128, 0, st>>>(fp, gb, in, out, iteration);
-	gi_visibility_kernel<<<vis_grid, 128, 0, st>>>(s, fp, gb, in, 0);
+	visibility(0);
 	gi_spatial_resample_kernel<<<grid, 128, 0, st>>>(fp, gb, in, iteration);
-	gi_visibility_kernel<<<vis_grid, 128, 0, st>>>(s, fp, gb, in, 1);
+	visibility(1);
 	gi_spatial_finish_kernel<<<grid, 128, 0, st>>>(fp, gb, in, out);
 	KGR_CUDA(cudaGetLastError());
 }

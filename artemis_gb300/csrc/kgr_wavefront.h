@@ -245,6 +245,16 @@ void restir_spatial(const DeviceScene &s, const FrameParams &fp, const RestirFra
 
 int device_sm_count();
 
+/* How many blocks of a kernel the current device holds at once. */
+template <class K>
+inline int resident_blocks(K kernel, int block)
+{
+	int per_sm = 0;
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess || per_sm < 1)
+		per_sm = 1;
+	return per_sm * device_sm_count();
+}
+
 } /* namespace kgr */
 
 #endif

@@ -434,21 +434,12 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) cw_persiste
 	ANY ? end_shadow(pb) : end_closest(pb);
 }
 
-template <class K>
-int resident_grid(K kernel, int block)
-{
-	int per_sm = 0;
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess || per_sm < 1)
-		per_sm = 1;
-	return per_sm * device_sm_count();
-}
-
 /* One launch of a persistent traversal kernel over a resident grid (the
  * grid of each instantiation is computed once). */
 template <bool ANY, bool COUNT, int LAYOUT, int BLOCK, int OCC = 0, int SHORT = 0>
 void launch_persistent(const DeviceScene &s, const PathBuffers &pb, int q, cudaStream_t st)
 {
-	static const int g = resident_grid(fast_persistent_kernel<ANY, COUNT, LAYOUT, BLOCK, OCC, SHORT>, BLOCK);
+	static const int g = resident_blocks(fast_persistent_kernel<ANY, COUNT, LAYOUT, BLOCK, OCC, SHORT>, BLOCK);
 	fast_persistent_kernel<ANY, COUNT, LAYOUT, BLOCK, OCC, SHORT><<<g, BLOCK, 0, st>>>(s, pb, q);
 }
 
@@ -478,7 +469,7 @@ void launch_persistent_occ(const DeviceScene &s, const PathBuffers &pb, int q, i
 template <bool ANY, bool COUNT, int BLOCK, int OCC = 0>
 void launch_cw_persistent(const DeviceScene &s, const PathBuffers &pb, int q, cudaStream_t st)
 {
-	static const int g = resident_grid(cw_persistent_kernel<ANY, COUNT, BLOCK, OCC>, BLOCK);
+	static const int g = resident_blocks(cw_persistent_kernel<ANY, COUNT, BLOCK, OCC>, BLOCK);
 	cw_persistent_kernel<ANY, COUNT, BLOCK, OCC><<<g, BLOCK, 0, st>>>(s, pb, q);
 }
 
@@ -518,7 +509,7 @@ void launch_persistent_block(const DeviceScene &s, const PathBuffers &pb, int q,
 template <bool COUNT, int LAYOUT, int BLOCK, int OCC = 0, int SHORT = 0>
 void launch_shadow_grid(const DeviceScene &s, const PathBuffers &pb, cudaStream_t st)
 {
-	static const int g = resident_grid(shadow_resolve_kernel<LAYOUT, COUNT, BLOCK, OCC, SHORT>, BLOCK);
+	static const int g = resident_blocks(shadow_resolve_kernel<LAYOUT, COUNT, BLOCK, OCC, SHORT>, BLOCK);
 	shadow_resolve_kernel<LAYOUT, COUNT, BLOCK, OCC, SHORT><<<g, BLOCK, 0, st>>>(s, pb);
 }
 

@@ -138,17 +138,6 @@ int grid_for(uint32_t n, int block)
 	return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
-template <class K>
-int resident_blocks(K kernel, int block)
-{
-	int dev = 0, sms = 152, per_sm = 0;
-	cudaGetDevice(&dev);
-	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, 0) != cudaSuccess || per_sm < 1)
-		per_sm = 1;
-	return per_sm * sms;
-}
-
 template <bool ANY, int LAYOUT>
 void launch_trace_persistent(const DeviceScene &s, const float4 *rays, uint32_t n, kgr_hit *hits, uint32_t *occluded,
 		cudaStream_t st)
