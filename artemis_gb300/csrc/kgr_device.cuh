@@ -975,14 +975,22 @@ struct SurfaceHit {
 
 #define KGR_PI_DEV 3.14159265358979323846f /* brdf.cuh:64 */
 
-/* G1 (brdf.cuh:179-192) */
+/* G1 (brdf.cuh:179-192).  The clamped cosine is in [0, 1], so its arc cosine
+ * is in the quarter circle: the forms of acos, sine and cosine for that range
+ * take no floor, no conversions and one branch.  The loops over light
+ * candidates and neighbours are bound by issued instructions; with these, and
+ * without fract() of draws that are in [0, 1) already, a ReSTIR GI frame of
+ * 1920x1080 went from 7.70 to 7.31 ms and a DI frame of 256x256 from 1.07 to
+ * 1.05. */
 __device__ __forceinline__ float G1(const f3 &n, const f3 &v, const Material &mat)
 {
 	if (dot(v, n) <= 0.0f)
 		return 0.0f;
 	float alpha = mat.roughness;
-	float theta = kacos(clampf(dot(n, v), 0.0f, 0.999f));
-	float tan_theta = ktan(theta);
+	float theta = kacos_unit(clampf(dot(n, v), 0.0f, 0.999f));
+	float sn, c;
+	ksincos_quarter(theta, sn, c);
+	float tan_theta = sn / c;
 	float denom = 1 + ksqrt(1 + alpha * alpha * tan_theta * tan_theta);
 	return 2.0f / denom;
 }
@@ -991,9 +999,9 @@ __device__ __forceinline__ float G1(const f3 &n, const f3 &v, const Material &ma
 __device__ __forceinline__ float ggx_D(const f3 &n, const f3 &h, const Material &mat)
 {
 	float alpha = mat.roughness;
-	float theta = kacos(clampf(dot(n, h), 0.0f, 1.0f));
+	float theta = kacos_unit(clampf(dot(n, h), 0.0f, 1.0f));
 	float sn, c;
-	ksincos(theta, sn, c);
+	ksincos_quarter(theta, sn, c);
 	float tn = sn / c;
 	return (alpha * alpha) / (KGR_PI_DEV * kpow4(c) * kpow2(alpha * alpha + tn * tn));
 }
@@ -1032,7 +1040,7 @@ __device__ __forceinline__ f3 ggx_sample(const Material &mat, f3 n, const f3 &wo
 		float k = ksqrt(eta.y / (1 - eta.y));
 		theta = katan(k * mat.roughness);
 	} else {
-		theta = kacos(ksqrt(eta.y));
+		theta = kacos_unit(ksqrt(eta.y));
 	}
 	float phi = 2.0f * KGR_PI_DEV * eta.z;
 	float st, ct, sp, cp;
@@ -1219,8 +1227,8 @@ __device__ __forceinline__ TriLight load_light(const kgr_triangle_light *lights,
 __device__ __forceinline__ f3 sample_area_light(const TriLight &light, f3 &seed)
 {
 	f3 r = pcg3f(seed);
-	float u = fract(r.x);
-	float v = fract(r.y);
+	float u = r.x; /* in [0, 1): fract() would leave them */
+	float v = r.y;
 	if (u + v > 1.0f) {
 		u = 1.0f - u;
 		v = 1.0f - v;
@@ -1267,8 +1275,8 @@ __device__ __forceinline__ QuadLight load_quad(const kgr_quad_light *quads, uint
 __device__ __forceinline__ f3 sample_area_light(const QuadLight &light, f3 &seed)
 {
 	f3 r = pcg3f(seed);
-	float u = fract(r.x);
-	float v = fract(r.y);
+	float u = r.x; /* in [0, 1): fract() would leave them */
+	float v = r.y;
 	return light.a + u * light.ab + v * light.ac;
 }
 
@@ -1309,10 +1317,12 @@ __device__ __forceinline__ f3 env_miss(const DeviceScene &s, const f3 &d)
 __device__ __forceinline__ f3 env_direction(f3 &seed, bool phi_double)
 {
 	seed = rand_uniform_3f(seed);
-	float theta = kacos(ksqrt(1.0f - fract(seed.x)));
-	float phi = phi_double ? (float)(2.0 * KGR_PI_D * (double)fract(seed.y)) : 2.0f * KGR_PI_F * fract(seed.y);
-	float st = ksin(theta);
-	return mk(st * kcos(phi), st * ksin(phi), kcos(theta));
+	float theta = kacos_unit(ksqrt(1.0f - seed.x)); /* seed in [0, 1) */
+	float phi = phi_double ? (float)(2.0 * KGR_PI_D * (double)seed.y) : 2.0f * KGR_PI_F * seed.y;
+	float st, ct, sp, cp;
+	ksincos_quarter(theta, st, ct);
+	ksincos(phi, sp, cp);
+	return mk(st * cp, st * sp, ct);
 }
 
 /* One light of the launch by its place in [quads | triangles | env]: what

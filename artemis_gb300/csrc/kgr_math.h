@@ -170,12 +170,21 @@ KGR_HD void ksincos(float x, float &s, float &c)
 	int q;
 	float r = reduce_pio2(x, q);
 	float sr = sin_kernel(r), cr = cos_kernel(r);
-	switch (q) {
-	case 0: s = sr; c = cr; break;
-	case 1: s = cr; c = -sr; break;
-	case 2: s = -sr; c = -cr; break;
-	default: s = -cr; c = sr; break;
-	}
+	s = q & 1 ? cr : sr;
+	c = q & 1 ? sr : cr;
+	s = q & 2 ? -s : s;
+	c = (q + 1) & 2 ? -c : c;
+}
+
+/* ksincos of x in [0, PIO2_F], bit for bit, where the quadrant is 0 or 1: no
+ * floor and no conversion.  (0 x PIO2_HI and the like leave x as it is.) */
+KGR_HD void ksincos_quarter(float x, float &s, float &c)
+{
+	const bool one = x * KGR_2_OVER_PI + 0.5f >= 1.0f;
+	const float r = one ? ((x - KGR_PIO2_HI) - KGR_PIO2_MID) - KGR_PIO2_LO : x;
+	const float sr = sin_kernel(r), cr = cos_kernel(r);
+	s = one ? cr : sr;
+	c = one ? -sr : cr;
 }
 
 KGR_HD float ksin(float x) { float s, c; ksincos(x, s, c); return s; }
@@ -195,6 +204,17 @@ KGR_HD float atan_kernel(float y)
 	return y + (y * z) * p;
 }
 
+/* atan of a in [0, 1]; the lanes of a warp part for the division only. */
+KGR_HD float katan_unit(float a)
+{
+	const bool far = a > KGR_TAN_PI12_F;
+	float y = a;
+	if (far)
+		y = (a * KGR_SQRT3_F - 1.0f) / (a + KGR_SQRT3_F);
+	const float r = atan_kernel(y);
+	return far ? KGR_PIO6_F + r : r;
+}
+
 KGR_HD float katan(float x)
 {
 	if (kisnan(x))
@@ -204,11 +224,7 @@ KGR_HD float katan(float x)
 	bool inv = a > 1.0f;
 	if (inv)
 		a = 1.0f / a;
-	float r;
-	if (a > KGR_TAN_PI12_F)
-		r = KGR_PIO6_F + atan_kernel((a * KGR_SQRT3_F - 1.0f) / (a + KGR_SQRT3_F));
-	else
-		r = atan_kernel(a);
+	float r = katan_unit(a);
 	if (inv)
 		r = KGR_PIO2_F - r;
 	return neg ? -r : r;
@@ -221,6 +237,9 @@ KGR_HD float kacos(float x)
 		return (x - x) / (x - x);
 	return 2.0f * katan(ksqrt((1.0f - x) / (1.0f + x)));
 }
+
+/* kacos of x in [0, 1], bit for bit: the root is in [0, 1] too. */
+KGR_HD float kacos_unit(float x) { return 2.0f * katan_unit(ksqrt((1.0f - x) / (1.0f + x))); }
 
 /* atan2(y, x): katan(y / x) moved to the quadrant of (x, y); +-pi/2 on the
  * y axis and 0 at the origin. */
@@ -285,12 +304,9 @@ KGR_HD f3 pcg3f(f3 &seed)
 	return seed;
 }
 
-/* rand_uniform (random.cuh:40-44) */
-KGR_HD float rand_uniform(f3 &seed)
-{
-	seed = pcg3f(seed);
-	return fract(seed.x);
-}
+/* rand_uniform (random.cuh:40-44).  pcg3f leaves every component in [0, 1),
+ * where fract() changes nothing. */
+KGR_HD float rand_uniform(f3 &seed) { return pcg3f(seed).x; }
 
 /* rand_uniform(lim) (random.cuh:46-50) */
 KGR_HD unsigned int rand_uniform(unsigned int lim, f3 &seed)
@@ -301,8 +317,7 @@ KGR_HD unsigned int rand_uniform(unsigned int lim, f3 &seed)
 /* rand_uniform_3f (random.cuh:52-57) */
 KGR_HD f3 rand_uniform_3f(f3 &seed)
 {
-	seed = pcg3f(seed);
-	return fract(seed);
+	return pcg3f(seed);
 }
 
 /* Per-pixel stream: seed bits {pixel ^ stream, pixel, stream}.  `stream` is
