@@ -572,8 +572,10 @@ __device__ __forceinline__ float from_lane(float v, int lane) { return __shfl_sy
  * lane has one.  Inside the loop they ran with 12.6 lanes of a warp.  Bound by
  * issued instructions (0.65 of the cycles): 1920x1080, 8 neighbours, 327 -> 271
  * us on the terrain, and the rays queued together start nearer each other (the
- * visibility launches after it 200 -> 171 us). */
-__global__ void __launch_bounds__(128) gi_spatial_gather_kernel(FrameParams fp, GiFrameBuffers gb, int in, int out,
+ * visibility launches after it 200 -> 171 us).  The gathered work holds two
+ * receivers' registers, so the bounds ask for seven blocks an SM (72 registers,
+ * some spilled, of 93): the frame of three iterations 7.31 -> 7.2 ms. */
+__global__ void __launch_bounds__(128, 7) gi_spatial_gather_kernel(FrameParams fp, GiFrameBuffers gb, int in, int out,
 		int iteration)
 {
 	__shared__ uint2 lists[4][64];
@@ -765,8 +767,9 @@ __global__ void __launch_bounds__(128) gi_visibility_walk_kernel(DeviceScene s, 
  * the selected sample shifted back to every neighbour receiver,
  * p^_i(y) |J_q->i|, with a visibility ray queued for each positive one.  The
  * shifts are gathered over the warp like gather's weights (in the loop they
- * ran with 8.6 lanes): 311 -> 163 us. */
-__global__ void __launch_bounds__(128) gi_spatial_resample_kernel(FrameParams fp, GiFrameBuffers gb, int in,
+ * ran with 8.6 lanes): 311 -> 163 us.  Ten blocks an SM (48 registers of 63): the
+ * frame 7.2 -> 7.13 ms. */
+__global__ void __launch_bounds__(128, 10) gi_spatial_resample_kernel(FrameParams fp, GiFrameBuffers gb, int in,
 		int iteration)
 {
 	__shared__ uint2 lists[4][64];
