@@ -484,13 +484,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__
  * points are those of mlp_train_kernel.
  *
  * What bounds it is the latency of a stage (arrive, issue, MMA, commit, read,
- * convert, store), which the second chain hides half of; the tensor cores are
- * busy for about a quarter of the time.  Operands stored a second time,
- * transposed two bytes at a time with bank conflicts, the weights in both
- * layouts, one chain of 128 threads and a barrier on either side of every
- * stage: 114 us for 65,536 rows of FP16; one issuing warp 34, this kernel 32 (a
- * training step 125, now 39
- * us; one tile an SM 27).
+ * convert, store: 0.7 us), of which the second chain hides half; the tensor
+ * cores are busy for 17% of the time.  So what does not depend on the stage's
+ * MMAs is done before the wait for them (descriptors, masks: 3%).  Operands
+ * stored a second time, transposed two bytes at a time with bank conflicts, the
+ * weights in both layouts, one chain of 128 threads and a barrier on either side
+ * of every stage: 114 us for 65,536 rows of FP16; two chains with one issuing
+ * warp 34, this kernel 31.  A training step: 125 us then, now 38; 27 with one
+ * tile an SM.
  *
  * Every wait is bounded; a warp whose wait runs out leaves, so that every
  * later wait of its chain and of the issuer runs out too, and bit 0 of the
@@ -699,10 +700,12 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 				return ok;
 			};
 			for (uint32_t b = blockIdx.x + gridDim.x * c; ok && b < tiles; b += stride) {
-				for (uint32_t l = 0; l < TC_LAYERS && next(); l++) {
+				for (uint32_t l = 0; l < TC_LAYERS; l++) {
 					const uint64_t a = k64 + ((buf0 + tile_at(start, l > 0 ? l - 1u : 0u) * TT_TILE_BYTES) >> 4);
 					const uint64_t w = k64 + ((base + l * TC_LAYER_BYTES) >> 4);
 					const uint32_t id = l == TC_LAYERS - 1 ? id_out : id_hidden;
+					if (!next())
+						break;
 #pragma unroll
 					for (uint32_t kc = 0; kc < 4; kc++)
 						tc_mma(acc, a + kc * 16u, w + kc * 16u, id, kc > 0 ? 1u : 0u);
@@ -713,9 +716,11 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 				tc_mma(acc, k16 + ((buf0 + TT_BUFS * TT_TILE_BYTES) >> 4),
 					m64 + ((base + (TC_LAYERS - 1) * TC_LAYER_BYTES) >> 4), id_delta, 0u);
 				tc_commit(bar + 8u);
-				for (uint32_t l = TC_LAYERS - 2; l > 0 && next(); l--) {
+				for (uint32_t l = TC_LAYERS - 2; l > 0; l--) {
 					const uint64_t d = k64 + ((buf0 + tile_at(start, l) * TT_TILE_BYTES) >> 4);
 					const uint64_t w = m64 + ((base + l * TC_LAYER_BYTES) >> 4);
+					if (!next())
+						break;
 #pragma unroll
 					for (uint32_t kc = 0; kc < 4; kc++)
 						tc_mma(acc, d + kc * 16u, w + kc * 128u, id_delta, kc > 0 ? 1u : 0u);
@@ -806,22 +811,26 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 			publish(true);
 			/* ---- backward ---- */
 			for (uint32_t l = TC_LAYERS - 1; l > 0; l--) {
-				ok = wait();
-				if (!ok)
-					break;
-				uint32_t v[64], h[32];
-				tmem_ld64(acc, v);
-				tmem_wait_ld();
+				/* the mask is ready before the MMAs are */
 				unsigned char *dst = mine + tile_at(start, l - 1) * TT_TILE_BYTES;
+				uint32_t h[32];
 #pragma unroll
 				for (int kb = 0; kb < 8; kb++) {
 					const uint4 a = *reinterpret_cast<const uint4 *>(dst + kb * TC_LBO);
-					const uint32_t m[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-					for (int e = 0; e < 4; e++)
-						h[4 * kb + e] = pack2<T>(__uint_as_float(v[8 * kb + 2 * e]), __uint_as_float(v[8 * kb + 2 * e + 1]))
-							& positive2(m[e]);
+					h[4 * kb] = positive2(a.x);
+					h[4 * kb + 1] = positive2(a.y);
+					h[4 * kb + 2] = positive2(a.z);
+					h[4 * kb + 3] = positive2(a.w);
 				}
+				ok = wait();
+				if (!ok)
+					break;
+				uint32_t v[64];
+				tmem_ld64(acc, v);
+				tmem_wait_ld();
+#pragma unroll
+				for (int e = 0; e < 32; e++)
+					h[e] &= pack2<T>(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1]));
 				/* dW(l) reads A(l), whose place D(l - 1) takes */
 				ok = wait_dw();
 				if (!ok)
