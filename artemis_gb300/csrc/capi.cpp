@@ -1239,6 +1239,7 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 		 * recursion. */
 		att->ensure_side_stream();
 		cudaStream_t side = att->side;
+		pb.likely_rays = likely_rays(fp.paths, 0);
 		pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
 		m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 		for (int d = 0; d <= last; d++) {
@@ -1253,6 +1254,7 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 			pt_shadow_resolve(s, pb, fp.layout, fp.tune, side);
 			att->mark(STAGE_SHADOW, side, ms);
 			KGR_CUDA(cudaEventRecord(att->ev_shadowed, side));
+			pb.likely_rays = likely_rays(fp.paths, d + 1);
 			if (d < last) {
 				pt_trace_closest(s, pb, q ^ 1, fp.layout, fp.tune, st);
 				m = att->mark(STAGE_TRACE_CLOSEST, st, m);
@@ -1264,6 +1266,7 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 	} else {
 		for (int d = 0; d <= last; d++) {
 			int q = d & 1;
+			pb.likely_rays = likely_rays(fp.paths, d);
 			pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 			m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 			pt_shade(s, pb, fp, d, q, st);
@@ -1300,6 +1303,7 @@ uint32_t trace_bounces(kgr_attachment *att, const DeviceScene &s, PathBuffers pb
 	/* the primary vertex's queue; shade empties the later ones */
 	reset_counters(pb, 1 << CNT_Q0, st);
 	int m = att->mark(-1, st);
+	pb.likely_rays = likely_rays(fp.paths, 1);
 	pt_trace_closest(s, pb, 1, fp.layout, fp.tune, st);
 	m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 	for (int d = 1; d <= fp.max_depth; d++) {
@@ -1320,6 +1324,7 @@ uint32_t trace_bounces(kgr_attachment *att, const DeviceScene &s, PathBuffers pb
 			KGR_CUDA(cudaEventRecord(att->ev_shadowed, shadow));
 		else
 			m = me;
+		pb.likely_rays = likely_rays(fp.paths, d + 1);
 		if (d < fp.max_depth) {
 			pt_trace_closest(s, pb, q ^ 1, fp.layout, fp.tune, st);
 			m = att->mark(STAGE_TRACE_CLOSEST, st, m);
@@ -1383,6 +1388,7 @@ void render_restir_di(kgr_attachment *att, const kgr_launch_info *info, const kg
 	att->mark(-1, st);
 	pt_generate(pb, fp, st);
 	att->mark(STAGE_GENERATE, st);
+	pb.likely_rays = likely_rays(fp.paths, 0);
 	pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
 	att->mark(STAGE_TRACE_CLOSEST, st);
 	restir_primary(s, pb, fp, rb, cur, st);
@@ -1580,6 +1586,7 @@ void render_pt_cached(kgr_attachment *att, const kgr_launch_info *info, const kg
 	int m = att->mark(-1, st);
 	pt_generate(pb, fp, st);
 	m = att->mark(STAGE_GENERATE, st, m);
+	pb.likely_rays = likely_rays(fp.paths, 0);
 	pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
 	m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 	pt_shade(s, pb, fp, 0, 0, st);
@@ -1596,6 +1603,7 @@ void render_pt_cached(kgr_attachment *att, const kgr_launch_info *info, const kg
 		pt_shadow_resolve(s, pb, fp.layout, fp.tune, st);
 		m = att->mark(STAGE_SHADOW, st, m);
 	}
+	pb.likely_rays = likely_rays(fp.paths, 1);
 	pt_trace_closest(s, pb, 1, fp.layout, fp.tune, st);
 	m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 	cache_query(s, pb, 1, cp, att->q_feat.ptr, att->q_le.ptr, st);
@@ -1692,6 +1700,7 @@ void render_restir_gi(kgr_attachment *att, const kgr_launch_info *info, const kg
 	att->mark(-1, st);
 	pt_generate(pb, fp, st);
 	att->mark(STAGE_GENERATE, st);
+	pb.likely_rays = likely_rays(fp.paths, 0);
 	pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
 	att->mark(STAGE_TRACE_CLOSEST, st);
 	gi_primary(s, pb, fp, gb, st);

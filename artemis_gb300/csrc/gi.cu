@@ -962,6 +962,7 @@ void gi_walk(const DeviceScene &s, const FrameParams &fp, const GiFrameBuffers &
 	vb.shadow_flags = gb.vis_flag;
 	vb.visits = nullptr;
 	vb.capacity = gb.vis_capacity;
+	vb.likely_rays = fp.npix;
 	pt_shadow_resolve(s, vb, fp.layout, fp.tune, st);
 }
 

@@ -62,7 +62,14 @@ struct PathBuffers {
 	/* the walks go to the cooperative walk (eight lanes a ray) up to this
 	 * many rays for each of the groups the launch holds */
 	uint32_t coop_rounds = KGR_COOP_ROUNDS;
+	/* how many rays the next walk is likely to have, as far as the host knows
+	 * (0: it does not); only the launch's register bound follows it */
+	uint32_t likely_rays = 0;
 };
+
+/* The rays of bounce `depth`: on a scene open to the sky about half a bounce's
+ * rays miss. */
+inline uint32_t likely_rays(uint32_t paths, int depth) { return depth < 32 ? paths >> depth : 0; }
 
 /* The float4 arrays of the path state, in the order their allocators lay
  * them out. */

@@ -240,9 +240,21 @@ __global__ void __launch_bounds__(SHADE_BLOCK) shade_kernel(DeviceScene s, PathB
 /* is_occluded for every queued shadow ray, then Ld = contr / pdf and
  * L += beta * (Le + Ld) in the order of the recursion.  One ray per thread,
  * grid-stride over the queue. */
-/* Minimum resident blocks per SM a launch shape asks the compiler for:
- * OCC = 1 caps registers so that 1536 threads (48 warps) fit an SM. */
-#define KGR_MIN_BLOCKS(BLOCK, OCC) ((OCC) ? 1536 / (BLOCK) : 1)
+/* Minimum resident blocks per SM a launch shape asks the compiler for: OCC = 1
+ * caps registers so that 1536 threads (48 warps) fit an SM.  OCC = 2, 1280
+ * threads (48 registers, a few spilled, of 62), is what walks that are likely
+ * to be long take instead of OCC = 0 (KGR_MANY_RAYS, fast layout, no shared
+ * stack): they are bound by latency that more warps hide, where a short walk
+ * waits for single rays and the spills lie on that path.  The terrain at 1080p,
+ * 4 samples: 10.54 ms a frame with OCC = 0 throughout, 10.27 (1152 threads),
+ * 10.09 (1280), 10.25 (1408), 10.16 (1536); 256x256 on the box scene 752 us and
+ * with 1280 threads 843. */
+#define KGR_MIN_BLOCKS(BLOCK, OCC) ((OCC) == 1 ? 1536 / (BLOCK) : (OCC) == 2 ? 1280 / (BLOCK) : 1)
+/* The walk of a bounce that is likely to have this many rays takes OCC = 2.
+ * 1080p frames, never / 100,000 / 250,000 / 1,000,000: path tracing 4 samples
+ * 10.54, 10.12, 10.12, 10.11 ms, 1 sample 3.36, 3.30, 3.27, 3.30; cached 1.650,
+ * 1.584, 1.584, 1.587; frames of 116,000 paths are 1 to 2% slower with it. */
+#define KGR_MANY_RAYS 250000u
 
 /* The traversal stack of a kernel instantiation: SHORT entries a thread in
  * shared memory (the rest in local memory), or all in local memory. */
@@ -466,6 +478,17 @@ void launch_persistent_occ(const DeviceScene &s, const PathBuffers &pb, int q, i
 		launch_persistent_stack<ANY, LAYOUT, OCC, 128>(s, pb, q, stack, st);
 }
 
+template <bool ANY>
+void launch_persistent_many(const DeviceScene &s, const PathBuffers &pb, int q, int block, cudaStream_t st)
+{
+	if (block == 64)
+		launch_persistent<ANY, false, KGR_LAYOUT_FAST, 64, 2>(s, pb, q, st);
+	else if (block == 256)
+		launch_persistent<ANY, false, KGR_LAYOUT_FAST, 256, 2>(s, pb, q, st);
+	else
+		launch_persistent<ANY, false, KGR_LAYOUT_FAST, 128, 2>(s, pb, q, st);
+}
+
 template <bool ANY, bool COUNT, int BLOCK, int OCC = 0>
 void launch_cw_persistent(const DeviceScene &s, const PathBuffers &pb, int q, cudaStream_t st)
 {
@@ -502,6 +525,8 @@ void launch_persistent_block(const DeviceScene &s, const PathBuffers &pb, int q,
 {
 	if (t.occupancy)
 		launch_persistent_occ<ANY, LAYOUT, 1>(s, pb, q, t.block, t.stack, st);
+	else if (LAYOUT == KGR_LAYOUT_FAST && t.stack == 0 && pb.likely_rays >= KGR_MANY_RAYS)
+		launch_persistent_many<ANY>(s, pb, q, t.block, st);
 	else
 		launch_persistent_occ<ANY, LAYOUT, 0>(s, pb, q, t.block, t.stack, st);
 }

@@ -674,6 +674,7 @@ void vis_walk(const DeviceScene &s, const FrameParams &fp, const RestirFrameBuff
 	vb.shadow_flags = rb.vis_flag;
 	vb.visits = nullptr;
 	vb.capacity = rb.vis_capacity;
+	vb.likely_rays = fp.npix;
 	pt_shadow_resolve(s, vb, fp.layout, fp.tune, st);
 }
 

@@ -88,3 +88,28 @@ def test_restir_bounces_overlapped_or_not(plugin, side):
         att.close()
     assert images[0][:, :3].mean() > 0.0
     assert np.array_equal(images[0].view(np.uint32), images[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("block", [64, 128, 256])
+@pytest.mark.parametrize("side", [499, 500, 512])
+def test_frames_on_both_sides_of_the_register_bound(block, side):
+    """Path counts around the one above which a walk takes more warps an SM:
+    the same bits as with the register cap and on the threaded layout."""
+    torch = pytest.importorskip("torch")
+    g, sc, _ = helpers.both("box64", 5)
+    cam = kgr.camera(g.eye, g.target, g.fov, 1.0)
+    images = []
+    for layout, occupancy in (("fast", 0), ("fast", 1), ("threaded", 0)):
+        bufs = helpers.device_buffers(torch, side * side)
+        att = kgr.Attachment("path_tracer")
+        att.attach(side, side)
+        att.load()
+        att.set_option("layout", layout)
+        att.set_option("trace_block", block)
+        att.set_option("trace_occupancy", occupancy)
+        att.render(helpers.launch(cam, side, side, bufs, frame=0, max_depth=3), sc)
+        torch.cuda.synchronize()
+        images.append(bufs[0].cpu().numpy().view(np.uint32))
+        att.close()
+    assert np.array_equal(images[0], images[1])
+    assert np.array_equal(images[0], images[2])
