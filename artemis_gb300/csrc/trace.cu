@@ -11,10 +11,29 @@ namespace kgr {
 
 namespace {
 
-template <bool ANY, int LAYOUT>
-__global__ void __launch_bounds__(128) trace_rays_kernel(DeviceScene s, const float4 *__restrict__ rays,
+#define TRACE_BLOCK 128
+#define TRACE_COHERENT 0.9f
+
+/* Whether the rays are coherent: whether the 32 consecutive ones at each of
+ * four places of the buffer head the same way (within 18 degrees of the first
+ * of them).  Every thread of a block of TRACE_BLOCK takes part; n >= 256. */
+__device__ __forceinline__ bool rays_agree(const float4 *__restrict__ rays, uint32_t n)
+{
+	const uint32_t at = (2u * (threadIdx.x >> 5) + 1u) * (n / 8u) + (threadIdx.x & 31u);
+	const float4 d = __ldg(&rays[2 * (size_t)at + 1]);
+	const float x = __shfl_sync(0xffffffffu, d.x, 0), y = __shfl_sync(0xffffffffu, d.y, 0), z = __shfl_sync(0xffffffffu, d.z, 0);
+	const float c = d.x * x + d.y * y + d.z * z;
+	return __syncthreads_and(c > 0.0f &&
+		c * c >= TRACE_COHERENT * (d.x * d.x + d.y * d.y + d.z * d.z) * (x * x + y * y + z * z)) != 0;
+}
+
+/* COHERENT: does nothing for other rays. */
+template <bool ANY, int LAYOUT, bool COHERENT = false>
+__global__ void __launch_bounds__(TRACE_BLOCK) trace_rays_kernel(DeviceScene s, const float4 *__restrict__ rays,
 		uint32_t n, kgr_hit *__restrict__ hits, uint32_t *__restrict__ occluded)
 {
+	if (COHERENT && !rays_agree(rays, n))
+		return;
 	uint32_t stride = gridDim.x * blockDim.x;
 	for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
 		float4 a = __ldg(&rays[2 * (size_t)i]);
@@ -34,10 +53,10 @@ __global__ void __launch_bounds__(128) trace_rays_kernel(DeviceScene s, const fl
 	}
 }
 
-#define TRACE_BLOCK 128
 #define TRACE_CHUNK 64u
-/* between a bounce's best (31) and a camera ray's (8 to 20) */
+/* between a bounce's best (31) and a mixed buffer's (8 to 20) */
 #define TRACE_REFILL 24
+#define TRACE_MANY_COHERENT 1000000u
 
 /* The k-th ray of this block: it owns the chunks blockIdx, blockIdx + grid,
  * blockIdx + 2 grid, ... of `chunk` consecutive rays.  Grows with k. */
@@ -55,20 +74,33 @@ __device__ __forceinline__ uint64_t block_ray(uint32_t k, uint32_t chunk)
  * Against one ray per thread over a grid-stride loop, 2,073,600 rays on the
  * box scene, the 0.26M- and the 1.16M-triangle terrain: bounce rays 1089, 857,
  * 1084 -> 899, 718, 883 us, shadow rays 786, 539, 707 -> 562, 436, 554, camera
- * rays 514, 374, 562 -> 572, 357, 483. */
-template <bool ANY, int LAYOUT>
+ * rays 512, 372, 562 -> 490, 343, 476.
+ *
+ * Camera rays end together, so refilling only mixes warps that belong together,
+ * and what they lose is balance: a block keeps its share to the end, where the
+ * hardware would have put a new block on an SM that is done.  The kernel comes
+ * in two launches, of which the one that does not suit the rays (COHERENT,
+ * rays_agree) returns at once (about 2 us): coherent rays take new rays a whole
+ * warp at a time, in four times the blocks the GPU holds, or below
+ * TRACE_MANY_COHERENT the kernel above.  Box scene, 400,000, 600,000 and 2.07M
+ * camera rays: 158, 217, 616 us without the distinction, 143, 198, 490 with it,
+ * and 139, 195, 512 with one ray per thread throughout; the larger terrain's
+ * 162, 205, 482 without, 176, 204, 476 with it.  Bounce rays pay the empty
+ * launch: 600,000 on the box scene 303 and 306. */
+template <bool ANY, int LAYOUT, bool COHERENT>
 __global__ void __launch_bounds__(TRACE_BLOCK) trace_persistent_kernel(DeviceScene s, const float4 *__restrict__ rays,
 		uint32_t n, kgr_hit *__restrict__ hits, uint32_t *__restrict__ occluded)
 {
 	__shared__ uint32_t taken;
 	if (threadIdx.x == 0)
 		taken = 0;
-	__syncthreads();
+	if (rays_agree(rays, n) != COHERENT) /* a barrier too */
+		return;
 	const int lane = threadIdx.x & 31;
 	int32_t entries[KGR_STACK_DEPTH];
 	LocalStack stack(nullptr, entries);
 	uint32_t i = 0;
-	persistent_walk<ANY, false, LAYOUT>(s, stack, TRACE_REFILL, nullptr,
+	persistent_walk<ANY, false, LAYOUT>(s, stack, COHERENT ? 0 : TRACE_REFILL, nullptr,
 		[&](bool need, float4 &a, float4 &b) {
 			unsigned m = __ballot_sync(0xffffffffu, need);
 			int leader = __ffs(m) - 1;
@@ -142,7 +174,7 @@ template <bool ANY, int LAYOUT>
 void launch_trace_persistent(const DeviceScene &s, const float4 *rays, uint32_t n, kgr_hit *hits, uint32_t *occluded,
 		cudaStream_t st)
 {
-	static const int resident = resident_blocks(trace_persistent_kernel<ANY, LAYOUT>, TRACE_BLOCK);
+	static const int resident = resident_blocks(trace_persistent_kernel<ANY, LAYOUT, false>, TRACE_BLOCK);
 	if (LAYOUT == KGR_LAYOUT_FAST && s.coop_nodes) {
 		/* up to KGR_COOP_ROUNDS rays for each of the resident groups */
 		static const int coop = resident_blocks(trace_coop_kernel<ANY>, TRACE_BLOCK);
@@ -161,7 +193,12 @@ void launch_trace_persistent(const DeviceScene &s, const float4 *rays, uint32_t 
 		trace_rays_kernel<ANY, LAYOUT><<<grid_for(n, TRACE_BLOCK), TRACE_BLOCK, 0, st>>>(s, rays, n, hits, occluded);
 		return;
 	}
-	trace_persistent_kernel<ANY, LAYOUT><<<resident, TRACE_BLOCK, 0, st>>>(s, rays, n, hits, occluded);
+	trace_persistent_kernel<ANY, LAYOUT, false><<<resident, TRACE_BLOCK, 0, st>>>(s, rays, n, hits, occluded);
+	if (n >= TRACE_MANY_COHERENT)
+		trace_persistent_kernel<ANY, LAYOUT, true><<<4 * resident, TRACE_BLOCK, 0, st>>>(s, rays, n, hits, occluded);
+	else
+		trace_rays_kernel<ANY, LAYOUT, true><<<grid_for(n, TRACE_BLOCK), TRACE_BLOCK, 0, st>>>(s, rays, n, hits,
+			occluded);
 }
 
 template <bool ANY>

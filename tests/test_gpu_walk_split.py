@@ -113,3 +113,18 @@ def test_frames_on_both_sides_of_the_register_bound(block, side):
         att.close()
     assert np.array_equal(images[0], images[1])
     assert np.array_equal(images[0], images[2])
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("layout", [kgr.LAYOUT_FAST, kgr.LAYOUT_WIDE])
+@pytest.mark.parametrize("side", [700, 1001])
+def test_coherent_ray_buffers(layout, side, mixed):
+    """Camera rays, on both sides of the count where their launch changes, and
+    the same with every 97th ray turned round: the threaded walk's hits."""
+    g, sc, _ = helpers.both("box64", 5)
+    rays = helpers.camera_rays(kgr.camera(g.eye, g.target, g.fov, 1.0), side, side)
+    if mixed:
+        rays[::97, 4:7] *= -1.0
+    ref = sc.trace_closest_host(rays, kgr.LAYOUT_THREADED)
+    assert np.array_equal(sc.trace_closest_host(rays, layout).view(np.uint32), ref.view(np.uint32))
+    assert np.array_equal(sc.trace_any_host(rays, layout), sc.trace_any_host(rays, kgr.LAYOUT_THREADED))
