@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(128, 10) atrous_kernel(const float4 *__restric
 {
 	AtrousPixel p;
 	p.x = (int)(blockIdx.x * 32 + threadIdx.x);
-	p.y = (int)(blockIdx.y * 4 + threadIdx.y);
+	p.y = (int)((blockIdx.z * gridDim.y + blockIdx.y) * 4 + threadIdx.y);
 	if (p.x >= (int)ps.width || p.y >= (int)ps.height)
 		return;
 	const size_t ip = (size_t)p.y * ps.width + p.x;
@@ -320,7 +320,10 @@ void denoise(const float4 *color, const float4 *normal, const float4 *albedo, co
 		ps.step = 1 << i;
 		ps.half_sigma = p.sigma_color * (1.0f / (float)(1 << i)) * 0.5f;
 		ps.remodulate = use_albedo && i == p.iterations - 1;
-		dim3 grid((width + 31) / 32, (height + 3) / 4);
+		/* four rows a block: an image of more than 262,140 rows takes
+		 * several layers of the grid (65,535 is the most in y) */
+		const uint32_t rows = (height + 3) / 4, layer = 65535u;
+		dim3 grid((width + 31) / 32, rows < layer ? rows : layer, (rows + layer - 1) / layer);
 		float4 *dst = target(i);
 		const bool use_position = (guides & KGR_DENOISE_POSITION) != 0;
 		if (power == POWER_64)

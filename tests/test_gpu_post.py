@@ -120,3 +120,21 @@ def test_infinite_and_nan_pixels_stay_where_they_are():
     assert np.isfinite(got[:, :16]).all()
     assert np.isnan(got[4, 20, 0]) and not np.isfinite(got[2, 25, 1])
     dn.close()
+
+
+@pytest.mark.parametrize("w,h", [(2, 262140), (2, 262141), (1, 600001), (3000001, 1)])
+def test_narrow_images_of_many_rows_or_columns(w, h):
+    """More rows than a grid's second dimension holds blocks of, and one row
+    of many columns: every extent that the creation accepts is filtered."""
+    rng = np.random.default_rng(h)
+    color = rng.uniform(0.1, 2.0, (h, w, 4)).astype(np.float32)
+    normal = np.zeros((h, w, 4), np.float32)
+    normal[..., 2] = 1.0
+    bufs = [torch.from_numpy(b).cuda() for b in (color, normal)]
+    dn = kgr.Denoiser(w, h, kgr.DENOISE_NORMAL)
+    dn.denoise(bufs[0].data_ptr(), bufs[1].data_ptr(), iterations=2)
+    torch.cuda.synchronize()
+    got = result_array(dn, w, h).reshape(h, w, 4)
+    ref = post_ref.denoise(color, normal, None, None, kgr.DENOISE_NORMAL, iterations=2)
+    np.testing.assert_allclose(got, ref, rtol=1e-4, atol=1e-6)
+    dn.close()
