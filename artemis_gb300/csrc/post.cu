@@ -106,28 +106,19 @@ __device__ __forceinline__ float3 albedo_div(float4 a)
 	return make_float3(a.x > 1e-3f ? a.x : 1.0f, a.y > 1e-3f ? a.y : 1.0f, a.z > 1e-3f ? a.z : 1.0f);
 }
 
-/* c ^ (2 ^ n) to within an ulp: each squaring keeps its rounding error, and the
- * last rounds once (into the denormal numbers too) */
+/* c ^ (2 ^ n) to within an ulp, c >= 0: each squaring keeps its rounding error,
+ * and the last rounds once (into the denormal numbers too).  Above the largest
+ * float the errors are not numbers: infinity then. */
 __device__ __forceinline__ float squared(float c, int n)
 {
 	float lo = 0.0f;
+#pragma unroll
 	for (int q = 1; q < n; q++) {
 		float sq = c * c;
 		lo = __fmaf_rn(c + c, lo, __fmaf_rn(c, c, -sq));
 		c = sq;
 	}
-	return n ? __fmaf_rn(c, c, (c + c) * lo) : c;
-}
-
-/* c ^ 64, 32 ulp */
-__device__ __forceinline__ float pow64(float c)
-{
-	c *= c;
-	c *= c;
-	c *= c;
-	c *= c;
-	c *= c;
-	return c * c;
+	return n ? fminf(__fmaf_rn(c, c, (c + c) * lo), INFINITY) : c;
 }
 
 /* 3/8, 1/4, 1/16 at 0, 1, 2 */
@@ -149,7 +140,8 @@ __global__ void demodulate_kernel(const float4 *in, const float4 *__restrict__ a
 }
 
 /* How a pass raises the normal cosine to its power: the default 64 and other
- * powers of two by squaring, anything else by powf. */
+ * powers of two by squaring (the default's chain unrolled), anything else by
+ * powf. */
 enum { POWER_NONE = 0, POWER_SQUARES = 1, POWER_ANY = 2, POWER_64 = 3 };
 
 struct AtrousPass {
@@ -198,8 +190,7 @@ __device__ __forceinline__ void atrous_taps(AtrousPixel &p, const float4 *__rest
 			if (p.hit) {
 				if (POWER != POWER_NONE) {
 					float c = fmaxf(p.n.x * nq.x + p.n.y * nq.y + p.n.z * nq.z, 0.0f);
-					w *= POWER == POWER_ANY ? powf(c, ps.normal_power)
-						: POWER == POWER_64 ? pow64(c) : squared(c, ps.squarings);
+					w *= POWER == POWER_ANY ? powf(c, ps.normal_power) : squared(c, POWER == POWER_64 ? 6 : ps.squarings);
 				}
 				if (POSITION && (dx != 0 || dy != 0)) {
 					float3 v = make_float3(xq.x - p.pos.x, xq.y - p.pos.y, xq.z - p.pos.z);
@@ -223,11 +214,15 @@ __device__ __forceinline__ void atrous_taps(AtrousPixel &p, const float4 *__rest
  *
  * Bound by the arithmetic of a tap (issue slots 62% busy, L1 24%, DRAM 8%).  The
  * divisions are products with a reciprocal or a reciprocal square root (MUFU,
- * 1 ulp); a power-of-two exponent is that many squarings; the sums are fused.
+ * 1 ulp); a power-of-two exponent is that many squarings, good to an ulp also
+ * where the normals are means of several samples' and the weights denormal
+ * numbers (plain squarings for the others and a second loop for these: 781 us
+ * behind a frame of one sample a pixel, but 1430 to 1560 behind several, 2330
+ * on the box scene); the sums are fused.
  * The three weights are multiplied in this order because the power may leave
  * only a few bits of a denormal number.  1080p, five passes, all guides: 1787
- * -> 781 us (the first pass no longer divides every tap by its albedo:
- * demodulate_kernel), error against 64 bits 6.0e-7 as before.  Two pixels of a
+ * -> 831 us, and 1722 -> 833 behind four samples a pixel (the first pass no
+ * longer divides every tap by its albedo: demodulate_kernel).  Two pixels of a
  * column a thread, which halves the loads, were no faster; all 25 taps unrolled
  * 840 to 930 us, waiting for instructions; a branch past the loads of a tap of
  * the other kind 900 us; no cap on the registers 812 us. */
@@ -249,12 +244,7 @@ __global__ void __launch_bounds__(128, 10) atrous_kernel(const float4 *__restric
 	p.l = lum(f3of(c));
 	p.sum = make_float3(0.0f, 0.0f, 0.0f);
 	p.wsum = 0.0f;
-	/* a mean of different normals is short: its weights are small, some of
-	 * them denormal numbers, and the result hangs on their roundings */
-	if (POWER == POWER_64 && p.hit && dot3(p.n, p.n) < 0.99f)
-		atrous_taps<POWER_SQUARES, POSITION>(p, in, normal, position, ps);
-	else
-		atrous_taps<POWER, POSITION>(p, in, normal, position, ps);
+	atrous_taps<POWER, POSITION>(p, in, normal, position, ps);
 	float3 r = p.wsum > 0.0f ? make_float3(p.sum.x / p.wsum, p.sum.y / p.wsum, p.sum.z / p.wsum) : f3of(c);
 	if (ps.remodulate) {
 		float3 d = albedo_div(albedo[ip]);

@@ -138,3 +138,54 @@ def test_narrow_images_of_many_rows_or_columns(w, h):
     ref = post_ref.denoise(color, normal, None, None, kgr.DENOISE_NORMAL, iterations=2)
     np.testing.assert_allclose(got, ref, rtol=1e-4, atol=1e-6)
     dn.close()
+
+
+def pairs(n, tap_normals, tap_colors, tap_positions=None):
+    """n pairs of pixels that only meet each other: three rows apart, sky
+    between them.  The left pixel of a pair is black, at the origin, its
+    normal (0, 0, 1).  (color, normal, position), float32 (3 n, 2, 4)."""
+    bufs = [np.zeros((3 * n, 2, 4), np.float32) for _ in range(3)]
+    bufs[0][::3, 1, :3] = np.asarray(tap_colors, np.float32)[:, None]
+    bufs[1][::3, 0, 2] = 1.0
+    bufs[1][::3, 1, :3] = tap_normals
+    if tap_positions is not None:
+        bufs[2][::3, 1, :3] = tap_positions
+    return bufs
+
+
+def tap_weight(bufs, guides, **params):
+    """The weight of a pair's right pixel in the left one's mean, from the
+    filter's result in double precision: r = w c / (9/64 + w)."""
+    dev = [torch.from_numpy(b).cuda() for b in bufs]
+    h = len(bufs[0])
+    dn = kgr.Denoiser(2, h, guides)
+    dn.denoise(dev[0].data_ptr(), dev[1].data_ptr(), None, dev[2].data_ptr(), iterations=1, **params)
+    torch.cuda.synchronize()
+    r = result_array(dn, 2, h).reshape(h, 2, 4)[::3, 0, 0].astype(np.float64)
+    dn.close()
+    c = bufs[0][::3, 1, 0].astype(np.float64)
+    return r * (9.0 / 64.0) / (c - r)
+
+
+@pytest.mark.parametrize("power", [64.0, 32.0, 2.0])
+def test_normal_weight_is_good_to_a_few_ulp(power):
+    """The cosine is the tap normal's z itself.  Roundings: the power 1 ulp,
+    its product with the spline, the sum's product, the sum of weights and
+    the mean half an ulp each: 3 ulp, of 2^-23 relative at most.  Cosines
+    whose power is below 2^-18, so that w + 9/64 does not feel w's error."""
+    rng = np.random.default_rng(int(power))
+    z = (rng.uniform(2.0 ** -60, 2.0 ** -18, 4096) ** (1.0 / power)).astype(np.float32)
+    normals = np.stack([np.sqrt(1.0 - z.astype(np.float64) ** 2), np.zeros(len(z)), z], 1).astype(np.float32)
+    bufs = pairs(len(z), normals, np.ones(len(z)))
+    got = tap_weight(bufs, kgr.DENOISE_NORMAL, normal_power=power, sigma_color=1e30)
+    want = 3.0 / 32.0 * z.astype(np.float64) ** power
+    assert np.abs(got / want - 1.0).max() <= 3.0 * 2.0 ** -23
+
+
+def test_normals_longer_than_one_overflow_as_a_power_does():
+    """A cosine above 1 whose power exceeds the largest float: the weight is
+    infinite and the mean not a number, as with powf."""
+    normals = np.tile(np.array([[0.0, 0.0, 100.0]], np.float32), (4, 1))
+    bufs = pairs(4, normals, np.ones(4))
+    got = [tap_weight(bufs, kgr.DENOISE_NORMAL, normal_power=p, sigma_color=1e30) for p in (64.0, 65.0)]
+    assert np.isnan(got[0]).all() and np.isnan(got[1]).all()
