@@ -29,6 +29,8 @@
  * end, so texture and material detail is not blurred.  Pixels without a hit
  * (zero normal) only average among themselves.
  */
+#include <float.h>
+
 #include "kgr_post.h"
 
 namespace kgr {
@@ -101,6 +103,27 @@ __device__ __forceinline__ float rcp(float x)
 	return r;
 }
 
+/* a / b, within an ulp: the product with the reciprocal and what its residual
+ * a - b q (exact in a fused operation; Markstein 1990) adds to it.  Where the
+ * residual is not a number the product is 0 or infinite already, as the
+ * quotient is. */
+__device__ __forceinline__ float quotient(float a, float b)
+{
+	const float r = rcp(b), q = a * r;
+	const float t = __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
+	return t == t ? t : q;
+}
+
+/* a / sqrt(x), within two ulp, x > 0: a step of Newton's iteration on the
+ * reciprocal root.  A residual that is not a number (x infinite, r 0) counts
+ * as 1. */
+__device__ __forceinline__ float over_root(float a, float x)
+{
+	const float r = rsqrtf(x), q = a * r;
+	const float h = fminf(__fmaf_rn(-x * r, r, 1.0f), 1.0f);
+	return __fmaf_rn(q * 0.5f, h, q);
+}
+
 __device__ __forceinline__ float3 albedo_div(float4 a)
 {
 	return make_float3(a.x > 1e-3f ? a.x : 1.0f, a.y > 1e-3f ? a.y : 1.0f, a.z > 1e-3f ? a.z : 1.0f);
@@ -114,8 +137,8 @@ __device__ __forceinline__ float squared(float c, int n)
 	float lo = 0.0f;
 #pragma unroll
 	for (int q = 1; q < n; q++) {
-		float sq = c * c;
-		lo = __fmaf_rn(c + c, lo, __fmaf_rn(c, c, -sq));
+		const float sq = c * c, e = __fmaf_rn(c, c, -sq);
+		lo = q == 1 ? e : __fmaf_rn(c + c, lo, e);
 		c = sq;
 	}
 	return n ? fminf(__fmaf_rn(c, c, (c + c) * lo), INFINITY) : c;
@@ -148,7 +171,7 @@ struct AtrousPass {
 	uint32_t width, height;
 	int step;
 	float half_sigma;    /* sigma_color 2^-i / 2 */
-	float position_rate; /* 1 / sigma_position */
+	float position_rate; /* 1 / sigma_position, finite */
 	float normal_power;
 	int squarings;       /* POWER_64, POWER_SQUARES: normal_power = 2^squarings */
 	int remodulate;      /* the last pass of an albedo-guided filter */
@@ -183,10 +206,11 @@ __device__ __forceinline__ void atrous_taps(AtrousPixel &p, const float4 *__rest
 			const float3 cq = f3of(in[iq]);
 			const float3 nq = f3of(normal[iq]);
 			const float3 xq = POSITION ? f3of(position[iq]) : p.pos;
-			const bool hit_q = nq.x != 0.0f || nq.y != 0.0f || nq.z != 0.0f;
+			/* not all zero (of either sign) */
+			const bool hit_q = ((__float_as_uint(nq.x) | __float_as_uint(nq.y) | __float_as_uint(nq.z)) << 1) != 0u;
 			const float lq = lum(cq);
 			float w = spline(dx) * spline(dy) *
-				__expf(-fabsf(p.l - lq) * rcp(__fmaf_rn(ps.half_sigma, p.l + lq, 1e-4f)));
+				expf(-quotient(fabsf(p.l - lq), __fmaf_rn(ps.half_sigma, p.l + lq, 1e-4f)));
 			if (p.hit) {
 				if (POWER != POWER_NONE) {
 					float c = fmaxf(p.n.x * nq.x + p.n.y * nq.y + p.n.z * nq.z, 0.0f);
@@ -195,37 +219,43 @@ __device__ __forceinline__ void atrous_taps(AtrousPixel &p, const float4 *__rest
 				if (POSITION && (dx != 0 || dy != 0)) {
 					float3 v = make_float3(xq.x - p.pos.x, xq.y - p.pos.y, xq.z - p.pos.z);
 					float len2 = dot3(v, v);
-					float d = len2 > 0.0f ? fabsf(dot3(p.n, v)) * rsqrtf(len2) : 0.0f;
-					w *= __expf(-d * ps.position_rate);
+					float d = len2 > 0.0f ? over_root(fabsf(dot3(p.n, v)), len2) : 0.0f;
+					w *= expf(-d * ps.position_rate);
 				}
 			}
 			/* a tap of the other kind adds nothing, whatever its colour */
-			const bool ok = p.hit == hit_q;
-			w = ok ? w : 0.0f;
-			p.sum.x = __fmaf_rn(w, ok ? cq.x : 0.0f, p.sum.x);
-			p.sum.y = __fmaf_rn(w, ok ? cq.y : 0.0f, p.sum.y);
-			p.sum.z = __fmaf_rn(w, ok ? cq.z : 0.0f, p.sum.z);
-			p.wsum += w;
+			if (p.hit == hit_q) {
+				p.sum.x = __fmaf_rn(w, cq.x, p.sum.x);
+				p.sum.y = __fmaf_rn(w, cq.y, p.sum.y);
+				p.sum.z = __fmaf_rn(w, cq.z, p.sum.z);
+				p.wsum += w;
+			}
 		}
 	}
 }
 
 /* One a-trous pass, one pixel a thread.
  *
- * Bound by the arithmetic of a tap (issue slots 62% busy, L1 24%, DRAM 8%).  The
- * divisions are products with a reciprocal or a reciprocal square root (MUFU,
- * 1 ulp); a power-of-two exponent is that many squarings, good to an ulp also
- * where the normals are means of several samples' and the weights denormal
- * numbers (plain squarings for the others and a second loop for these: 781 us
- * behind a frame of one sample a pixel, but 1430 to 1560 behind several, 2330
- * on the box scene); the sums are fused.
- * The three weights are multiplied in this order because the power may leave
- * only a few bits of a denormal number.  1080p, five passes, all guides: 1787
- * -> 831 us, and 1722 -> 833 behind four samples a pixel (the first pass no
- * longer divides every tap by its albedo: demodulate_kernel).  Two pixels of a
- * column a thread, which halves the loads, were no faster; all 25 taps unrolled
- * 840 to 930 us, waiting for instructions; a branch past the loads of a tap of
- * the other kind 900 us; no cap on the registers 812 us. */
+ * Bound by the arithmetic of a tap (issued instructions; L1 and DRAM are far
+ * from busy).  Every step of a weight is good to an ulp or two, but cheaper than
+ * its general form: quotients from the MUFU's reciprocal and a residual, a
+ * Newton step on the reciprocal root, squarings that carry their error for the
+ * power of two, fused sums.  One loop for every pixel: normals that are means
+ * of several samples' give weights down to the denormal numbers, whose result
+ * hangs on the roundings, and the three weights are multiplied in this order
+ * because the power may leave only a few bits of one.
+ *
+ * 1080p, five passes, every guide, behind 1 and 4 samples a pixel on the
+ * terrain, then on the box scene: 1785, 1722, 2350, 2146 us with divisions,
+ * powf and a demodulation of every tap (demodulate_kernel has taken that out),
+ * now 847, 851, 1030, 1030; the error against 64 bits is 0.96 to 1.00 of what
+ * it was.  Bare MUFU results, plain squarings (32 ulp) and a second loop for
+ * averaged normals took 781, 1553, 908, 2332 us and left a weight several
+ * times the error.  Two pixels of a column a thread, which halves the loads, were no
+ * faster; packed operations on two taps (f32x2) 15% slower; all 25 taps
+ * unrolled 840 to 930 us where this loop took 781, waiting for instructions; a
+ * branch past the loads of a tap of the other kind 900; 8, 9, 11 and 12 blocks
+ * an SM 1 to 5% slower. */
 template <int POWER, bool POSITION>
 __global__ void __launch_bounds__(128, 10) atrous_kernel(const float4 *__restrict__ in, float4 *__restrict__ out,
 		const float4 *__restrict__ normal, const float4 *__restrict__ albedo, const float4 *__restrict__ position,
@@ -281,7 +311,8 @@ void denoise(const float4 *color, const float4 *normal, const float4 *albedo, co
 	AtrousPass ps;
 	ps.width = width;
 	ps.height = height;
-	ps.position_rate = 1.0f / p.sigma_position;
+	/* not infinite for a denormal sigma: a distance of 0 weighs 1 */
+	ps.position_rate = fminf(1.0f / p.sigma_position, FLT_MAX);
 	ps.normal_power = p.normal_power;
 	ps.squarings = 0;
 	int power = POWER_NONE;

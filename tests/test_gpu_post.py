@@ -189,3 +189,64 @@ def test_normals_longer_than_one_overflow_as_a_power_does():
     bufs = pairs(4, normals, np.ones(4))
     got = [tap_weight(bufs, kgr.DENOISE_NORMAL, normal_power=p, sigma_color=1e30) for p in (64.0, 65.0)]
     assert np.isnan(got[0]).all() and np.isnan(got[1]).all()
+
+
+def test_color_weight_is_good_to_its_argument():
+    """The argument x = l / (sigma l / 2 + 1e-4) has three rounded steps
+    (2^-24 relative each; the luminance's own rounding cancels but for the
+    1e-4); the exponential may be 2 ulp off, the other steps 2 ulp."""
+    rng = np.random.default_rng(3)
+    sigma = 2.0 / 64.0
+    c = rng.uniform(0.5, 8.0, 4096).astype(np.float32)
+    normals = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (len(c), 1))
+    got = tap_weight(pairs(len(c), normals, c), kgr.DENOISE_NONE, sigma_color=sigma)
+    k = [float(np.float32(v)) for v in (0.2126, 0.7152, 0.0722)]
+    lum = c.astype(np.float64) * sum(k)
+    x = lum / (0.5 * sigma * lum + float(np.float32(1e-4)))
+    want = 3.0 / 32.0 * np.exp(-x)
+    # the luminance's rounding (3 ulp at most) changes x by 1e-4 / (sigma l / 2) of itself
+    bound = x * (3.0 * 2.0 ** -24 + 3.0 * 2.0 ** -23 * 1e-4 / (0.5 * sigma * lum)) + 4.0 * 2.0 ** -23
+    assert (np.abs(got / want - 1.0) <= bound).all()
+
+
+def test_position_weight_is_good_to_its_argument():
+    """The argument d / sigma: the squared length (two rounded steps, half of
+    them through the root), the quotient over the root (3.5), the rate and
+    its product: 6.5 x 2^-24 relative; the exponential and the rest 4 ulp."""
+    rng = np.random.default_rng(4)
+    n, sigma = 4096, 1.0 / 64.0
+    q = np.zeros((n, 3), np.float32)
+    q[:, 0], q[:, 2] = rng.uniform(0.5, 2.0, n), rng.uniform(0.2, 1.0, n)
+    normals = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (n, 1))
+    got = tap_weight(pairs(n, normals, np.ones(n), q), kgr.DENOISE_POSITION, sigma_color=1e30, sigma_position=sigma)
+    v = q.astype(np.float64)
+    x = v[:, 2] / np.sqrt((v * v).sum(1)) / sigma
+    want = 3.0 / 32.0 * np.exp(-x)
+    assert (np.abs(got / want - 1.0) <= x * 6.5 * 2.0 ** -24 + 4.0 * 2.0 ** -23).all()
+
+
+@pytest.mark.parametrize("sigma_position", [1e-39, 1e-30, 1e30])
+def test_extreme_sigmas_and_values(sigma_position):
+    """Taps in the centre's plane weigh 1 whatever the sigma; positions and
+    colours whose squares or sums leave the range of a float, and negative
+    colours that make a denominator 0, give what the formula gives."""
+    n = 4
+    normals = np.tile(np.array([[0.0, 0.0, 1.0]], np.float32), (n, 1))
+    q = np.array([[1.0, 0, 0], [1e-30, 0, 0], [1e25, 0, 0], [3e38, 0, 0]], np.float32)
+    got = tap_weight(pairs(n, normals, np.ones(n), q), kgr.DENOISE_POSITION, sigma_color=1e30,
+                     sigma_position=sigma_position)
+    np.testing.assert_allclose(got, 3.0 / 32.0, rtol=1e-6)
+    # luminances of 3e38 (their sum is infinite, the weight 1), and of -1e-4 with sigma 2 (the denominator 0,
+    # the weight exp(-inf))
+    for color, sigma, weight in ((3e38, 2.0, 3.0 / 32.0), (-1e-4, 2.0, 0.0)):
+        bufs = pairs(n, normals, np.full(n, color, np.float32))
+        if color > 0:
+            bufs[0][::3, 0, :3] = 1e38
+        dev = [torch.from_numpy(b).cuda() for b in bufs]
+        dn = kgr.Denoiser(2, 3 * n, kgr.DENOISE_NONE)
+        dn.denoise(dev[0].data_ptr(), dev[1].data_ptr(), iterations=1, sigma_color=sigma)
+        torch.cuda.synchronize()
+        r = result_array(dn, 2, 3 * n).reshape(3 * n, 2, 4)[::3, 0, 0]
+        dn.close()
+        c0, c1 = float(bufs[0][0, 0, 0]), float(np.float32(color))
+        np.testing.assert_allclose(r, (c0 * 9 / 64 + weight * c1) / (9 / 64 + weight), rtol=1e-5)
