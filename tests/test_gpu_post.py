@@ -250,3 +250,28 @@ def test_extreme_sigmas_and_values(sigma_position):
         dn.close()
         c0, c1 = float(bufs[0][0, 0, 0]), float(np.float32(color))
         np.testing.assert_allclose(r, (c0 * 9 / 64 + weight * c1) / (9 / 64 + weight), rtol=1e-5)
+
+
+@pytest.mark.parametrize("own_result", [False, True])
+@pytest.mark.parametrize("iterations", [1, 2, 4, 5])
+def test_albedo_guide_at_every_parity_of_the_passes(iterations, own_result):
+    """The demodulated image goes where the first pass does not write, scratch
+    or result by the number of passes; the colour may be the denoiser's own
+    result buffer."""
+    g, sc, _ = helpers.both("box4k", 1)
+    w, h = 53, 35
+    bufs = render_with_aovs(g, sc, w, h, 2, 9)
+    dn = kgr.Denoiser(w, h)
+    cpu = [b.cpu().numpy().reshape(h, w, 4) for b in bufs]
+    color = bufs[0].data_ptr()
+    if own_result:
+        dn.denoise(*[b.data_ptr() for b in bufs], iterations=3)
+        torch.cuda.synchronize()
+        cpu[0] = result_array(dn, w, h).reshape(h, w, 4).copy()
+        color = dn.result()
+    dn.denoise(color, *[b.data_ptr() for b in bufs[1:]], iterations=iterations)
+    torch.cuda.synchronize()
+    got = result_array(dn, w, h).reshape(h, w, 4)
+    ref = post_ref.denoise(*cpu, 7, iterations=iterations)
+    np.testing.assert_allclose(got, ref, rtol=1e-4, atol=1e-6)
+    dn.close()
