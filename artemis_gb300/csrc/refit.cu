@@ -28,6 +28,7 @@
  */
 #include <float.h>
 
+#include "kgr_cw8.h"
 #include "kgr_internal.h"
 #include "kgr_wavefront.h"
 
@@ -281,7 +282,7 @@ __device__ __forceinline__ float pow2i(int k) { return ldexpf(1.0f, k); }
 
 /* cw_axis_grid of kgr_cw8.h: the same exponent and origin with all but one
  * operation in single precision (the origin's rounding, which has to see the
- * double). */
+ * double); for extents up to half the largest float. */
 __device__ __forceinline__ void axis_grid(float lo, float hi, int &e, float &p)
 {
 	float d, r;
@@ -332,6 +333,28 @@ __device__ __forceinline__ uint32_t plane_hi(float plane, float p, int e)
 	float x = ldexpf(d, -e), f = floorf(x), r = x - f;
 	float q = (r > 0.5f || (r == 0.5f && t > 0.0f)) ? f + 2.0f : f + 1.0f;
 	return (uint32_t)fminf(fmaxf(q, 0.0f), 255.0f);
+}
+
+/* Slot j of a node whose extent [lo, hi] a float may not hold, by the double
+ * precision rules themselves.  Out of line: the others' registers do not see
+ * it (inlined, a refit of the 1.16M-triangle terrain took 5 us longer). */
+__device__ __noinline__ void wide_slot(CwNode *node, uint32_t j, bool used, uint32_t imask, f3 lo, f3 hi, f3 mn, f3 mx)
+{
+	uint8_t *q = reinterpret_cast<uint8_t *>(&node->qa) + j;
+	const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
+	const float a[3] = {mn.x, mn.y, mn.z}, b[3] = {mx.x, mx.y, mx.z};
+	uint32_t bits = imask << 24;
+	float p[3];
+	for (int x = 0; x < 3; x++) {
+		int e;
+		cw_axis_grid(l[x], h[x], e, p[x]);
+		bits |= (uint32_t)(e + 127) << (8 * x);
+		const double s = ldexp(1.0, e);
+		q[8 * x] = (uint8_t)(used ? cw_qlo(a[x], p[x], s) : 255u);
+		q[24 + 8 * x] = (uint8_t)(used ? cw_qhi(b[x], p[x], s) : 0u);
+	}
+	if (j == 0u)
+		node->origin = make_float4(p[0], p[1], p[2], __uint_as_float(bits));
 }
 
 /* The slots of the eight-child nodes, one a thread, eight lanes a node: the
@@ -403,6 +426,11 @@ __global__ void __launch_bounds__(REFIT_BLOCK) slot_nodes_kernel(const int32_t *
 		}
 		if (!in)
 			continue;
+		if (!(fmaxf(hi[0] - lo[0], fmaxf(hi[1] - lo[1], hi[2] - lo[2])) < 0.5f * FLT_MAX)) {
+			wide_slot(&cw[c], j, k >= 0, imask, mk(lo[0], lo[1], lo[2]), mk(hi[0], hi[1], hi[2]), mk(mn[0], mn[1], mn[2]),
+				mk(mx[0], mx[1], mx[2]));
+			continue;
+		}
 		/* planes: lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, a byte a slot */
 		uint8_t *q = reinterpret_cast<uint8_t *>(&cw[c].qa) + j;
 		for (int x = 0; x < 3; x++) {

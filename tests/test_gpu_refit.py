@@ -329,3 +329,24 @@ def test_refit_requantises_the_compressed_layout(gen):
     sc.set_transforms([1, 2], [M0[1], M0[2]])
     assert np.array_equal(sc.array(kgr.ARRAY_CW8_NODES), before)
     sc.close()
+
+
+@pytest.mark.parametrize("scale", [1e30, 1.6e38, 1.75e38, 2e38, 3e38])
+def test_refit_of_scenes_as_wide_as_a_float(scale):
+    """Extents up to and above the largest float: the compressed nodes of a
+    refit to the same positions are those that the host builder made (their
+    bytes; nothing is traced)."""
+    rng = np.random.default_rng(5)
+    n = 300
+    at = rng.uniform(-1.0, 1.0, (n, 1, 3))
+    pos = ((at + rng.uniform(-0.01, 0.01, (n, 3, 3))).clip(-1.0, 1.0) * scale).astype(np.float32).reshape(-1, 3)
+    idx = np.arange(3 * n, dtype=np.uint32).reshape(-1, 3)
+    g = kgr.Generated("box4k", 1)
+    sc = kgr.Scene(pos, idx, g.materials_raw, builder=kgr.BUILDER_SAH_HOST)
+    assert sc.info().cw8_node_count > 0
+    before = sc.array(kgr.ARRAY_CW8_NODES).copy()
+    dev = torch.from_numpy(pos).cuda()
+    sc.refit(dev.data_ptr())
+    torch.cuda.synchronize()
+    assert np.array_equal(sc.array(kgr.ARRAY_CW8_NODES), before)
+    sc.close()
