@@ -106,7 +106,7 @@ void batch_frame(const DeviceScene &s, const PathBuffers &pb, const FrameParams 
 		/* the plain tracer's overlap (render_pt): bounce d's shadow rays on
 		 * the side stream, bounce d + 1's closest hits here, joined before
 		 * the next shade */
-		pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
+		pt_trace_camera(s, pb, fp.layout, fp.tune, st);
 		for (int d = 0; d <= fp.max_depth; d++) {
 			int q = d & 1;
 			pt_shade(s, pb, fp, d, q, st);
@@ -121,7 +121,10 @@ void batch_frame(const DeviceScene &s, const PathBuffers &pb, const FrameParams 
 	} else {
 		for (int d = 0; d <= fp.max_depth; d++) {
 			int q = d & 1;
-			pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
+			if (d == 0)
+				pt_trace_camera(s, pb, fp.layout, fp.tune, st);
+			else
+				pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 			pt_shade(s, pb, fp, d, q, st);
 			pt_shadow_resolve(s, pb, fp.layout, fp.tune, st);
 		}

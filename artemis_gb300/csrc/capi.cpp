@@ -1240,7 +1240,7 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 		att->ensure_side_stream();
 		cudaStream_t side = att->side;
 		pb.likely_rays = likely_rays(fp.paths, 0);
-		pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
+		pt_trace_camera(s, pb, fp.layout, fp.tune, st);
 		m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 		for (int d = 0; d <= last; d++) {
 			int q = d & 1;
@@ -1267,7 +1267,10 @@ void render_pt(kgr_attachment *att, const kgr_launch_info *info, const kgr_scene
 		for (int d = 0; d <= last; d++) {
 			int q = d & 1;
 			pb.likely_rays = likely_rays(fp.paths, d);
-			pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
+			if (d == 0)
+				pt_trace_camera(s, pb, fp.layout, fp.tune, st);
+			else
+				pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 			m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 			pt_shade(s, pb, fp, d, q, st);
 			m = att->mark(STAGE_SHADE, st, m);
@@ -1389,7 +1392,7 @@ void render_restir_di(kgr_attachment *att, const kgr_launch_info *info, const kg
 	pt_generate(pb, fp, st);
 	att->mark(STAGE_GENERATE, st);
 	pb.likely_rays = likely_rays(fp.paths, 0);
-	pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
+	pt_trace_camera(s, pb, fp.layout, fp.tune, st);
 	att->mark(STAGE_TRACE_CLOSEST, st);
 	restir_primary(s, pb, fp, rb, cur, st);
 	att->mark(STAGE_RESTIR_PRIMARY, st);
@@ -1587,7 +1590,7 @@ void render_pt_cached(kgr_attachment *att, const kgr_launch_info *info, const kg
 	pt_generate(pb, fp, st);
 	m = att->mark(STAGE_GENERATE, st, m);
 	pb.likely_rays = likely_rays(fp.paths, 0);
-	pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
+	pt_trace_camera(s, pb, fp.layout, fp.tune, st);
 	m = att->mark(STAGE_TRACE_CLOSEST, st, m);
 	pt_shade(s, pb, fp, 0, 0, st);
 	m = att->mark(STAGE_SHADE, st, m);
@@ -1701,7 +1704,7 @@ void render_restir_gi(kgr_attachment *att, const kgr_launch_info *info, const kg
 	pt_generate(pb, fp, st);
 	att->mark(STAGE_GENERATE, st);
 	pb.likely_rays = likely_rays(fp.paths, 0);
-	pt_trace_closest(s, pb, 0, fp.layout, fp.tune, st);
+	pt_trace_camera(s, pb, fp.layout, fp.tune, st);
 	att->mark(STAGE_TRACE_CLOSEST, st);
 	gi_primary(s, pb, fp, gb, st);
 	att->mark(STAGE_RESTIR_PRIMARY, st);

@@ -462,11 +462,16 @@ __device__ __forceinline__ bool test_leaves(const DeviceScene &s, const FastRay 
 /* Lanes of a warp that still walk when the persistent walk fetches new rays.
  * With many rays a lane (at least KGR_REFILL_ROUNDS of them) a fetch waits
  * until few enough walk: a fetch runs for all 32 lanes whoever needs it, and
- * rays that start together stay together.  1080p terrain frame at 31, 24, 20,
- * 16, 12, 8: 10.75, 10.62, 10.54, 10.51, 10.55, 10.67 ms; 2,073,600 bounce rays
- * 862, 863, 877, 883, 896, 914 us, camera rays 525, 503, 485, 483, 486, 476.
- * With few, an idle lane costs more than the fetch. */
+ * rays that start together stay together.  At 31, 24, 20, 16, 12, 8 on the
+ * terrain 2,073,600 camera rays 525, 503, 485, 483, 486, 476 us, bounce rays 862,
+ * 863, 877, 883, 896, 914: bounces have a value of their own, since in a closed
+ * scene most rays are bounces.  960x540, 2 samples, depth 8 on the box scene
+ * with bounces at 18, 24, 31: 8.74, 8.64, 8.64 ms (8.67 with one ray fetched for
+ * each that ends); 1080p, 4 samples on the terrain 10.12, 10.09, 10.10, with
+ * camera rays at 24 10.21.  Shadow rays at 18, 24, 31 the same within 0.2%.
+ * With few rays, an idle lane costs more than the fetch. */
 #define KGR_REFILL_MANY 18
+#define KGR_REFILL_BOUNCE 24
 #define KGR_REFILL_FEW 31
 #define KGR_REFILL_ROUNDS 2u
 

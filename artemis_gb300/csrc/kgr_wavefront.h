@@ -65,6 +65,8 @@ struct PathBuffers {
 	/* how many rays the next walk is likely to have, as far as the host knows
 	 * (0: it does not); only the launch's register bound follows it */
 	uint32_t likely_rays = 0;
+	/* the next closest-hit walk's rays leave the camera (pt_trace_camera) */
+	bool camera = false;
 };
 
 /* The rays of bounce `depth`: on a scene open to the sky about half a bounce's
@@ -229,6 +231,8 @@ struct OutputBuffers {
 void pt_generate(const PathBuffers &pb, const FrameParams &fp, cudaStream_t st);
 void pt_trace_closest(const DeviceScene &s, const PathBuffers &pb, int q, int layout, const TraceTune &tune,
 		cudaStream_t st);
+/* pt_trace_closest for queue 0's camera rays */
+void pt_trace_camera(const DeviceScene &s, const PathBuffers &pb, int layout, const TraceTune &tune, cudaStream_t st);
 void pt_shade(const DeviceScene &s, const PathBuffers &pb, const FrameParams &fp, int depth, int q,
 		cudaStream_t st);
 /* shade that also advances the RNG at the last depth (ReSTIR keeps the

@@ -1741,7 +1741,7 @@ uint32_t mamba_render(const DeviceScene &s, const PathBuffers &pb, const MambaPa
 	uint32_t launches = 0;
 	gbuffer_rays_kernel<<<blocks_for(npix, 256), 256, 0, st>>>(pb, mp);
 	done(STAGE_GENERATE);
-	pt_trace_closest(s, pb, 0, mp.layout, tune, st);
+	pt_trace_camera(s, pb, mp.layout, tune, st);
 	done(STAGE_TRACE_CLOSEST);
 	gbuffer_store_kernel<<<blocks_for(npix, 256), 256, 0, st>>>(s, pb, mp, mb);
 	done(STAGE_GENERATE);

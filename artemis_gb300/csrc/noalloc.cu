@@ -158,7 +158,10 @@ extern "C" kgr_status kgr_render_pt_noalloc(const kgr_scene *sc, const kgr_launc
 		pt_generate(pb, fp, st);
 		for (int d = 0; d <= fp.max_depth; d++) {
 			int q = d & 1;
-			pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
+			if (d == 0)
+				pt_trace_camera(s, pb, fp.layout, fp.tune, st);
+			else
+				pt_trace_closest(s, pb, q, fp.layout, fp.tune, st);
 			pt_shade(s, pb, fp, d, q, st);
 			pt_shadow_resolve(s, pb, fp.layout, fp.tune, st);
 		}

@@ -363,7 +363,8 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) fast_persis
 	}
 	int32_t local_stack[KGR_STACK_DEPTH - SHORT];
 	typename StackOf<SHORT, BLOCK>::type stack(short_stack + threadIdx.x, local_stack);
-	persistent_walk<ANY, COUNT, LAYOUT>(s, stack, n >= KGR_REFILL_ROUNDS * threads ? KGR_REFILL_MANY : KGR_REFILL_FEW, &cnt,
+	const int many = ANY || pb.camera ? KGR_REFILL_MANY : KGR_REFILL_BOUNCE;
+	persistent_walk<ANY, COUNT, LAYOUT>(s, stack, n >= KGR_REFILL_ROUNDS * threads ? many : KGR_REFILL_FEW, &cnt,
 		[&](bool need, float4 &a, float4 &b) {
 			unsigned m = __ballot_sync(0xffffffffu, need);
 			int leader = __ffs(m) - 1;
@@ -626,6 +627,13 @@ void pt_trace_closest(const DeviceScene &s, const PathBuffers &pb, int q, int la
 		}
 	}
 	KGR_CUDA(cudaGetLastError());
+}
+
+void pt_trace_camera(const DeviceScene &s, const PathBuffers &pb, int layout, const TraceTune &tune, cudaStream_t st)
+{
+	PathBuffers camera = pb;
+	camera.camera = true;
+	pt_trace_closest(s, camera, 0, layout, tune, st);
 }
 
 void pt_shade(const DeviceScene &s, const PathBuffers &pb, const FrameParams &fp, int depth, int q,
