@@ -737,8 +737,7 @@ __global__ void __launch_bounds__(128) gi_visibility_walk_kernel(DeviceScene s, 
 	LocalStack stack(nullptr, entries);
 	uint32_t slot = 0;
 	persistent_walk<true, false, LAYOUT>(s, stack, GI_VIS_REFILL, nullptr,
-		[&](bool need, float4 &a, float4 &b) {
-			const uint32_t m = __ballot_sync(0xffffffffu, need);
+		[&](bool need, unsigned m, float4 &a, float4 &b) {
 			const int leader = __ffs(m) - 1;
 			uint32_t base = 0;
 			if ((int)lane == leader)

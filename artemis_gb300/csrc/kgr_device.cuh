@@ -480,8 +480,8 @@ __device__ __forceinline__ bool test_leaves(const DeviceScene &s, const FastRay 
  * a lane whose ray ends early does not idle until the longest ray of its warp
  * is done.  One iteration descends to a leaf with the postponed-leaf rule
  * (speculative_descend) and tests it.  All 32 lanes call it.
- *   next(need, a, b)   warp-collective: whether a lane that needs a ray got
- *                      one, {origin, -} and {direction, tmax}
+ *   next(need, m, a, b)  warp-collective: whether a lane that needs a ray (m:
+ *                      the warp's) got one, {origin, -} and {direction, tmax}
  *   done(best, hit)    the lane's ray is finished (hit: occluded, for ANY) */
 template <bool ANY, bool COUNT, int LAYOUT, class STACK, class Next, class Done>
 __device__ __forceinline__ void persistent_walk(const DeviceScene &s, STACK &stack, int refill, TraceCounters *cnt,
@@ -494,9 +494,12 @@ __device__ __forceinline__ void persistent_walk(const DeviceScene &s, STACK &sta
 	int32_t ref = 0;
 	for (;;) {
 		bool need = !have && !exhausted;
-		if (__popc(__ballot_sync(0xffffffffu, have)) <= refill && __any_sync(0xffffffffu, need)) {
+		/* the last rays' lanes walk alone for long: one vote an iteration
+		 * once the others have no ray to wait for */
+		const unsigned m = __ballot_sync(0xffffffffu, need);
+		if (m && __popc(__ballot_sync(0xffffffffu, have)) <= refill) {
 			float4 a, b;
-			if (next(need, a, b)) {
+			if (next(need, m, a, b)) {
 				r = fast_ray(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z));
 				best.prim = -1;
 				best.t = b.w;

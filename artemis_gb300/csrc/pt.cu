@@ -365,8 +365,7 @@ __global__ void __launch_bounds__(BLOCK, KGR_MIN_BLOCKS(BLOCK, OCC)) fast_persis
 	typename StackOf<SHORT, BLOCK>::type stack(short_stack + threadIdx.x, local_stack);
 	const int many = ANY || pb.camera ? KGR_REFILL_MANY : KGR_REFILL_BOUNCE;
 	persistent_walk<ANY, COUNT, LAYOUT>(s, stack, n >= KGR_REFILL_ROUNDS * threads ? many : KGR_REFILL_FEW, &cnt,
-		[&](bool need, float4 &a, float4 &b) {
-			unsigned m = __ballot_sync(0xffffffffu, need);
+		[&](bool need, unsigned m, float4 &a, float4 &b) {
 			int leader = __ffs(m) - 1;
 			uint32_t base = 0;
 			if (lane == leader)

@@ -86,8 +86,7 @@ __device__ __forceinline__ void trace_refill(const DeviceScene &s, const float4 
 	LocalStack stack(nullptr, entries);
 	uint32_t i = 0;
 	persistent_walk<ANY, false, LAYOUT>(s, stack, refill, nullptr,
-		[&](bool need, float4 &a, float4 &b) {
-			unsigned m = __ballot_sync(0xffffffffu, need);
+		[&](bool need, unsigned m, float4 &a, float4 &b) {
 			int leader = __ffs(m) - 1;
 			uint32_t base = 0;
 			if (lane == leader)
