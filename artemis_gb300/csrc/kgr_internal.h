@@ -178,7 +178,11 @@ struct CoopNode {
 	float4 slot[16];
 };
 /* The cooperative walk runs when there are at most this many rays for each of
- * the groups the GPU holds at once (19,456 to 23,104 of them).  Closest-hit
+ * the groups that the launch holds at once: 19,456 of them, 24,320 and 29,184
+ * where the launch's bound on the registers is 48 and 40.  The limit follows
+ * the bound because the per-thread walk spills under it and loses more: 256x256
+ * and 300x300 with the cap of 40 on the larger terrain 570, 672 us, with the
+ * limit of 19,456 groups 622, 687 (box scene 906, 975 and 902, 971).  Closest-hit
  * bounce rays on the box scene, the 0.26M- and the 1.16M-triangle terrain, us,
  * this walk / the persistent one: 4,096 rays 31, 39, 43 / 48, 45, 58; 16,384
  * rays 33, 45, 60 / 70, 68, 75; 65,536 rays 83, 88, 107 / 97, 91, 114; 131,072
@@ -192,6 +196,12 @@ struct CoopNode {
  * on the box scene 85 us with this walk and 66 with one ray per thread, 40,000
  * of them 54 and 70. */
 #define KGR_COOP_ROUNDS_RAYS 3u
+/* So camera walks of frames take that limit too where nodes and triangles are
+ * about what two SMs' L1 hold and the per-thread walk seldom waits for L2.
+ * Cached frames of 256x256 and 276x276 on the box scene (437 KB) with 4 rounds
+ * 248, 264 us and with 3 235, 241; its triangles divided into 16,944 (1.5 MB)
+ * 287, 303 and 293, 298, into 67,776 323, 342 and 342, 349. */
+#define KGR_SMALL_TREE (512u << 10)
 /* most nodes on a path of the cooperative walk */
 #define KGR_COOP_LEVELS 16
 

@@ -632,6 +632,11 @@ void pt_trace_camera(const DeviceScene &s, const PathBuffers &pb, int layout, co
 {
 	PathBuffers camera = pb;
 	camera.camera = true;
+	/* camera rays on a tree that stays in L1: the cooperative walk loses
+	 * earlier */
+	const size_t tree = (size_t)s.fast_node_count * sizeof(FastNode) + (size_t)s.triangle_count * 3 * sizeof(float4);
+	if (tree <= KGR_SMALL_TREE && camera.coop_rounds > KGR_COOP_ROUNDS_RAYS)
+		camera.coop_rounds = KGR_COOP_ROUNDS_RAYS;
 	pt_trace_closest(s, camera, 0, layout, tune, st);
 }
 
