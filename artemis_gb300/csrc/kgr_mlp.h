@@ -43,14 +43,15 @@ void mlp_infer_tc(const MlpParams &mp, const void *x, uint32_t n, float4 *out, u
  * its loss in the slice's MLP_LOSS_SLOT and nothing in the other unused
  * outputs; sets bit 0 of *mp.tc_err if a wait ran out. */
 void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, cudaStream_t st,
-		const uint32_t *n_dev);
+		const uint32_t *n_dev, bool withhold = false);
 /* grad (FP32, [6][64][64]) = d loss / d W over n rows; loss = sum of the
  * relative L2 terms (not divided by n).  Uses mp.partial as scratch; the
  * result does not depend on block scheduling.  max_blocks > 0 caps the grid
  * (each block takes one SM's shared memory): training that runs beside a
- * frame leaves the other SMs to the frame. */
+ * frame leaves the other SMs to the frame.  withhold: a test of the tcgen05
+ * kernel's bounded waits. */
 void mlp_gradients(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, float *grad, float *loss,
-		cudaStream_t st, const uint32_t *n_dev = nullptr, int max_blocks = 0);
+		cudaStream_t st, const uint32_t *n_dev = nullptr, int max_blocks = 0, bool withhold = false);
 /* One Adam step (lr, bias correction for `step`); step <= 0 only refreshes
  * the half-precision copies from the master weights. */
 void mlp_adam(const MlpParams &mp, const float *grad, float lr, int step, cudaStream_t st);

@@ -599,7 +599,7 @@ constexpr int REDUCE_GRID = (MLP_LAYERS * MLP_W * MLP_W + REDUCE_THREADS - 1) / 
 /* The blocks' slices of the gradient over n > 0 rows.  Returns their number,
  * and in *summed whether the loss is in them (else it is in *loss). */
 int train_pass(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, float *loss, cudaStream_t st,
-		const uint32_t *n_dev, int max_blocks, bool *summed)
+		const uint32_t *n_dev, int max_blocks, bool *summed, bool withhold = false)
 {
 	size_t sm = train_smem();
 	int grid = mp.partial_blocks;
@@ -612,7 +612,7 @@ int train_pass(const MlpParams &mp, const void *x, const float4 *target, uint32_
 		grid = (int)tiles;
 	KGR_REQUIRE(grid >= 1 && mp.partial, KGR_ERR_INTERNAL, "MLP gradient scratch missing");
 	if (*summed) {
-		mlp_train_tc(mp, x, target, n, grid, st, n_dev);
+		mlp_train_tc(mp, x, target, n, grid, st, n_dev, withhold);
 		return grid;
 	}
 	KGR_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), st));
@@ -643,7 +643,7 @@ AdamState adam_state(const MlpParams &mp, float lr, int step)
 } /* namespace */
 
 void mlp_gradients(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, float *grad, float *loss,
-		cudaStream_t st, const uint32_t *n_dev, int max_blocks)
+		cudaStream_t st, const uint32_t *n_dev, int max_blocks, bool withhold)
 {
 	if (n == 0) {
 		KGR_CUDA(cudaMemsetAsync(loss, 0, sizeof(float), st));
@@ -651,7 +651,7 @@ void mlp_gradients(const MlpParams &mp, const void *x, const float4 *target, uin
 		return;
 	}
 	bool summed;
-	int blocks = train_pass(mp, x, target, n, loss, st, n_dev, max_blocks, &summed);
+	int blocks = train_pass(mp, x, target, n, loss, st, n_dev, max_blocks, &summed, withhold);
 	reduce_partials_kernel<<<REDUCE_GRID, REDUCE_THREADS, 0, st>>>(mp.partial, blocks, grad, summed ? loss : nullptr);
 	KGR_CUDA(cudaGetLastError());
 }

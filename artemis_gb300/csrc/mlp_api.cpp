@@ -186,6 +186,19 @@ kgr_status kgr_mlp_test_wait_timeout(kgr_mlp *m, const void *x, uint32_t n, floa
 	});
 }
 
+kgr_status kgr_mlp_test_train_wait_timeout(kgr_mlp *m, const void *x, const float *targets, uint32_t n,
+		float *grad_host)
+{
+	return guard([&] {
+		KGR_REQUIRE(m && n > 0 && x && targets && grad_host, KGR_ERR_INVALID_ARGUMENT, "NULL argument");
+		KGR_REQUIRE(m->train == KGR_MLP_TRAIN_TCGEN05, KGR_ERR_INVALID_ARGUMENT, "not the tcgen05 kernel");
+		DeviceGuard g(m->device);
+		mlp_gradients(m->params(), x, reinterpret_cast<const float4 *>(targets), n, m->grad.ptr, m->loss.ptr, 0, nullptr, 0,
+			true);
+		KGR_CUDA(cudaMemcpy(grad_host, m->grad.ptr, KGR_MLP_PARAMS * 4, cudaMemcpyDeviceToHost));
+	});
+}
+
 kgr_status kgr_mlp_check(kgr_mlp *m)
 {
 	return guard([&] {
@@ -196,7 +209,7 @@ kgr_status kgr_mlp_check(kgr_mlp *m)
 		KGR_CUDA(cudaMemcpy(&e, m->tc_err.ptr, sizeof(e), cudaMemcpyDeviceToHost));
 		if (e) {
 			KGR_CUDA(cudaMemset(m->tc_err.ptr, 0, sizeof(uint32_t)));
-			throw Error(KGR_ERR_CUDA, "tensor-core inference: an mbarrier wait ran out of its iteration limit");
+			throw Error(KGR_ERR_CUDA, "tensor-core network kernel: an mbarrier wait ran out of its iteration limit");
 		}
 	});
 }

@@ -446,7 +446,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__
 
 /* Training (forward, loss, backward) on the fifth-generation tensor cores.
  * One CTA an SM: two chains of 128 threads, each walking tiles of 128 rows
- * (thread = row = TMEM lane), and a warp that issues every MMA.  All operands
+ * (thread = row = TMEM lane), a warp a chain that issues its forward and delta
+ * MMAs, and one that issues both chains' weight gradients.  All operands
  * are in the canonical layout without swizzle (8 x 8 core matrices of 128
  * contiguous bytes, column neighbours 128 bytes apart, 8-row groups 1024), and
  * each is stored once and read both ways, K-major or, with the descriptor's
@@ -494,8 +495,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__
  * tile an SM.
  *
  * Every wait is bounded; a warp whose wait runs out leaves, so that every
- * later wait of its chain and of the issuer runs out too, and bit 0 of the
- * error word is set. */
+ * later wait of its chain and of the issuers runs out too.  The block meets at
+ * its barrier, each issuer waits (bounded) for the MMAs it has issued, the block
+ * sets bit 0 of the error word, writes zeros for its gradient, frees its tensor
+ * memory and returns.  kgr_mlp_test_train_wait_timeout exercises that path
+ * (WITHHOLD: each block's first warp never reports its first tile's rows, so
+ * chain, issuer and the issuer of dW run out). */
 #define TT_ROWS 128
 #define TT_CHAINS 2
 #define TT_WARPS (5 * TT_CHAINS + 1)            /* four a chain, its issuer, the issuer of dW */
@@ -505,10 +510,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_infer_tc_kernel(const T *__
 #define TT_CHAIN_OFF TC_W_BYTES                   /* 43,008 */
 #define TT_CHAIN_BYTES (TT_BUFS * TT_TILE_BYTES + TT_ROWS * TC_OUT * 2u)
 #define TT_BAR_OFF (TT_CHAIN_OFF + TT_CHAINS * TT_CHAIN_BYTES) /* per chain: ready, done, the same for dW */
-#define TT_SLOT_OFF (TT_BAR_OFF + TT_CHAINS * 32u)
-#define TT_SMEM (TT_SLOT_OFF + 8u)              /* 215,112 bytes */
+#define TT_DRAIN_OFF (TT_BAR_OFF + TT_CHAINS * 32u)            /* per issuer: its MMAs after a give-up */
+#define TT_SLOT_OFF (TT_DRAIN_OFF + (TT_CHAINS + 1u) * 8u)
+#define TT_SMEM (TT_SLOT_OFF + 8u)              /* 215,136 bytes */
 #define TT_TMEM_COLS 512u
-#define TT_WAIT_LIMIT (1u << 18)    /* mbarrier polls before a wait gives up */
+/* mbarrier polls before a wait gives up.  A poll suspends the thread for a while:
+ * a pass whose waits run out after 2^16 of them takes 0.24 s, one with this
+ * limit about a second, a million times a stage */
+#define TT_WAIT_LIMIT (1u << 18)
 #define TT_DW_COL(l) (64u * TT_CHAINS + 64u * (uint32_t)(l))   /* dW of layer l (layer 5: 16 columns) */
 #define TT_TRANSPOSE_A (1u << 15)                 /* instruction descriptor: MN-major operands */
 #define TT_TRANSPOSE_B (1u << 16)
@@ -581,7 +590,7 @@ __device__ __forceinline__ void store32(float *dst, const uint32_t *v, bool vali
 		"r"(valid ? v[4] : 0u), "r"(valid ? v[5] : 0u), "r"(valid ? v[6] : 0u), "r"(valid ? v[7] : 0u) : "memory");
 }
 
-template <class T>
+template <class T, bool WITHHOLD>
 __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__restrict__ wt_g,
 		const T *__restrict__ x, const float4 *__restrict__ target, uint32_t n, float *__restrict__ partial,
 		const uint32_t *__restrict__ n_dev, uint32_t *__restrict__ err)
@@ -590,6 +599,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 		uint32_t c = *n_dev;
 		n = c < n ? c : n;
 	}
+	constexpr uint32_t limit = WITHHOLD ? TC_WAIT_TEST_LIMIT : TT_WAIT_LIMIT;
 	extern __shared__ __align__(1024) unsigned char sm[];
 	const int tid = threadIdx.x, warp = tid >> 5;
 	const uint32_t lane = (uint32_t)tid & 31u;
@@ -620,6 +630,9 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 	if (tid == 0) {
 		for (uint32_t i = 0; i < 4u * TT_CHAINS; i++)
 			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bars + 8u * i), "r"(i & 1u ? 1u : 4u)
+				: "memory");
+		for (uint32_t i = 0; i <= TT_CHAINS; i++)
+			asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(base + TT_DRAIN_OFF + 8u * i), "r"(1u)
 				: "memory");
 		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 	}
@@ -658,7 +671,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 						const uint64_t a = m64 + ((buf0 + ia * TT_TILE_BYTES) >> 4);
 						const uint32_t d = (buf0 + (l == TC_LAYERS - 1 ? TT_BUFS : id) * TT_TILE_BYTES) >> 4;
 						const uint32_t sum = b != blockIdx.x || c > 0 ? 1u : 0u, dw = tmem + TT_DW_COL(l);
-						ok = bar_wait(bar, phase, TT_WAIT_LIMIT);
+						ok = bar_wait(bar, phase, limit);
 						if (!ok)
 							break;
 						tc_after();
@@ -692,7 +705,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 			bool first = true;
 			auto next = [&]() -> bool {
 				phase ^= 1u;
-				ok = first || bar_wait(bar, phase, TT_WAIT_LIMIT);
+				ok = first || bar_wait(bar, phase, limit);
 				if (first)
 					phase ^= 1u;
 				first = false;
@@ -739,7 +752,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 		uint32_t phase = 0, dw_phase = 0, start = 0;
 		/* wait for the committed MMAs: the chain's, a dW's */
 		auto wait_for = [&](uint32_t bar, uint32_t &parity) -> bool {
-			bool got = bar_wait(bar, parity, TT_WAIT_LIMIT);
+			bool got = bar_wait(bar, parity, limit);
 			parity ^= 1u;
 			got = __all_sync(0xffffffffu, got) != 0;
 			tc_after();
@@ -752,7 +765,7 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 			fence_async_smem();
 			tc_before();
 			__syncwarp();
-			if (lane == 0) {
+			if (lane == 0 && !(WITHHOLD && warp == 0)) {
 				asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(ready) : "memory");
 				if (dw)
 					asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(dw_ready) : "memory");
@@ -857,9 +870,18 @@ __global__ void __launch_bounds__(TT_THREADS, 1) mlp_train_tc_kernel(const T *__
 	}
 	tc_before();
 	ok = __syncthreads_and(ok) != 0;
+	if (!ok) {
+		/* MMAs that nobody has waited for: this thread's own, or none */
+		if (chain >= TT_CHAINS && lane == 0) {
+			const uint32_t bar = base + TT_DRAIN_OFF + 8u * ((uint32_t)warp - 4u * TT_CHAINS);
+			tc_commit(bar);
+			bar_wait(bar, 0u, limit);
+		}
+		if (tid == 0)
+			atomicOr(err, 1u);
+		__syncthreads();
+	}
 	tc_after();
-	if (!ok && tid == 0)
-		atomicOr(err, 1u);
 	/* this block's dW: lanes 32q..32q+15 hold rows 16q..16q+15 of 64 */
 	float *slice = partial + (size_t)blockIdx.x * TC_LAYERS * TC_W * TC_W;
 	float *warp_loss = reinterpret_cast<float *>(sm); /* the weights are done with */
@@ -942,21 +964,29 @@ void set_train_smem(K kernel)
 
 } /* namespace */
 
+namespace {
+
+template <class T, bool WITHHOLD>
+void launch_train(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, const uint32_t *n_dev,
+		cudaStream_t st)
+{
+	static bool once = (set_train_smem(mlp_train_tc_kernel<T, WITHHOLD>), true);
+	(void)once;
+	mlp_train_tc_kernel<T, WITHHOLD><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const T *>(mp.wt),
+		static_cast<const T *>(x), target, n, mp.partial, n_dev, mp.tc_err);
+}
+
+} /* namespace */
+
 void mlp_train_tc(const MlpParams &mp, const void *x, const float4 *target, uint32_t n, int grid, cudaStream_t st,
-		const uint32_t *n_dev)
+		const uint32_t *n_dev, bool withhold)
 {
 	KGR_REQUIRE(((uintptr_t)x & 15u) == 0, KGR_ERR_INVALID_ARGUMENT, "inputs must be 16-byte aligned");
-	if (mp.dtype == KGR_MLP_BF16) {
-		static bool once = (set_train_smem(mlp_train_tc_kernel<__nv_bfloat16>), true);
-		(void)once;
-		mlp_train_tc_kernel<__nv_bfloat16><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const __nv_bfloat16 *>(mp.wt),
-			static_cast<const __nv_bfloat16 *>(x), target, n, mp.partial, n_dev, mp.tc_err);
-	} else {
-		static bool once = (set_train_smem(mlp_train_tc_kernel<__half>), true);
-		(void)once;
-		mlp_train_tc_kernel<__half><<<grid, TT_THREADS, TT_SMEM, st>>>(static_cast<const __half *>(mp.wt),
-			static_cast<const __half *>(x), target, n, mp.partial, n_dev, mp.tc_err);
-	}
+	const bool bf16 = mp.dtype == KGR_MLP_BF16;
+	if (withhold)
+		(bf16 ? launch_train<__nv_bfloat16, true> : launch_train<__half, true>)(mp, x, target, n, grid, n_dev, st);
+	else
+		(bf16 ? launch_train<__nv_bfloat16, false> : launch_train<__half, false>)(mp, x, target, n, grid, n_dev, st);
 	KGR_CUDA(cudaGetLastError());
 }
 

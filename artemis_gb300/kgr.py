@@ -174,6 +174,7 @@ def lib():
             "kgr_denoiser_copy_result": (c_i32, [vp, vp, c_u64]),
             "kgr_mlp_check": (c_i32, [vp]),
             "kgr_mlp_test_wait_timeout": (c_i32, [vp, vp, c_u32, vp, vp]),
+            "kgr_mlp_test_train_wait_timeout": (c_i32, [vp, vp, vp, c_u32, vp]),
             "kgr_get_visit_counts": (c_i32, [vp, vp]),
             "kgr_measure_read_bandwidth": (c_i32, [c_i32, c_u64, c_i32, vp]),
             "kgr_load_attachment": (PluginRet, [ctypes.c_char_p]),
@@ -579,6 +580,12 @@ class Mlp:
     def test_wait_timeout(self, x_ptr, n, out_ptr, stream=None):
         """One tcgen05 inference whose loads are withheld, so its waits run out (a test of that path)."""
         check(lib().kgr_mlp_test_wait_timeout(self.handle, x_ptr, n, out_ptr, stream))
+
+    def test_train_wait_timeout(self, x_ptr, t_ptr, n):
+        """One tcgen05 gradient pass whose waits run out (a test of that path); its gradients."""
+        g = np.full((6, 64, 64), np.nan, np.float32)
+        check(lib().kgr_mlp_test_train_wait_timeout(self.handle, x_ptr, t_ptr, n, _ptr(g)))
+        return g
 
     def close(self):
         if self.handle:

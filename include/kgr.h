@@ -544,8 +544,8 @@ kgr_status kgr_mlp_set_inference(kgr_mlp *mlp, int32_t kernel);
  * runs out is reported by kgr_mlp_check. */
 enum { KGR_MLP_TRAIN_MMA = 0, KGR_MLP_TRAIN_TCGEN05 = 1 };
 kgr_status kgr_mlp_set_training(kgr_mlp *mlp, int32_t kernel);
-/* Synchronise the device and report a tcgen05 inference whose mbarrier wait
- * ran out (KGR_ERR_CUDA; the flag is then cleared).  KGR_OK otherwise. */
+/* Synchronise the device and report a tcgen05 inference or gradient pass whose
+ * mbarrier wait ran out (KGR_ERR_CUDA; the flag is then cleared).  KGR_OK otherwise. */
 kgr_status kgr_mlp_check(kgr_mlp *mlp);
 /* A test of the timeout path: one tcgen05 inference over x (n rows) whose
  * blocks never issue their first tile's load, so each block's wait on it
@@ -553,6 +553,13 @@ kgr_status kgr_mlp_check(kgr_mlp *mlp);
  * tensor memory and return without writing `out`.  kgr_mlp_check then
  * reports KGR_ERR_CUDA, and the network stays usable. */
 kgr_status kgr_mlp_test_wait_timeout(kgr_mlp *mlp, const void *x, uint32_t n, float *out, void *stream);
+/* The same of training: one tcgen05 gradient pass over n rows whose blocks
+ * never report the first tile's activations, so the waits of the chains and of
+ * the issuing warps run out after 65,536 polls each; the blocks set the error
+ * word, free their tensor memory and return with gradients of zero (host
+ * memory, 6*64*64 floats).  The weights are not touched.  Synchronous. */
+kgr_status kgr_mlp_test_train_wait_timeout(kgr_mlp *mlp, const void *x, const float *targets, uint32_t n,
+		float *grad_host);
 
 /* ------------------------------------------------------ after the frame -- */
 

@@ -214,3 +214,26 @@ def test_training_tile_counts(dtype, tiles, rest):
     _, again = gradients(net, "tcgen05", xd, td, n)
     assert np.array_equal(np.asarray(g_tc).view(np.uint32), np.asarray(again).view(np.uint32))
     net.check()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("n", [77, 400 * 128 + 5])
+def test_training_wait_timeout_is_reported_and_the_network_recovers(dtype, n):
+    """A gradient pass whose blocks never report their first activations, with
+    one chain at work in a block and with both: every chain's and issuer's
+    wait runs out, kgr_mlp_check raises, the gradients are zero, and the next
+    ordinary pass gives the same gradients as the one before."""
+    net = kgr.Mlp(dtype, seed=9)
+    rng = np.random.default_rng(4)
+    xd = half_tensor(mlp_ref.encode_inputs(rng, n, dtype), dtype)
+    td = torch.rand((n, 4), device="cuda")
+    before = gradients(net, "tcgen05", xd, td, n)
+    g = net.test_train_wait_timeout(xd.data_ptr(), td.data_ptr(), n)
+    with pytest.raises(kgr.KgrError, match="iteration limit"):
+        net.check()
+    assert not g.any()
+    net.check()  # the flag was cleared
+    after = gradients(net, "tcgen05", xd, td, n)
+    assert np.abs(before[1]).max() > 0
+    np.testing.assert_array_equal(before[1], after[1])
+    assert before[0] == after[0]
