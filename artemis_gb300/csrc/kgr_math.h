@@ -14,7 +14,7 @@
  * rotate :2653): e.g. `v / s` is `v * (1.0f / s)`, `normalize(v)` is
  * `v * (1.0f / sqrtf(dot(v, v)))`, `dot` sums left to right.
  *
- * The transcendental functions (sin, cos, tan, atan, acos) are this
+ * The transcendental functions (sin, cos, atan, acos) are this
  * project's own: Cody-Waite reduction by pi/2 (three-part split computed
  * from pi to 200 bits) followed by Taylor polynomials on |r| <= pi/4
  * (sin/cos) or |r| <= tan(pi/12) (atan).  Their error is within a couple of
@@ -117,9 +117,10 @@ KGR_HD f3 fmax3(const f3 &a, const f3 &b) { return mk(kmax(a.x, b.x), kmax(a.y, 
 KGR_HD float comp(const f3 &v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : v.z); }
 KGR_HD bool anynan(const f3 &v) { return kisnan(v.x) || kisnan(v.y) || kisnan(v.z); }
 
-/* math.cuh:2604-2607 */
+/* math.cuh:2604-2607.  Draws (pcg3f) are in [0, 1) already, where it changes
+ * nothing: loops over draws leave it out, and the calls that remain, one a ray
+ * or a vertex, follow the reference's lines. */
 KGR_HD float fract(float x) { return x - kfloor(x); }
-KGR_HD f3 fract(const f3 &v) { return mk(fract(v.x), fract(v.y), fract(v.z)); }
 
 /* ------------------------------------------------------ transcendentals -- */
 
@@ -189,7 +190,6 @@ KGR_HD void ksincos_quarter(float x, float &s, float &c)
 
 KGR_HD float ksin(float x) { float s, c; ksincos(x, s, c); return s; }
 KGR_HD float kcos(float x) { float s, c; ksincos(x, s, c); return c; }
-KGR_HD float ktan(float x) { float s, c; ksincos(x, s, c); return s / c; }
 
 /* atan for |y| <= tan(pi/12) (Taylor series, truncation < 2e-9). */
 KGR_HD float atan_kernel(float y)

@@ -207,15 +207,6 @@ __device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&v)[64])
 		: "r"(taddr) : "memory");
 }
 
-/* 32 consecutive FP32 columns of this thread's TMEM lane. */
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
-{
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-		"{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-		"%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-		: TC_R8(0), TC_R8(8), TC_R8(16), TC_R8(24) : "r"(taddr) : "memory");
-}
-
 /* 16 consecutive FP32 columns of this thread's TMEM lane. */
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16])
 {

@@ -202,7 +202,7 @@ void launch_trace_persistent(const DeviceScene &s, const float4 *rays, uint32_t 
 	static const uint32_t resident = (uint32_t)resident_blocks(trace_many_kernel<ANY, LAYOUT, false>, TRACE_BLOCK);
 	static const uint32_t resident_many = (uint32_t)resident_blocks(trace_many_kernel<ANY, LAYOUT, true>, TRACE_BLOCK);
 	if (LAYOUT == KGR_LAYOUT_FAST && s.coop_nodes) {
-		/* up to KGR_COOP_ROUNDS rays for each of the resident groups */
+		/* up to KGR_COOP_ROUNDS_RAYS rays for each of the resident groups */
 		static const int coop = resident_blocks(trace_coop_kernel<ANY>, TRACE_BLOCK);
 		const uint32_t groups = (uint32_t)coop * (TRACE_BLOCK / 8);
 		if (n <= KGR_COOP_ROUNDS_RAYS * groups) {
