@@ -60,16 +60,18 @@ KGR_HD void cw_axis_grid(float lo, float hi, int &e, float &p)
 	e = k;
 }
 
+/* (Planes at infinity, where padding overflows, may give no number: 0, the
+ * same on host and device.) */
 KGR_HD uint32_t cw_qlo(float plane, float p, double s)
 {
 	double q = floor(((double)plane - (double)p) / s - 0.5);
-	return (uint32_t)(q < 0.0 ? 0.0 : (q > 255.0 ? 255.0 : q));
+	return (uint32_t)(q >= 0.0 ? (q > 255.0 ? 255.0 : q) : 0.0);
 }
 
 KGR_HD uint32_t cw_qhi(float plane, float p, double s)
 {
 	double q = ceil(((double)plane - (double)p) / s + 0.5);
-	return (uint32_t)(q < 0.0 ? 0.0 : (q > 255.0 ? 255.0 : q));
+	return (uint32_t)(q >= 0.0 ? (q > 255.0 ? 255.0 : q) : 0.0);
 }
 
 /* Fill origin (p, exponents, imask) and the three quantised plane words of

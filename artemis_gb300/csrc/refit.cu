@@ -335,26 +335,24 @@ __device__ __forceinline__ uint32_t plane_hi(float plane, float p, int e)
 	return (uint32_t)fminf(fmaxf(q, 0.0f), 255.0f);
 }
 
-/* Slot j of a node whose extent [lo, hi] a float may not hold, by the double
- * precision rules themselves.  Out of line: the others' registers do not see
- * it (inlined, a refit of the 1.16M-triangle terrain took 5 us longer). */
-__device__ __noinline__ void wide_slot(CwNode *node, uint32_t j, bool used, uint32_t imask, f3 lo, f3 hi, f3 mn, f3 mx)
+/* Node c by the double precision rules themselves: for one whose extent a float
+ * may not hold.  Out of line, and bounded like its caller, so that the others'
+ * registers do not see it. */
+__device__ __noinline__ void wide_node(const int32_t *kids, uint32_t c, const float4 *boxes, CwNode *cw)
 {
-	uint8_t *q = reinterpret_cast<uint8_t *>(&node->qa) + j;
-	const float l[3] = {lo.x, lo.y, lo.z}, h[3] = {hi.x, hi.y, hi.z};
-	const float a[3] = {mn.x, mn.y, mn.z}, b[3] = {mx.x, mx.y, mx.z};
-	uint32_t bits = imask << 24;
-	float p[3];
-	for (int x = 0; x < 3; x++) {
-		int e;
-		cw_axis_grid(l[x], h[x], e, p[x]);
-		bits |= (uint32_t)(e + 127) << (8 * x);
-		const double s = ldexp(1.0, e);
-		q[8 * x] = (uint8_t)(used ? cw_qlo(a[x], p[x], s) : 255u);
-		q[24 + 8 * x] = (uint8_t)(used ? cw_qhi(b[x], p[x], s) : 0u);
+	float lo[8][3], hi[8][3];
+	uint32_t used = 0;
+	for (int j = 0; j < 8; j++) {
+		const int32_t k = kids[8 * (size_t)c + j];
+		for (int x = 0; x < 3; x++)
+			lo[j][x] = hi[j][x] = 0.0f;
+		if (k < 0)
+			continue;
+		used |= 1u << j;
+		padded(boxes, k, lo[j], hi[j]);
 	}
-	if (j == 0u)
-		node->origin = make_float4(p[0], p[1], p[2], __uint_as_float(bits));
+	CwNode &n = cw[c];
+	cw_quantize(lo, hi, used, __float_as_uint(n.origin.w) >> 24, n.origin, n.qa, n.qb, n.qc);
 }
 
 /* The slots of the eight-child nodes, one a thread, eight lanes a node: the
@@ -367,7 +365,7 @@ __device__ __noinline__ void wide_slot(CwNode *node, uint32_t j, bool used, uint
  * its eight boxes in local memory: 420 us for the 1.16M-triangle terrain's
  * 196,000 nodes, and the cooperative nodes 20 us; this kernel 36 us for both. */
 template <bool QUANT>
-__global__ void __launch_bounds__(REFIT_BLOCK) slot_nodes_kernel(const int32_t *__restrict__ kids, uint32_t slots,
+__global__ void __launch_bounds__(REFIT_BLOCK, 8) slot_nodes_kernel(const int32_t *__restrict__ kids, uint32_t slots,
 		const float4 *__restrict__ boxes, CwNode *__restrict__ cw, CoopNode *__restrict__ out)
 {
 	const unsigned full = 0xffffffffu;
@@ -427,8 +425,8 @@ __global__ void __launch_bounds__(REFIT_BLOCK) slot_nodes_kernel(const int32_t *
 		if (!in)
 			continue;
 		if (!(fmaxf(hi[0] - lo[0], fmaxf(hi[1] - lo[1], hi[2] - lo[2])) < 0.5f * FLT_MAX)) {
-			wide_slot(&cw[c], j, k >= 0, imask, mk(lo[0], lo[1], lo[2]), mk(hi[0], hi[1], hi[2]), mk(mn[0], mn[1], mn[2]),
-				mk(mx[0], mx[1], mx[2]));
+			if (j == 0u)
+				wide_node(kids, c, boxes, cw);
 			continue;
 		}
 		/* planes: lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, a byte a slot */
