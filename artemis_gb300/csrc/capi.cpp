@@ -369,6 +369,7 @@ void finish_scene(kgr_scene *sc, const Tree &tree, const std::vector<PrimBox> &b
 		sc->cw_node_count = (uint32_t)cw.size();
 		sc->cw_depth = cw_depth;
 		static_assert(sizeof(CwNode) == 80, "compressed node size");
+		static_assert(2 * KGR_COOP_LEVELS >= KGR_CW_STACK, "cooperative walk's stack");
 		KGR_REQUIRE(((uintptr_t)sc->d_cw_nodes.ptr & 15) == 0, KGR_ERR_INTERNAL, "compressed nodes misaligned");
 		/* the cooperative walk's nodes: made on the device, as a refit makes
 		 * them again */

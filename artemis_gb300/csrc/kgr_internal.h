@@ -193,8 +193,9 @@ struct CoopNode {
 #define KGR_COOP_ROUNDS 4u
 #define KGR_COOP_ROUNDS_OVERLAPPED 2u
 /* A caller's ray buffer may be more coherent than a bounce: 65,000 camera rays
- * on the box scene 85 us with this walk and 66 with one ray per thread, 40,000
- * of them 54 and 70. */
+ * on the box scene 85 us with this walk and 66 with one ray per thread.  52,000
+ * rays on the three scenes, this walk / one ray per thread: camera 68, 54, 76 /
+ * 66, 84, 96, bounce 66, 71, 90 / 84, 77, 98, shadow 50, 49, 56 / 81, 65, 84. */
 #define KGR_COOP_ROUNDS_RAYS 3u
 /* So camera walks of frames take that limit too where nodes and triangles are
  * about what two SMs' L1 hold and the per-thread walk seldom waits for L2.
@@ -202,7 +203,8 @@ struct CoopNode {
  * 248, 264 us and with 3 235, 241; its triangles divided into 16,944 (1.5 MB)
  * 287, 303 and 293, 298, into 67,776 323, 342 and 342, 349. */
 #define KGR_SMALL_TREE (512u << 10)
-/* most nodes on a path of the cooperative walk */
+/* most nodes on a path of the cooperative walk: the compressed layout is kept
+ * when twice its depth and two fit KGR_CW_STACK */
 #define KGR_COOP_LEVELS 16
 
 /* traversal stack entries of the compressed layout (node groups) */

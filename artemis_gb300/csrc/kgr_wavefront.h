@@ -70,7 +70,8 @@ struct PathBuffers {
 };
 
 /* The rays of bounce `depth`: on a scene open to the sky about half a bounce's
- * rays miss. */
+ * rays miss.  (In a closed scene none does; its later bounces are longer than
+ * this says and keep the launch of short walks.) */
 inline uint32_t likely_rays(uint32_t paths, int depth) { return depth < 32 ? paths >> depth : 0; }
 
 /* The float4 arrays of the path state, in the order their allocators lay

@@ -1,6 +1,8 @@
-"""The ray-buffer walk at the counts where its split over warps changes: one
-ray, a partial warp, block and chunk edges, one ray a warp, a few lanes a
-warp, and lanes that refill."""
+"""Walks at the counts where their kernels and launch shapes change: ray buffers
+of one ray, a partial warp, block and group edges, eight lanes a ray and one
+ray a thread (test_gpu_ray_buffers.py has the larger, refilling ones), and
+frames on both sides of the cooperative walk's limits and of the register
+bound."""
 import numpy as np
 import pytest
 
